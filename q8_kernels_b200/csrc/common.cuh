@@ -34,6 +34,8 @@ void set_error_detail(const char* fmt, ...);
         }                                                                          \
     } while (0)
 
+int gemm_num_sms();                          // SMs of the current device (148 if it cannot be asked)
+
 inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
 
 // ---------------------------------------------------------------- element types
@@ -120,6 +122,14 @@ template <> __device__ __forceinline__ float from_float<float>(float v) { return
 template <> __device__ __forceinline__ __half from_float<__half>(float v) { return __float2half_rn(v); }
 template <> __device__ __forceinline__ __nv_bfloat16 from_float<__nv_bfloat16>(float v) { return __float2bfloat16_rn(v); }
 template <> __device__ __forceinline__ e4m3_t from_float<e4m3_t>(float v) { return e4m3_t{float_to_e4m3_c10(v)}; }
+
+// Four e4m3 bytes widened through two packed e4m3x2 -> f16x2 conversions (exact).
+__device__ __forceinline__ void e4m3x4_to_float(uint32_t w, float (&o)[4]) {
+    const __half2_raw lo = __nv_cvt_fp8x2_to_halfraw2((__nv_fp8x2_storage_t)(w & 0xffffu), __NV_E4M3);
+    const __half2_raw hi = __nv_cvt_fp8x2_to_halfraw2((__nv_fp8x2_storage_t)(w >> 16), __NV_E4M3);
+    const float2 a = __half22float2(__half2(lo)), c = __half22float2(__half2(hi));
+    o[0] = a.x; o[1] = a.y; o[2] = c.x; o[3] = c.y;
+}
 
 // ---------------------------------------------------------------- vector access
 // N consecutive elements of T <-> fp32 registers.  N * sizeof(T) must be 4, 8,

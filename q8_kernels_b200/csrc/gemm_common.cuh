@@ -60,8 +60,6 @@ __device__ __forceinline__ float2 epilogue_pair(uint32_t r0, uint32_t r1, float2
     return y;
 }
 
-int gemm_num_sms();
-
 // CTA-pair (cta_group::2) variant: 256 x 256 output tiles per cluster of two CTAs.  Returns
 // Q8K_ERR_UNSUPPORTED (without touching the error detail) when the device cannot co-schedule
 // the clusters, in which case the caller falls back to the single-CTA kernel.

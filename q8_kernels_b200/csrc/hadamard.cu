@@ -11,11 +11,9 @@
 //  * rows of <= 256 elements: a group of G = n/8 lanes owns a row (8 elements
 //    per lane, one 16-byte load), 32/G rows per warp; stages 0-2 in registers,
 //    the rest by xor-shuffles inside the group.
-//  * rows of 512 .. 16384 elements: 16-64 threads per row with 32-128 values
-//    each; the first 5-7 stages run in registers on consecutive elements, the
-//    rest after one swizzled shared-memory exchange (two for 16384), all on
-//    packed fp32 pairs; no shuffles.  Shared-memory traffic, not issue slots or
-//    HBM, is what this schedule is sized for: 12 bytes per element in total.
+//  * rows of 512 .. 16384 elements: 64 values per thread; stages 0-5 run in registers on consecutive
+//    elements, the rest after one padded shared-memory exchange (two above 2048), all on packed fp32
+//    pairs; no shuffles.
 
 #include <type_traits>
 #include "common.cuh"
@@ -53,18 +51,6 @@ __device__ __forceinline__ void fwht_lanes(float (&v)[N], int lane, int mask) {
 // Round the scaled transform to the dtype the unfused chain would have stored.
 template <typename T> __device__ __forceinline__ float round_through(float v) {
     return to_float<T>(from_float<T>(v));
-}
-
-// Two values at once: for bf16 one packed conversion (an ALU-pipe F2FP instead of two conversions on
-// the 16-lane special-function unit) and two bit operations to widen the halves again.
-template <typename T> __device__ __forceinline__ float2 round_through2(float a, float b) {
-    if constexpr (std::is_same_v<T, __nv_bfloat16>) {
-        const __nv_bfloat162 p = __floats2bfloat162_rn(a, b);  // a in the low half
-        const uint32_t w = *reinterpret_cast<const uint32_t*>(&p);
-        return make_float2(__uint_as_float(w << 16), __uint_as_float(w & 0xffff0000u));
-    } else {
-        return make_float2(round_through<T>(a), round_through<T>(b));
-    }
 }
 
 template <typename Tq> __device__ __forceinline__ uint8_t quantize_one(float y) {
@@ -149,17 +135,8 @@ hadamard_small_kernel(const Tin* __restrict__ x, Tout* __restrict__ out, float* 
 }
 
 // ------------------------------------------------------------------ large rows
-// One CTA per row of N = 2^LOG_N (padded) elements, T = N / V threads, V = 2^LOG_V values per
-// thread.  The row is staged raw in shared memory by coalesced loads; each thread then owns V
-// consecutive elements and runs stages 0 .. LOG_V-1 in registers.  The remaining stages run in
-// phases of up to LOG_V-2 bits: the row is exchanged through shared memory (fp32, natural element
-// order, float4 chunks XOR-swizzled so that both sides are conflict free) into a layout where a
-// thread owns 2^b groups x C consecutive elements, the groups being the butterfly partners.
-// Butterflies work on packed fp32 pairs (add/sub.f32x2), so a stage costs half an instruction per
-// element; only the stride-1 stage is scalar.
-
-
-__device__ __forceinline__ int swz4(int q) { return q ^ ((q >> 3) & 7); }      // float4-chunk swizzle
+// Butterflies work on packed fp32 pairs (add/sub.f32x2), so a stage costs half an instruction per element; only the
+// stride-1 stage is scalar.
 
 // Layout of a phase that butterflies bits [LO, LO+B): thread t owns groups j = 0 .. 2^B-1 of
 // C = V >> B consecutive elements each.  The thread index supplies the other bits of the
@@ -177,61 +154,6 @@ struct PhaseLayout {
         return ((t & ((1 << LOWT) - 1)) << LOG_C) + (j << LO) + ((t >> LOWT) << (LO + B));
     }
 };
-
-// Shared-memory exchange in natural element order, float4 chunks XOR-swizzled (swz4).  elem(t, j)
-// is a bitwise OR of disjoint bit fields and swz4 is linear over XOR, so the swizzled byte offset of
-// (t, j, k) is  offset(t) ^ offset(j, k)  with the second term a compile-time constant: one XOR per
-// access instead of re-deriving the swizzle.  Runs of 2 use float2 accesses inside the chunk (the
-// half-chunk select bit belongs to the thread term).
-template <typename L>
-__device__ __forceinline__ uint32_t exchange_thread_offset(int t) {
-    const int e = L::elem(t, 0);
-    uint32_t off = (uint32_t)swz4(e >> 2) << 4;
-    if constexpr (L::C < 4) off |= (uint32_t)((e >> 1) & 1) << 3;
-    return off;
-}
-template <typename L>
-__device__ __forceinline__ constexpr uint32_t exchange_const_offset(int j, int k) {
-    const int q = ((j << L::LOW) >> 2) + k;
-    return (uint32_t)(q ^ ((q >> 3) & 7)) << 4;
-}
-
-// registers (layout L) -> shared memory
-template <typename L, int V>
-__device__ __forceinline__ void exchange_write(float* xch, const float (&v)[V], int t) {
-    char* xb = reinterpret_cast<char*>(xch);
-    const uint32_t tb = exchange_thread_offset<L>(t);
-#pragma unroll
-    for (int j = 0; j < L::G; ++j) {
-        if constexpr (L::C >= 4) {
-#pragma unroll
-            for (int k = 0; k < L::C / 4; ++k)
-                *reinterpret_cast<float4*>(xb + (tb ^ exchange_const_offset<L>(j, k))) =
-                    make_float4(v[j * L::C + 4 * k], v[j * L::C + 4 * k + 1], v[j * L::C + 4 * k + 2], v[j * L::C + 4 * k + 3]);
-        } else {
-            *reinterpret_cast<float2*>(xb + (tb ^ exchange_const_offset<L>(j, 0))) = make_float2(v[j * 2], v[j * 2 + 1]);
-        }
-    }
-}
-template <typename L, int V>
-__device__ __forceinline__ void exchange_read(const float* xch, float (&v)[V], int t) {
-    const char* xb = reinterpret_cast<const char*>(xch);
-    const uint32_t tb = exchange_thread_offset<L>(t);
-#pragma unroll
-    for (int j = 0; j < L::G; ++j) {
-        if constexpr (L::C >= 4) {
-#pragma unroll
-            for (int k = 0; k < L::C / 4; ++k) {
-                const float4 f = *reinterpret_cast<const float4*>(xb + (tb ^ exchange_const_offset<L>(j, k)));
-                v[j * L::C + 4 * k] = f.x; v[j * L::C + 4 * k + 1] = f.y;
-                v[j * L::C + 4 * k + 2] = f.z; v[j * L::C + 4 * k + 3] = f.w;
-            }
-        } else {
-            const float2 f = *reinterpret_cast<const float2*>(xb + (tb ^ exchange_const_offset<L>(j, 0)));
-            v[j * 2] = f.x; v[j * 2 + 1] = f.y;
-        }
-    }
-}
 
 // butterflies between groups (stride = whole groups of C >= 4 elements): all packed
 template <typename L, int V>
@@ -279,241 +201,414 @@ __device__ __forceinline__ void butterfly_consecutive(float (&v)[V]) {
     }
 }
 
-// Exact round-half-away-from-zero (C round()) of |y| < 2^22 with one add: adding the largest
-// float below 0.5 with y's sign and truncating gives floor(|y| + 0.5) for every fp32 y, ties
-// included (the sum of a tie k + 0.5 rounds up to k + 1, and 0.5 - 2^-25 stays below 1).
-__device__ __forceinline__ int round_half_away_int(float y) {
-    return __float2int_rz(__fadd_rn(y, copysignf(0.49999997f, y)));
-}
+// Units of whole warps walk over the rows (a grid of as many CTAs as fit the device): a row of up to 2048 elements
+// belongs to one warp or a part of one, a longer row to one CTA.  A thread has 64 values.  Per row: the raw elements
+// were copied into the unit's staging buffer by cp.async while the row before was being transformed; a thread reads
+// its 64 consecutive elements, does stages 0-5 in registers, and the remaining stages after one exchange through
+// shared memory (two above 2048).  The first exchange never leaves a warp and the staged elements are read by the
+// warp that copied them, so rows of up to 2048 elements need no block barrier at all and longer ones two.
+//
+// Bound by instruction issue and the FMA pipe (add/sub.f32x2 issue every second clock: 11 stages are 11 clocks per
+// element and scheduler), no longer by barriers and shared memory: 8 bytes per element of exchange (16 above 2048)
+// and 2 x the input size of staging, all accesses conflict-free with immediate offsets.  128 registers, 16 warps per SM.
+// Measured, 24576 x 2048, bf16 in, CUDA graph over inputs larger than L2 (one CTA per row pair, block-wide barriers,
+// two exchanges before): bf16 out 43.6 -> 33.7 us (0.92 of the copy rate), e4m3 rows 45.3 -> 35.9 us, int8 rows
+// 47.1 -> 41.5 us (one F2I per element on the 8-clock conversion unit), with norm + modulation 72.3 -> 52.1 us (int8).
+// 6144 x 8192: 49.5 -> 41.2, 50.1 -> 43.1, 53.2 -> 49.0, 109 -> 73.7 us.  Tried: 128 values per thread for 4096 and
+// 8192 (one exchange, half the warps; 59 us for int8 rows of 8192), XOR swizzles instead of pads (39.4 us, e4m3 rows).
 
-template <typename Tq>
-__device__ __forceinline__ uint8_t quantize_fast(float y) {
-    if constexpr (std::is_same_v<Tq, int8_t>) return (uint8_t)(int8_t)round_half_away_int(y);
-    else return float_to_e4m3_c10(y);
+__device__ __forceinline__ void cp_async_zfill(uint32_t dst, const void* src, int cp_bytes, bool valid) {
+    if (cp_bytes == 16)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(valid ? 16 : 0) : "memory");
+    else
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(dst), "l"(src), "r"(valid ? 8 : 0) : "memory");
 }
-
-// Four quantised bytes from four fp32 values, lowest address first.  INT8: round half away from zero
-// (one add + truncation each) and three byte permutes.  E4M3: two packed saturating conversions and
-// one permute; the caller guarantees |y| <= 448 (1 + 2^-23) for finite rows (y = v * (448 / amax) with
-// |v| <= amax), where the saturating cast and the c10 cast (overflow -> NaN beyond 464) agree, and a
-// NaN stays a NaN in both.
-template <typename Tq>
-__device__ __forceinline__ uint32_t quantize_pack4(float y0, float y1, float y2, float y3) {
-    if constexpr (std::is_same_v<Tq, int8_t>) {
-        const uint32_t q0 = (uint32_t)round_half_away_int(y0), q1 = (uint32_t)round_half_away_int(y1);
-        const uint32_t q2 = (uint32_t)round_half_away_int(y2), q3 = (uint32_t)round_half_away_int(y3);
-        return __byte_perm(__byte_perm(q0, q1, 0x0040), __byte_perm(q2, q3, 0x0040), 0x5410);
-    } else {
-        return (uint32_t)float2_to_e4m3x2_sat(y0, y1) | ((uint32_t)float2_to_e4m3x2_sat(y2, y3) << 16);
-    }
-}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_group 0;" ::: "memory"); }
 
 // NORM_MOD adds the block's pre-linear prologue in front of the transform, with the bf16 roundings
 // of the separate ops it replaces: n = bf16(x * rsqrt(mean x^2)); u = bf16(bf16(n * bf16(1 + s)) + h)
-// where s, h are the per-batch modulation rows (bf16 [rows / rows_per_mod, dim]).
-// FULL: dim == 2^LOG_N, so no element of a row needs a bounds test.
-template <typename Tin, typename Tout, int LOG_N, int LOG_V, int ROWS, Epilogue EPI, bool NORM_MOD = false, bool FULL = false>
-__global__ void __launch_bounds__(ROWS << (LOG_N - LOG_V))
-hadamard_row_kernel(const Tin* __restrict__ x, Tout* __restrict__ out, float* __restrict__ scales,
-                    int64_t rows, int dim, int64_t x_row_stride, float scale,
-                    const __nv_bfloat16* __restrict__ mod_scale = nullptr,
-                    const __nv_bfloat16* __restrict__ mod_shift = nullptr, int64_t rows_per_mod = 1) {
-    constexpr int N = 1 << LOG_N;
-    constexpr int V = 1 << LOG_V;
-    constexpr int T = N / V;                                   // threads per row
-    constexpr int ITEMS = V / 8;                               // 8-element input items per thread
-    constexpr int R = LOG_N - LOG_V;                           // bits left after the register phase
-    // one exchange when the bits fit (runs of >= 2 consecutive elements), else two balanced ones so
-    // that both keep runs of >= 4 (float4 accesses)
-    constexpr int BMAX = LOG_V - 1;
-    constexpr int B1 = R <= BMAX ? R : (R + 1) / 2;
-    constexpr int B2 = R - B1;
-    static_assert(B1 <= BMAX && B2 <= BMAX, "row too long for this values-per-thread choice");
-    using L0 = PhaseLayout<LOG_V, 0, LOG_V>;                   // V consecutive elements
+// where s, h are the per-batch modulation rows (bf16 [rows / rows_per_mod, dim]).  A CTA stays inside one batch entry
+// and keeps its two modulation rows in shared memory.
+// FULL: dim is the power of two itself, so no element of a row needs a bounds test.
+
+// Raw staging: position of the 16-byte chunk c (row order) of a row whose threads own CPT chunks each, such
+// that eight consecutive threads reading their k-th chunk touch eight different bank groups.
+template <int CPT>
+__device__ __forceinline__ constexpr int raw_pos(int c) {
+    if constexpr (CPT >= 8) return c ^ ((c / CPT) & 7);
+    else return c ^ ((c / CPT / (8 / CPT)) & (CPT - 1));
+}
+
+// fp32 exchange, V = 64: natural element order in 16-byte chunks, one pad chunk after the 16 chunks that a
+// thread writes (eight consecutive threads hit eight bank groups) and, where a layout with runs of 8 elements
+// reads it, one more after every 8.  Pads instead of an XOR: the position is thread term + constant, so every
+// access has an immediate offset and costs no address arithmetic.
+template <bool PAD8>
+__device__ __forceinline__ constexpr int xpos(int q) { return q + (q >> 4) + (PAD8 ? q >> 3 : 0); }
+
+template <typename L, bool PAD8, bool WRITE>
+__device__ __forceinline__ void xch_access(char* xb, float (&v)[64], int t) {
+    const int e0 = L::elem(t, 0);
+    char* base = xb + (xpos<PAD8>(e0 >> 2) << 4) + (L::C < 4 ? ((e0 >> 1) & 1) << 3 : 0);
+#pragma unroll
+    for (int j = 0; j < L::G; ++j) {
+        if constexpr (L::C >= 4) {
+#pragma unroll
+            for (int k = 0; k < L::C / 4; ++k) {
+                float4* a = reinterpret_cast<float4*>(base + (xpos<PAD8>(((j << L::LOW) >> 2) + k) << 4));
+                float* r = v + j * L::C + 4 * k;
+                if constexpr (WRITE) *a = make_float4(r[0], r[1], r[2], r[3]);
+                else { const float4 f = *a; r[0] = f.x; r[1] = f.y; r[2] = f.z; r[3] = f.w; }
+            }
+        } else {
+            float2* a = reinterpret_cast<float2*>(base + (xpos<PAD8>((j << L::LOW) >> 2) << 4));
+            if constexpr (WRITE) *a = make_float2(v[2 * j], v[2 * j + 1]);
+            else { const float2 f = *a; v[2 * j] = f.x; v[2 * j + 1] = f.y; }
+        }
+    }
+}
+
+template <typename Tin, int LOG_N, bool NORM_MOD>
+struct StreamGeo {
+    static constexpr int LOG_V = 6, V = 64;                    // values per thread
+    static constexpr int N = 1 << LOG_N, T = N / V;
+    static constexpr int R = LOG_N - LOG_V;                    // stages left after the register phase
+    static constexpr int B1 = R <= LOG_V - 1 ? R : (R + 1) / 2;   // one exchange while runs of two elements remain, else two
+    static constexpr int B2 = R - B1;
+    static_assert(B1 <= 5, "the first exchange stays inside a warp");
+    static constexpr bool PAD8 = LOG_V - B1 == 3 || (B2 > 0 && LOG_V - B2 == 3);
+    static constexpr int UNIT = T < 32 ? 32 : T;               // threads that work on the same rows
+    static constexpr int RPU = UNIT / T;                       // rows per unit and turn
+    static constexpr int THREADS = T > 32 ? T : 128;
+    static constexpr int UNITS = THREADS / UNIT;
+    static constexpr int RAW = RPU * N * (int)sizeof(Tin);     // bytes per unit
+    static constexpr int XROW = (N / 4 + N / 64 + (PAD8 ? N / 32 : 0)) * 16;
+    static constexpr int XCH = RPU * XROW;
+    static constexpr int MOD = NORM_MOD ? 2 * N * 2 : 0;       // bytes per CTA: 1 + scale and shift rows (bf16)
+    static constexpr int SMEM = UNITS * (RAW + XCH) + MOD;
+    static constexpr int BY_SMEM = (228 * 1024) / (SMEM + 1024);
+    static constexpr int BY_REGS = 65536 / (THREADS * 128);
+    static constexpr int CTAS = BY_SMEM < BY_REGS ? BY_SMEM : BY_REGS;
+};
+
+template <typename Tin, typename Tout, int LOG_N, Epilogue EPI, bool NORM_MOD, bool FULL>
+__global__ void __launch_bounds__(StreamGeo<Tin, LOG_N, NORM_MOD>::THREADS, StreamGeo<Tin, LOG_N, NORM_MOD>::CTAS)
+hadamard_stream_kernel(const Tin* __restrict__ x, Tout* __restrict__ out, float* __restrict__ scales, unsigned rows, int dim,
+                       int64_t x_row_stride, float scale, const __nv_bfloat16* __restrict__ mod_scale,
+                       const __nv_bfloat16* __restrict__ mod_shift, unsigned rows_per_mod, unsigned blocks_per_mod) {
+    using Geo = StreamGeo<Tin, LOG_N, NORM_MOD>;
+    constexpr int N = Geo::N, V = Geo::V, T = Geo::T, UNIT = Geo::UNIT, RPU = Geo::RPU, LOG_V = Geo::LOG_V;
+    constexpr int B1 = Geo::B1, B2 = Geo::B2;
+    constexpr bool PAD8 = Geo::PAD8;
+    using L0 = PhaseLayout<LOG_V, 0, LOG_V>;
     using L1 = PhaseLayout<LOG_V, B1, LOG_V>;
     using L2 = PhaseLayout<LOG_V, B2, LOG_V + B1>;
-
-    extern __shared__ __align__(16) float xch_all[];           // ROWS x N floats
-    __shared__ float red[32];
-    const int t = threadIdx.x % T;
-    const int r_in_cta = threadIdx.x / T;
-    const int64_t row = (int64_t)blockIdx.x * ROWS + r_in_cta;
-    const bool row_ok = row < rows;
-    float* xch = xch_all + r_in_cta * N;
-    const Tin* xr = x + row * x_row_stride;
-
-    // coalesced load of raw 8-element items into shared memory, then V consecutive elements per thread
-    {
-        using Item = typename Vec<8 * sizeof(Tin)>::type;
-        Item* stage = reinterpret_cast<Item*>(xch);
-#pragma unroll
-        for (int k = 0; k < ITEMS; ++k) {
-            const int item = t + k * T;
-            Item val;
-            if (row_ok && (FULL || item * 8 < dim)) val = *reinterpret_cast<const Item*>(xr + item * 8);
-            else memset(&val, 0, sizeof(val));
-            stage[item ^ ((item / ITEMS) & (ITEMS - 1))] = val;   // spread a thread's ITEMS reads over the banks
-        }
-    }
-    __syncthreads();
-    float v[V];
-    {
-        using Item = typename Vec<8 * sizeof(Tin)>::type;
-        const Item* stage = reinterpret_cast<const Item*>(xch);
-#pragma unroll
-        for (int k = 0; k < ITEMS; ++k) {
-            union { Item raw; Tin e[8]; } u;
-            u.raw = stage[(t * ITEMS + (t & (ITEMS - 1))) ^ k];   // == (t * ITEMS + k) ^ (t % ITEMS)
-#pragma unroll
-            for (int j = 0; j < 8; ++j) v[k * 8 + j] = to_float<Tin>(u.e[j]);
-        }
-    }
-    if constexpr (NORM_MOD) {
-        static_assert(std::is_same_v<Tin, __nv_bfloat16>, "the norm + modulation prologue takes bf16 rows");
-        __shared__ float red_ss[32];
-        float ss = 0.f;
-#pragma unroll
-        for (int i = 0; i < V; ++i) ss = fmaf(v[i], v[i], ss);
-#pragma unroll
-        for (int m = 1; m < (T < 32 ? T : 32); m <<= 1) ss += __shfl_xor_sync(0xffffffffu, ss, m);
-        if constexpr (T > 32) {
-            constexpr int WPR = T / 32;
-            if ((threadIdx.x & 31) == 0) red_ss[threadIdx.x >> 5] = ss;
-            __syncthreads();
-            ss = red_ss[r_in_cta * WPR];
-#pragma unroll
-            for (int k = 1; k < WPR; ++k) ss += red_ss[r_in_cta * WPR + k];
-        }
-        const float rr = rsqrtf(ss * (1.0f / (float)dim));
-        const int64_t mrow = row_ok ? row / rows_per_mod : 0;
-        const __nv_bfloat16* sc = mod_scale + mrow * dim + t * V;
-        const __nv_bfloat16* sh = mod_shift + mrow * dim + t * V;
-#pragma unroll
-        for (int k = 0; k < ITEMS; ++k) {
-            if (FULL || t * V + k * 8 < dim) {
-                // packed bf16 arithmetic gives exactly the roundings of the separate ops: a product of two
-                // bf16 values is exact in fp32, and a sum of two is either exact in fp32 or so lopsided that
-                // both roundings return the larger operand; _rn keeps multiply and add from fusing
-                const uint4 s8 = *reinterpret_cast<const uint4*>(sc + k * 8);
-                const uint4 h8 = *reinterpret_cast<const uint4*>(sh + k * 8);
-                const __nv_bfloat162 one2 = __floats2bfloat162_rn(1.0f, 1.0f);
-#pragma unroll
-                for (int j = 0; j < 8; j += 2) {
-                    const uint32_t sw = j == 0 ? s8.x : (j == 2 ? s8.y : (j == 4 ? s8.z : s8.w));
-                    const uint32_t hw = j == 0 ? h8.x : (j == 2 ? h8.y : (j == 4 ? h8.z : h8.w));
-                    const float2 xr2 = fmul2(make_float2(v[k * 8 + j], v[k * 8 + j + 1]), make_float2(rr, rr));
-                    const __nv_bfloat162 n = __floats2bfloat162_rn(xr2.x, xr2.y);
-                    const __nv_bfloat162 m1 = __hadd2_rn(one2, *reinterpret_cast<const __nv_bfloat162*>(&sw));
-                    const __nv_bfloat162 u = __hadd2_rn(__hmul2_rn(n, m1), *reinterpret_cast<const __nv_bfloat162*>(&hw));
-                    const uint32_t uw = *reinterpret_cast<const uint32_t*>(&u);
-                    v[k * 8 + j] = __uint_as_float(uw << 16);
-                    v[k * 8 + j + 1] = __uint_as_float(uw & 0xffff0000u);
-                }
-            }
-        }
-    }
-    butterfly_consecutive<V>(v);
-
-    if constexpr (B1 > 0) {
-        __syncthreads();                                       // everyone has read the raw staging area
-        exchange_write<L0, V>(xch, v, t);
-        __syncthreads();
-        exchange_read<L1, V>(xch, v, t);
-        butterfly_groups<L1, V>(v);
-    }
-    if constexpr (B2 > 0) {
-        __syncthreads();
-        exchange_write<L1, V>(xch, v, t);
-        __syncthreads();
-        exchange_read<L2, V>(xch, v, t);
-        butterfly_groups<L2, V>(v);
-    }
-    using LF = std::conditional_t<(B2 > 0), L2, std::conditional_t<(B1 > 0), L1, L0>>;
+    using LF = std::conditional_t<(B2 > 0), L2, L1>;
     constexpr int C = LF::C;
-    constexpr int PIECE = C < 8 ? C : 8;                       // elements per store; dim % 8 == 0 so a piece never straddles dim
+    static_assert(C >= 2 && C <= 8, "runs of 2, 4 or 8 elements");
+    constexpr bool IN8 = sizeof(Tin) == 1;
+    constexpr int CPB = IN8 ? 8 : 16;                          // bytes per copy: 8 elements, so a copy never straddles dim
+    constexpr int ITEMS = V / 8;                               // copies per thread and row
+    constexpr int CPT = V * (int)sizeof(Tin) / 16;             // 16-byte chunks per thread and row
+    constexpr int W = T < 32 ? T : 32;                         // threads of a row within one warp: they copy what they read
 
-    const float2 sc2 = make_float2(scale, scale);
+    extern __shared__ __align__(16) char stream_smem[];
+    __shared__ float red[8];
+    const int tu = threadIdx.x % UNIT;
+    const int unit = threadIdx.x / UNIT;
+    const int t = tu % T;
+    const int r_in = tu / T;
+    char* raw = stream_smem + unit * Geo::RAW + r_in * (N * (int)sizeof(Tin));
+    char* xch = stream_smem + Geo::UNITS * Geo::RAW + unit * Geo::XCH + r_in * Geo::XROW;
+    const uint32_t raw_addr = (uint32_t)__cvta_generic_to_shared(raw);
+    const unsigned mod = NORM_MOD ? blockIdx.x / blocks_per_mod : 0u;
+    const unsigned blk = NORM_MOD ? blockIdx.x - mod * blocks_per_mod : blockIdx.x;
+    const unsigned first = mod * rows_per_mod;
+    const unsigned count = NORM_MOD ? (rows - first < rows_per_mod ? rows - first : rows_per_mod) : rows;   // rows of this group
+    const unsigned step = (NORM_MOD ? blocks_per_mod : gridDim.x) * (unsigned)(Geo::UNITS * RPU);
+    unsigned rel = (blk * (unsigned)Geo::UNITS + (unsigned)unit) * (unsigned)RPU;   // first row of this unit, relative to the group
+
+    auto load_rows = [&](unsigned rel0) {
+        const bool ok = rel0 + r_in < count;
+        const Tin* xr = x + (int64_t)(ok ? first + rel0 + r_in : first) * x_row_stride;
 #pragma unroll
-    for (int i = 0; i < V; i += 2) {
-        const float2 m = fmul2(make_float2(v[i], v[i + 1]), sc2);
-        v[i] = m.x; v[i + 1] = m.y;
+        for (int k = 0; k < ITEMS; ++k) {
+            const int item = (t / W) * (W * ITEMS) + k * W + t % W;
+            const bool valid = ok && (FULL || item * 8 < dim);
+            const int c = IN8 ? item >> 1 : item;
+            cp_async_zfill(raw_addr + ((uint32_t)raw_pos<CPT>(c) << 4) + (IN8 ? (uint32_t)(item & 1) << 3 : 0u),
+                           xr + (valid ? item * 8 : 0), CPB, valid);
+        }
+        cp_async_commit();
+    };
+    load_rows(rel);
+
+    __nv_bfloat16* mod_smem = reinterpret_cast<__nv_bfloat16*>(stream_smem + Geo::UNITS * (Geo::RAW + Geo::XCH));
+    if constexpr (NORM_MOD) {
+        // 1 + scale and shift rows of this CTA's batch entry, staged like the raw rows (bf16: CPT = V / 8)
+        const __nv_bfloat16* sc = mod_scale + (int64_t)mod * dim;
+        const __nv_bfloat16* sh = mod_shift + (int64_t)mod * dim;
+        const __nv_bfloat162 one2 = __floats2bfloat162_rn(1.0f, 1.0f);
+        for (int c = threadIdx.x; c < N / 8; c += Geo::THREADS) {
+            uint4 s8 = make_uint4(0, 0, 0, 0), h8 = make_uint4(0, 0, 0, 0);
+            if (FULL || c * 8 < dim) {
+                s8 = *reinterpret_cast<const uint4*>(sc + c * 8);
+                h8 = *reinterpret_cast<const uint4*>(sh + c * 8);
+            }
+            uint32_t* w = &s8.x;
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const __nv_bfloat162 m1 = __hadd2_rn(one2, *reinterpret_cast<const __nv_bfloat162*>(w + j));
+                w[j] = *reinterpret_cast<const uint32_t*>(&m1);
+            }
+            reinterpret_cast<uint4*>(mod_smem)[raw_pos<CPT>(c)] = s8;
+            reinterpret_cast<uint4*>(mod_smem + N)[raw_pos<CPT>(c)] = h8;
+        }
+        __syncthreads();
     }
 
-    Tout* outr = out + row * (int64_t)dim;
-    if constexpr (EPI == Epilogue::Cast) {
+    for (; rel < count; rel += step) {
+        const unsigned row = first + rel + r_in;
+        const bool row_ok = rel + r_in < count;
+        cp_async_wait_all();
+        __syncwarp();                                          // the row has landed; the exchange of the row before has been read
+        float v[V];
 #pragma unroll
-        for (int j = 0; j < LF::G; ++j) {
-            const int e = LF::elem(t, j);
+        for (int k = 0; k < ITEMS; ++k) {
+            if constexpr (IN8) {
+                if (k % 2 == 0) {
+                    const uint4 u = *reinterpret_cast<const uint4*>(raw + (raw_pos<CPT>(t * CPT + k / 2) << 4));
+                    const uint32_t w[4] = {u.x, u.y, u.z, u.w};
 #pragma unroll
-            for (int pc = 0; pc < C / PIECE; ++pc) {
-                if (row_ok && (FULL || e + pc * PIECE < dim)) {
-                    float o[PIECE];
+                    for (int i = 0; i < 4; ++i) {
+                        float f[4];
+                        e4m3x4_to_float(w[i], f);
 #pragma unroll
-                    for (int i = 0; i < PIECE; ++i) o[i] = v[j * C + pc * PIECE + i];
-                    store_elems<Tout, PIECE>(outr + e + pc * PIECE, o);
-                }
-            }
-        }
-    } else {
-        // round to the input dtype (what the unfused chain stores), then the row's absmax
-        float amax = 0.f;
-#pragma unroll
-        for (int j = 0; j < LF::G; ++j) {
-            const bool in = FULL || LF::elem(t, j) < dim;      // dim % 8 == 0: a run of <= 8 is all in or all out
-            float m = 0.f;
-#pragma unroll
-            for (int i = 0; i < C; i += 2) {
-                const float2 rt = round_through2<Tin>(v[j * C + i], v[j * C + i + 1]);
-                v[j * C + i] = rt.x;
-                v[j * C + i + 1] = rt.y;
-                if (FULL || C <= 8 || LF::elem(t, j) + (i & ~7) < dim) m = fmaxf(m, fmaxf(fabsf(rt.x), fabsf(rt.y)));
-            }
-            if (C > 8 || in) amax = fmaxf(amax, m);
-        }
-        // reduce over the T threads of the row
-#pragma unroll
-        for (int m = 1; m < (T < 32 ? T : 32); m <<= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, m));
-        if constexpr (T > 32) {
-            constexpr int WPR = T / 32;                        // warps per row
-            if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = amax;
-            __syncthreads();
-            amax = red[r_in_cta * WPR];
-#pragma unroll
-            for (int k = 1; k < WPR; ++k) amax = fmaxf(amax, red[r_in_cta * WPR + k]);
-        }
-        const float qmax = std::is_same_v<Tout, int8_t> ? 127.0f : 448.0f;
-        const float qscale = __fdiv_rn(qmax, amax);
-        if (row_ok && t == 0) scales[row] = __fdiv_rn(1.0f, qscale);
-        const float qmul = amax == 0.f ? 0.f : qscale;         // an all-zero row quantises to zeros (0 * 0, not 0 * inf)
-#pragma unroll
-        for (int j = 0; j < LF::G; ++j) {
-            const int e = LF::elem(t, j);
-#pragma unroll
-            for (int pc = 0; pc < C / PIECE; ++pc) {
-                if (row_ok && (FULL || e + pc * PIECE < dim)) {
-                    using BV = typename ByteVec<PIECE>::type;
-                    union { BV vec; uint8_t b[PIECE]; uint32_t w[PIECE >= 4 ? PIECE / 4 : 1]; } u;
-                    const float2 q2 = make_float2(qmul, qmul);
-                    if constexpr (PIECE >= 4) {
-#pragma unroll
-                        for (int i = 0; i < PIECE; i += 4) {
-                            const float2 y0 = fmul2(make_float2(v[j * C + pc * PIECE + i], v[j * C + pc * PIECE + i + 1]), q2);
-                            const float2 y1 = fmul2(make_float2(v[j * C + pc * PIECE + i + 2], v[j * C + pc * PIECE + i + 3]), q2);
-                            u.w[i / 4] = quantize_pack4<Tout>(y0.x, y0.y, y1.x, y1.y);
-                        }
-                    } else {
-#pragma unroll
-                        for (int i = 0; i < PIECE; i += 2) {
-                            const float2 y = fmul2(make_float2(v[j * C + pc * PIECE + i], v[j * C + pc * PIECE + i + 1]), q2);
-                            u.b[i] = quantize_fast<Tout>(y.x);
-                            u.b[i + 1] = quantize_fast<Tout>(y.y);
-                        }
+                        for (int j = 0; j < 4; ++j) v[k * 8 + i * 4 + j] = f[j];
                     }
-                    *reinterpret_cast<BV*>(reinterpret_cast<uint8_t*>(outr) + e + pc * PIECE) = u.vec;
+                }
+            } else {
+                const uint4 u = *reinterpret_cast<const uint4*>(raw + (raw_pos<CPT>(t * CPT + k) << 4));
+                const uint32_t w[4] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    v[k * 8 + 2 * i] = __uint_as_float(w[i] << 16);
+                    v[k * 8 + 2 * i + 1] = __uint_as_float(w[i] & 0xffff0000u);
                 }
             }
         }
+        if constexpr (NORM_MOD) {
+            // rows of up to 2048 elements: partial sums of 32 elements; longer rows: of 64.  Then a tree over the
+            // partial sums of 1024 (2048) elements each, and those in sequence.
+            constexpr int PS = T <= 32 ? 32 : 64;
+            float ss = 0.f;
+#pragma unroll
+            for (int i = 0; i < PS; ++i) ss = fmaf(v[i], v[i], ss);
+            if constexpr (PS == 32) {
+                float ss1 = 0.f;
+#pragma unroll
+                for (int i = 32; i < 64; ++i) ss1 = fmaf(v[i], v[i], ss1);
+                ss += ss1;
+            }
+#pragma unroll
+            for (int m = 1; m < W; m <<= 1) ss += __shfl_xor_sync(0xffffffffu, ss, m);
+            if constexpr (T > 32) {
+                if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = ss;
+                __syncthreads();
+                ss = red[0];
+#pragma unroll
+                for (int k = 1; k < T / 32; ++k) ss += red[k];
+            }
+            const float rr = rsqrtf(ss * (1.0f / (float)dim));
+#pragma unroll
+            for (int k = 0; k < ITEMS; ++k) {
+                // packed bf16 arithmetic gives exactly the roundings of the separate ops: a product of two bf16
+                // values is exact in fp32, and a sum of two is either exact in fp32 or so lopsided that both
+                // roundings return the larger operand; _rn keeps multiply and add from fusing.  (Elements beyond
+                // dim are zero in x and in both rows, and stay zero.)
+                const int pos = raw_pos<CPT>(t * CPT + k);
+                const uint4 s8 = reinterpret_cast<const uint4*>(mod_smem)[pos];
+                const uint4 h8 = reinterpret_cast<const uint4*>(mod_smem + N)[pos];
+                const uint32_t sw[4] = {s8.x, s8.y, s8.z, s8.w}, hw[4] = {h8.x, h8.y, h8.z, h8.w};
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const float2 xr2 = fmul2(make_float2(v[k * 8 + 2 * i], v[k * 8 + 2 * i + 1]), make_float2(rr, rr));
+                    const __nv_bfloat162 n = __floats2bfloat162_rn(xr2.x, xr2.y);
+                    const __nv_bfloat162 u = __hadd2_rn(__hmul2_rn(n, *reinterpret_cast<const __nv_bfloat162*>(sw + i)),
+                                                        *reinterpret_cast<const __nv_bfloat162*>(hw + i));
+                    const uint32_t uw = *reinterpret_cast<const uint32_t*>(&u);
+                    v[k * 8 + 2 * i] = __uint_as_float(uw << 16);
+                    v[k * 8 + 2 * i + 1] = __uint_as_float(uw & 0xffff0000u);
+                }
+            }
+        }
+        butterfly_consecutive<V>(v);
+        xch_access<L0, PAD8, true>(xch, v, t);
+        __syncwarp();
+        load_rows(rel + step);                                 // this warp has read its part of the staging buffer
+        xch_access<L1, PAD8, false>(xch, v, t);
+        butterfly_groups<L1, V>(v);
+        if constexpr (B2 > 0) {
+            xch_access<L1, PAD8, true>(xch, v, t);             // a thread overwrites what it alone has read
+            __syncthreads();
+            xch_access<L2, PAD8, false>(xch, v, t);
+            butterfly_groups<L2, V>(v);
+        }
+
+        const float2 sc2 = make_float2(scale, scale);
+#pragma unroll
+        for (int i = 0; i < V; i += 2) {
+            const float2 m = fmul2(make_float2(v[i], v[i + 1]), sc2);
+            v[i] = m.x; v[i + 1] = m.y;
+        }
+        Tout* outr = out + (int64_t)row * dim;
+        if constexpr (EPI == Epilogue::Cast) {
+            if constexpr (std::is_same_v<Tout, __nv_bfloat16>) {
+#pragma unroll
+                for (int j = 0; j < LF::G; ++j) {
+                    const int e = LF::elem(t, j);
+                    float o[C];
+#pragma unroll
+                    for (int i = 0; i < C; ++i) o[i] = v[j * C + i];
+                    if (row_ok && (FULL || e < dim)) store_elems<Tout, C>(outr + e, o);
+                }
+            } else {
+                static_assert(std::is_same_v<Tout, e4m3_t>, "cast to bf16 or e4m3");
+#pragma unroll
+                for (int f = 0; f < V; f += 8) {
+                    float o[8];
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) o[i] = v[f + i];
+                    union { uint2 w; typename ByteVec<C>::type b[8 / C]; } u;
+                    u.w = pack8_e4m3_c10(o);
+#pragma unroll
+                    for (int g = 0; g < 8 / C; ++g) {
+                        const int e = LF::elem(t, f / C + g);
+                        if (row_ok && (FULL || e < dim))
+                            *reinterpret_cast<typename ByteVec<C>::type*>(reinterpret_cast<uint8_t*>(outr) + e) = u.b[g];
+                    }
+                }
+            }
+        } else {
+            // Round to the input dtype (what the unfused chain stores) and take the row's absmax on the packed
+            // values: bf16 pairs, or e4m3 bytes widened to fp16 pairs (exact).  NaNs do not count, as with fmaxf.
+            uint32_t pk[V / (IN8 ? 4 : 2)];
+            float amax;
+            if constexpr (IN8) {
+                __half2 m2 = __floats2half2_rn(0.f, 0.f);
+#pragma unroll
+                for (int f = 0; f < V; f += 8) {
+                    float o[8];
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) o[i] = v[f + i];
+                    const uint2 w = pack8_e4m3_c10(o);
+                    pk[f / 4] = w.x;
+                    pk[f / 4 + 1] = w.y;
+#pragma unroll
+                    for (int g = 0; g < 4; ++g) {
+                        const uint32_t ww = g < 2 ? w.x : w.y;
+                        const __half2_raw h = __nv_cvt_fp8x2_to_halfraw2((__nv_fp8x2_storage_t)(g & 1 ? ww >> 16 : ww & 0xffffu), __NV_E4M3);
+                        if (FULL || LF::elem(t, (f + 2 * g) / C) < dim) m2 = __hmax2(m2, __habs2(__half2(h)));
+                    }
+                }
+                amax = fmaxf(__low2float(m2), __high2float(m2));
+            } else {
+                __nv_bfloat162 m2 = __floats2bfloat162_rn(0.f, 0.f);
+#pragma unroll
+                for (int f = 0; f < V; f += 2) {
+                    const __nv_bfloat162 w = __floats2bfloat162_rn(v[f], v[f + 1]);
+                    pk[f / 2] = *reinterpret_cast<const uint32_t*>(&w);
+                    if (FULL || LF::elem(t, f / C) < dim) m2 = __hmax2(m2, __habs2(w));
+                }
+                amax = fmaxf(__low2float(m2), __high2float(m2));
+            }
+#pragma unroll
+            for (int m = 1; m < (T < 32 ? T : 32); m <<= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, m));
+            if constexpr (T > 32) {
+                if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = amax;
+                __syncthreads();
+                amax = red[0];
+#pragma unroll
+                for (int k = 1; k < T / 32; ++k) amax = fmaxf(amax, red[k]);
+            }
+            const float qmax = std::is_same_v<Tout, int8_t> ? 127.0f : 448.0f;
+            const float qscale = __fdiv_rn(qmax, amax);
+            if (row_ok && t == 0) scales[row] = __fdiv_rn(1.0f, qscale);
+            const float qmul = amax == 0.f ? 0.f : qscale;     // an all-zero row quantises to zeros (0 * 0, not 0 * inf)
+            const float2 q2 = make_float2(qmul, qmul);
+            constexpr int P = C < 4 ? C : 4;                   // values per packing step
+#pragma unroll
+            for (int j = 0; j < LF::G; ++j) {
+                const int e = LF::elem(t, j);
+                union { typename ByteVec<C>::type b; uint32_t w[C >= 4 ? C / 4 : 1]; } u;
+#pragma unroll
+                for (int i = 0; i < C; i += P) {
+                    float y[4];
+#pragma unroll
+                    for (int h = 0; h < P; h += 2) {
+                        const int f = j * C + i + h;
+                        float2 a;
+                        if constexpr (IN8) {
+                            const uint32_t ww = pk[f / 4];
+                            const __half2_raw hr = __nv_cvt_fp8x2_to_halfraw2((__nv_fp8x2_storage_t)(f & 2 ? ww >> 16 : ww & 0xffffu), __NV_E4M3);
+                            a = __half22float2(__half2(hr));
+                        } else {
+                            a = make_float2(__uint_as_float(pk[f / 2] << 16), __uint_as_float(pk[f / 2] & 0xffff0000u));
+                        }
+                        a = fmul2(a, q2);
+                        // round half away from zero (C round()) of |y| < 2^22: adding the largest float below 0.5 with
+                        // y's sign and truncating gives floor(|y| + 0.5) for every fp32 y, ties included
+                        if constexpr (std::is_same_v<Tout, int8_t>)
+                            a = fadd2(a, make_float2(copysignf(0.49999997f, a.x), copysignf(0.49999997f, a.y)));
+                        y[h] = a.x;
+                        y[h + 1] = a.y;
+                    }
+                    uint32_t w;
+                    if constexpr (std::is_same_v<Tout, int8_t>) {
+                        w = __byte_perm((uint32_t)__float2int_rz(y[0]), (uint32_t)__float2int_rz(y[1]), 0x0040);
+                        if constexpr (P == 4)
+                            w = __byte_perm(w, __byte_perm((uint32_t)__float2int_rz(y[2]), (uint32_t)__float2int_rz(y[3]), 0x0040), 0x5410);
+                    } else {
+                        // |y| <= 448 (1 + 2^-23) for finite rows, where the saturating cast and the c10 cast (overflow ->
+                        // NaN beyond 464) agree; a NaN stays a NaN in both
+                        w = (uint32_t)float2_to_e4m3x2_sat(y[0], y[1]);
+                        if constexpr (P == 4) w |= (uint32_t)float2_to_e4m3x2_sat(y[2], y[3]) << 16;
+                    }
+                    u.w[i / 4] = w;
+                }
+                if (row_ok && (FULL || e < dim))
+                    *reinterpret_cast<typename ByteVec<C>::type*>(reinterpret_cast<uint8_t*>(outr) + e) = u.b;
+            }
+        }
+        // the other warps have read the exchange before it is overwritten (with a quantizer: the absmax barrier)
+        if constexpr (T > 32 && EPI == Epilogue::Cast) __syncthreads();
     }
+    cp_async_wait_all();                                       // (the copies behind the last row were empty)
+}
+
+template <typename Tin, typename Tout, int LOG_N, Epilogue EPI, bool NORM_MOD>
+static int launch_stream(const Tin* x, Tout* out, float* scales, int64_t rows, int dim, int64_t stride, float scale,
+                         const __nv_bfloat16* ms, const __nv_bfloat16* mh, int64_t rows_per_mod, cudaStream_t st) {
+    using Geo = StreamGeo<Tin, LOG_N, NORM_MOD>;
+    auto kern = dim == Geo::N ? hadamard_stream_kernel<Tin, Tout, LOG_N, EPI, NORM_MOD, true>
+                              : hadamard_stream_kernel<Tin, Tout, LOG_N, EPI, NORM_MOD, false>;
+    if (Geo::SMEM > 47 * 1024)                                 // (with the static reduction words, above the 48 KB default)
+        Q8K_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Geo::SMEM));
+    const int64_t slots = (int64_t)gemm_num_sms() * Geo::CTAS;
+    constexpr int per_cta = Geo::UNITS * Geo::RPU;
+    int64_t groups = 1, group_rows = rows;
+    if (NORM_MOD) {
+        group_rows = rows_per_mod < rows ? rows_per_mod : rows;
+        groups = (rows + group_rows - 1) / group_rows;
+    }
+    const int64_t need = (group_rows + per_cta - 1) / per_cta;
+    int64_t blocks = slots / groups < 1 ? 1 : slots / groups;
+    if (blocks > need) blocks = need;
+    kern<<<(unsigned)(blocks * groups), Geo::THREADS, Geo::SMEM, st>>>(x, out, scales, (unsigned)rows, dim, stride, scale, ms, mh,
+                                                                      (unsigned)group_rows, (unsigned)blocks);
+    Q8K_CUDA_OK(cudaGetLastError());
+    return Q8K_OK;
 }
 
 // ------------------------------------------------------------------ dispatch
@@ -532,28 +627,12 @@ static int launch_hadamard(const void* x, void* out, float* scales, int64_t rows
         switch (log_g) { Q8K_HS(0); Q8K_HS(1); Q8K_HS(2); Q8K_HS(3); Q8K_HS(4); Q8K_HS(5); }
 #undef Q8K_HS
     } else {
-        if (log_n > 14) { set_error_detail("%s: dim %d exceeds 16384", op, dim); return Q8K_ERR_UNSUPPORTED; }
-#define Q8K_HR(LN, LV, NR)                                                                                \
-    case LN: {                                                                                            \
-        auto kern = dim == (1 << LN) ? hadamard_row_kernel<Tin, Tout, LN, LV, NR, EPI, false, true>       \
-                                     : hadamard_row_kernel<Tin, Tout, LN, LV, NR, EPI, false, false>;     \
-        constexpr int smem = NR * (1 << LN) * (int)sizeof(float);                                         \
-        if (smem > 48 * 1024)                                                                             \
-            Q8K_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));   \
-        kern<<<(unsigned)((rows + NR - 1) / NR), NR << (LN - LV), smem, st>>>(xi, o, scales, rows, dim, stride, scale, nullptr, nullptr, 1); \
-    } break
-        // (row length, values per thread, rows per CTA), chosen by measurement: the plain transform
-        // likes more values per thread (fewer exchanges), the fused quantizer more threads
-        if constexpr (EPI == Epilogue::Cast) {
-            switch (log_n) {
-                Q8K_HR(9, 5, 8); Q8K_HR(10, 6, 8); Q8K_HR(11, 6, 4); Q8K_HR(12, 6, 2); Q8K_HR(13, 6, 1); Q8K_HR(14, 7, 1);
-            }
-        } else {
-            switch (log_n) {
-                Q8K_HR(9, 5, 8); Q8K_HR(10, 5, 4); Q8K_HR(11, 5, 2); Q8K_HR(12, 6, 2); Q8K_HR(13, 6, 1); Q8K_HR(14, 7, 1);
-            }
+#define Q8K_HS(LN) case LN: return launch_stream<Tin, Tout, LN, EPI, false>(xi, o, scales, rows, dim, stride, scale, nullptr, nullptr, 1, st)
+        switch (log_n) {
+            Q8K_HS(9); Q8K_HS(10); Q8K_HS(11); Q8K_HS(12); Q8K_HS(13); Q8K_HS(14);
+            default: set_error_detail("%s: dim %d exceeds 16384", op, dim); return Q8K_ERR_UNSUPPORTED;
         }
-#undef Q8K_HR
+#undef Q8K_HS
     }
     Q8K_CUDA_OK(cudaGetLastError());
     return Q8K_OK;
@@ -569,22 +648,12 @@ static int launch_norm_mod_quant(const void* x, const void* mod_scale, const voi
     const __nv_bfloat16* ms = (const __nv_bfloat16*)mod_scale;
     const __nv_bfloat16* mh = (const __nv_bfloat16*)mod_shift;
     Tout* o = (Tout*)q;
-#define Q8K_NM(LN, LV, NR)                                                                                \
-    case LN: {                                                                                            \
-        auto kern = dim == (1 << LN) ? hadamard_row_kernel<__nv_bfloat16, Tout, LN, LV, NR, Epilogue::Quant, true, true>  \
-                                     : hadamard_row_kernel<__nv_bfloat16, Tout, LN, LV, NR, Epilogue::Quant, true, false>; \
-        constexpr int smem = NR * (1 << LN) * (int)sizeof(float);                                         \
-        if (smem > 48 * 1024)                                                                             \
-            Q8K_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));   \
-        kern<<<(unsigned)((rows + NR - 1) / NR), NR << (LN - LV), smem, st>>>(xi, o, scales, rows, dim, dim, scale, ms, mh, rows_per_mod); \
-    } break
+#define Q8K_NM(LN) case LN: return launch_stream<__nv_bfloat16, Tout, LN, Epilogue::Quant, true>(xi, o, scales, rows, dim, dim, scale, ms, mh, rows_per_mod, st)
     switch (log_n) {
-        Q8K_NM(9, 5, 8); Q8K_NM(10, 5, 4); Q8K_NM(11, 5, 2); Q8K_NM(12, 6, 2); Q8K_NM(13, 6, 1);
+        Q8K_NM(9); Q8K_NM(10); Q8K_NM(11); Q8K_NM(12); Q8K_NM(13);
         default: set_error_detail("norm_modulate_quant: dim %d not in [512, 8192]", dim); return Q8K_ERR_UNSUPPORTED;
     }
 #undef Q8K_NM
-    Q8K_CUDA_OK(cudaGetLastError());
-    return Q8K_OK;
 }
 
 static int check_hadamard_args(const char* op, const void* x, int x_dtype, const void* out, int64_t rows,

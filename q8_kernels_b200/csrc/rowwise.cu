@@ -179,12 +179,6 @@ rope_kernel(const Tin* __restrict__ x, const float* __restrict__ cosf_, const fl
 
 // fma_kernel (csrc/ops/fma_cuda.cu:92-95).  16 elements per thread (one 16-byte load of x and one store),
 // e4m3 -> fp32 through the packed e4m3x2 -> f16x2 conversion, the c10 cast eight values at a time.
-__device__ __forceinline__ void e4m3x4_to_float(uint32_t w, float (&o)[4]) {
-    const __half2_raw lo = __nv_cvt_fp8x2_to_halfraw2((__nv_fp8x2_storage_t)(w & 0xffffu), __NV_E4M3);
-    const __half2_raw hi = __nv_cvt_fp8x2_to_halfraw2((__nv_fp8x2_storage_t)(w >> 16), __NV_E4M3);
-    const float2 a = __half22float2(__half2(lo)), c = __half22float2(__half2(hi));
-    o[0] = a.x; o[1] = a.y; o[2] = c.x; o[3] = c.y;
-}
 template <typename Ty, typename Tz, int T>
 __global__ void __launch_bounds__(T)
 fma_kernel(const e4m3_t* __restrict__ x, const Ty* __restrict__ y, const Tz* __restrict__ z,

@@ -189,6 +189,26 @@ def test_norm_modulate_quant_matches_unfused_chain(q8, cuda_device):
     assert ((q.int() - qd.int()).abs() != 0).float().mean().item() < 0.01
 
 
+@pytest.mark.parametrize("B,S,C", [(3, 5, 512), (1, 4801, 1024), (2, 901, 2048), (2, 901, 1552), (5, 33, 4096), (3, 201, 8192),
+                                   (700, 1, 2048)])
+def test_norm_modulate_quant_groups_and_turns(q8, cuda_device, B, S, C):
+    """Every batch entry keeps to its own modulation rows, over group tails, several turns of a CTA, ragged dims and
+    more entries than the grid has CTAs: against the op chain on the device (the mean square is summed in another
+    order there, so a code may move by one where a bf16 rounding tips)."""
+    import math
+    d = cuda_device
+    g = Hp.gen(S + C)
+    x = Hp.activations(B * S, C, seed=C).reshape(B, S, C).to(d)
+    sc = torch.randn(B, 1, C, generator=g).to(torch.bfloat16).to(d)
+    sh = torch.randn(B, 1, C, generator=g).to(torch.bfloat16).to(d)
+    q, s = q8.native.norm_modulate_quant(x, sc, sh)
+    n = q8.native.rms_norm(x, None, torch.bfloat16)[0]
+    qd, sd = q8.native.hadamard_quant(n * (1 + sc) + sh, 1 / math.sqrt(C), torch.int8)
+    diff = (q.int() - qd.int()).abs()
+    assert diff.max().item() <= 1 and (diff != 0).float().mean().item() < 0.01
+    assert torch.allclose(s, sd, rtol=1e-2)
+
+
 @pytest.mark.parametrize("kind", ["int8", "fp8"])
 @pytest.mark.parametrize("with_gate", [True, False])
 @pytest.mark.parametrize("M,N,K", [(200, 512, 256), (384, 2048, 2048), (96, 128, 128), (300, 272, 192), (515, 1040, 320)])

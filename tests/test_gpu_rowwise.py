@@ -106,6 +106,34 @@ def test_fused_hadamard_quant_equals_chain(nat, cuda_device, rows, dim, q_dtype)
     Hp.assert_bit_equal(s, s2.cpu(), "fused vs chain scales")
 
 
+@pytest.mark.parametrize("rows,dim", [(9475, 512), (4737, 1024), (2371, 2048), (2371, 1544), (1187, 4096), (595, 8192),
+                                      (595, 6008), (299, 16384), (299, 10248)])
+def test_long_rows_stream_through_a_full_grid(nat, cuda_device, rows, dim):
+    """A few rows more than the CTAs of one full grid hold at once: the second turn of a CTA, the tail of the last
+    group of rows, power-of-two and ragged dims, e4m3 rows that start on 8-byte boundaries only, strided rows."""
+    x = Hp.activations(rows, dim, seed=rows, outliers=True)
+    x[rows - 1] *= 1e-30
+    x[0] = 0
+    s = 1.0 / math.sqrt(dim)
+    wide = torch.zeros(rows, dim + 24, dtype=torch.bfloat16)
+    wide[:, :dim] = x
+    xd = wide.to(cuda_device)[:, :dim]
+    h_ref = O.hadamard_transform(x, scale=s)
+    Hp.assert_bit_equal(nat.fast_hadamard_transform(xd, s, None), h_ref, "bf16 rows")
+    for qt in (torch.int8, E4M3):
+        q_ref, s_ref = O.tokenwise_quant(h_ref, qt)
+        q, sc = nat.hadamard_quant(xd, s, qt)
+        Hp.assert_bit_equal(q, q_ref, f"rows {qt}")
+        Hp.assert_bit_equal(sc, s_ref, f"scales {qt}")
+    x8 = O.c10_e4m3(x.float() * 0.05)
+    h8 = O.hadamard_transform(x8, scale=s)
+    Hp.assert_bit_equal(nat.fast_hadamard_transform(x8.to(cuda_device), s, None), h8, "e4m3 rows")
+    q_ref, s_ref = O.tokenwise_quant(h8, torch.int8)
+    q, sc = nat.hadamard_quant(x8.to(cuda_device), s, torch.int8)
+    Hp.assert_bit_equal(q, q_ref, "e4m3 in, int8 rows")
+    Hp.assert_bit_equal(sc, s_ref, "e4m3 in, scales")
+
+
 def test_fused_hadamard_quant_e4m3_input(nat, cuda_device):
     # the e4m3 attention output feeding to_out: intermediate is rounded to e4m3 (c10 cast)
     x8 = O.c10_e4m3(torch.randn(20, 2048, generator=Hp.gen(8)) * 0.5)
