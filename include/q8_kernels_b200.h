@@ -225,6 +225,15 @@ Q8K_API int q8k_attention_prep(const void* q, const void* k, const void* v,
                        int64_t k_stride_b, int64_t k_stride_s, int64_t k_stride_h,
                        int64_t v_stride_b, int64_t v_stride_s, int64_t v_stride_h,
                        int apply_hadamard, float qk_scale, void* stream);
+/* The same with V cast to rows v8 [B,H,S_kv,64] (what q8k_flash_attention_v_rows reads) instead of transposed:
+ * one launch for all three tensors.                                                                        */
+Q8K_API int q8k_attention_prep_rows(const void* q, const void* k, const void* v,
+                       void* q8, void* k8, void* v8,
+                       int B, int H, int S_q, int S_kv,
+                       int64_t q_stride_b, int64_t q_stride_s, int64_t q_stride_h,
+                       int64_t k_stride_b, int64_t k_stride_s, int64_t k_stride_h,
+                       int64_t v_stride_b, int64_t v_stride_s, int64_t v_stride_h,
+                       int apply_hadamard, float qk_scale, void* stream);
 
 /* Q or K after its projection, in one pass per tensor: RMS norm over all H*64 channels with the fp32
  * weight norm_w (result rounded to bf16), optional rotary embedding with fp32 tables [S, H*64] shared

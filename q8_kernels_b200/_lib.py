@@ -54,6 +54,7 @@ SIGNATURES = {
     "q8k_flash_attention_strided": (_c_int, [_c_ptr, _c_ptr, _c_ptr, _c_ptr, _c_int, _c_int, _c_int, _c_int, _c_int,
                                              _c_i64, _c_i64, _c_i64, _c_f32, _c_ptr, _c_ptr, _c_ptr]),
     "q8k_attention_prep": (_c_int, [_c_ptr] * 6 + [_c_int] * 4 + [_c_i64] * 9 + [_c_int, _c_f32, _c_ptr]),
+    "q8k_attention_prep_rows": (_c_int, [_c_ptr] * 6 + [_c_int] * 4 + [_c_i64] * 9 + [_c_int, _c_f32, _c_ptr]),
     "q8k_flash_attention_multi_out": (_c_int, [_c_ptr, _c_ptr, _c_ptr, _c_ptr, _c_int, _c_int, _c_int, _c_int, _c_int,
                                                _c_int, _c_i64, _c_i64, _c_i64, _c_f32, _c_ptr, _c_ptr, _c_ptr]),
     "q8k_flash_attention_v_rows": (_c_int, [_c_ptr, _c_ptr, _c_ptr, _c_ptr, _c_int, _c_int, _c_int, _c_int, _c_int,

@@ -623,52 +623,99 @@ flash_attn_fp8_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
 }
 
 // ------------------------------------------------------------------ pre-pass kernels
-// Q / K: one 64-element head row per group of 8 lanes; optional 64-point
-// Hadamard (fp32 butterflies, ascending stride), times `scale`, cast c10-style
-// to e4m3, written head-major [B,H,S,64].
+// Q, K and V as rows, in one launch: 64-element head rows, four lanes per row with 16 consecutive elements each;
+// optional 64-point Hadamard (fp32 butterflies, ascending stride: four stages in registers, two between lanes), times
+// `scale`, cast c10-style to e4m3, written head-major [B,H,S,64].  Rows are walked with the head index fastest, which
+// is the memory order of a [B,S,H*64] projection; a block takes 128 rows of one batch entry of one tensor and fetches
+// all of them before it computes.  Bound by memory: 3 bytes per element.  Measured, B = 2, H = 32, S = 6144 (Q, K and V,
+// 226 MB): 98 us as three launches of 8 lanes per row (64-bit row divisions, 3 shuffles per element) and a V
+// transpose -> 42 us (0.83 of the copy rate).
+struct PrepSeg {
+    const __nv_bfloat16* x;
+    uint8_t* out;
+    int64_t stride_b, stride_s, stride_h;
+    uint32_t H, S;
+    uint32_t step_h, step_s;                  // 32 rows further: h += step_h, s += step_s (and a carry)
+    uint32_t blocks_per_b;
+    uint32_t first_block;
+    float scale;
+    int hadamard;
+};
+struct PrepParams {
+    PrepSeg seg[3];
+    int n;
+};
+constexpr int kPrepRows = 128;                // rows per block: 4 passes of 32
 __global__ void __launch_bounds__(128)
-attn_prep_qk_kernel(const __nv_bfloat16* __restrict__ x, uint8_t* __restrict__ out, int B, int H, int S,
-                    int64_t stride_b, int64_t stride_s, int64_t stride_h, int apply_hadamard, float scale) {
+attn_prep_rows_kernel(const __grid_constant__ PrepParams p) {
+    int si = 0;
+    if (p.n > 1 && blockIdx.x >= p.seg[1].first_block) si = 1;
+    if (p.n > 2 && blockIdx.x >= p.seg[2].first_block) si = 2;
+    const PrepSeg& g = p.seg[si];
+    const uint32_t blk = blockIdx.x - g.first_block;
+    const uint32_t b = blk / g.blocks_per_b;
+    const uint32_t H = g.H, S = g.S;
     const int lane = threadIdx.x & 31;
-    const int sub = lane & 7;
-    const int64_t grp = (int64_t)blockIdx.x * 16 + (threadIdx.x >> 3);   // (b, s, h) flattened, h fastest
-    const int64_t total = (int64_t)B * S * H;
-    const bool row_ok = grp < total;
-    float v[8];
+    const int sub = lane & 3;
+    const uint32_t idx = (blk - b * g.blocks_per_b) * kPrepRows + (threadIdx.x >> 2);
+    uint32_t s = idx / H, h = idx - s * H;
+    const __nv_bfloat16* xb = g.x + (int64_t)b * g.stride_b + sub * 16;
+    uint8_t* ob = g.out + (int64_t)b * H * S * 64 + sub * 16;
+
+    uint4 raw[4][2];
+    int64_t off[4];                           // row of the output, -1 beyond the end
 #pragma unroll
-    for (int j = 0; j < 8; ++j) v[j] = 0.f;
-    int h = 0, s = 0, b = 0;
-    if (row_ok) {
-        h = (int)(grp % H);
-        s = (int)((grp / H) % S);
-        b = (int)(grp / ((int64_t)H * S));
-        load_vec<__nv_bfloat16, 8>(x + b * stride_b + s * stride_s + h * stride_h + sub * 8, v);
+    for (int it = 0; it < 4; ++it) {
+        off[it] = -1;
+        raw[it][0] = raw[it][1] = make_uint4(0, 0, 0, 0);
+        if (s < S) {
+            const __nv_bfloat16* xr = xb + (int64_t)s * g.stride_s + (int64_t)h * g.stride_h;
+            raw[it][0] = *reinterpret_cast<const uint4*>(xr);
+            raw[it][1] = *reinterpret_cast<const uint4*>(xr + 8);
+            off[it] = (int64_t)h * S + s;
+        }
+        h += g.step_h;
+        s += g.step_s;
+        if (h >= H) { h -= H; ++s; }
     }
-    if (apply_hadamard) {
 #pragma unroll
-        for (int st = 1; st < 8; st <<= 1) {
+    for (int it = 0; it < 4; ++it) {
+        float v[16];
+        const uint32_t w[8] = {raw[it][0].x, raw[it][0].y, raw[it][0].z, raw[it][0].w,
+                               raw[it][1].x, raw[it][1].y, raw[it][1].z, raw[it][1].w};
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                const int lo = j & (st - 1);
-                const int i = ((j - lo) << 1) + lo;
-                const float a = v[i], bb = v[i + st];
-                v[i] = __fadd_rn(a, bb);
-                v[i + st] = __fsub_rn(a, bb);
+        for (int j = 0; j < 8; ++j) {
+            v[2 * j] = __uint_as_float(w[j] << 16);
+            v[2 * j + 1] = __uint_as_float(w[j] & 0xffff0000u);
+        }
+        if (g.hadamard) {                     // uniform in the block
+            butterfly_consecutive<16>(v);
+#pragma unroll
+            for (int mk = 1; mk < 4; mk <<= 1) {
+                const float sg = (lane & mk) ? -1.f : 1.f;
+                const float2 sign = make_float2(sg, sg);
+#pragma unroll
+                for (int j = 0; j < 16; j += 2) {   // other - u for the upper lane, u + other for the lower: exact
+                    const float2 other = make_float2(__shfl_xor_sync(0xffffffffu, v[j], mk), __shfl_xor_sync(0xffffffffu, v[j + 1], mk));
+                    const float2 u = ffma2(sign, make_float2(v[j], v[j + 1]), other);
+                    v[j] = u.x;
+                    v[j + 1] = u.y;
+                }
+            }
+            const float2 sc = make_float2(g.scale, g.scale);
+#pragma unroll
+            for (int j = 0; j < 16; j += 2) {
+                const float2 u = fmul2(make_float2(v[j], v[j + 1]), sc);
+                v[j] = u.x;
+                v[j + 1] = u.y;
             }
         }
+        float lo[8], hi[8];
 #pragma unroll
-        for (int mk = 1; mk < 8; mk <<= 1) {
-            const bool upper = (lane & mk) != 0;
-#pragma unroll
-            for (int j = 0; j < 8; ++j) {
-                const float other = __shfl_xor_sync(0xffffffffu, v[j], mk);
-                v[j] = upper ? __fsub_rn(other, v[j]) : __fadd_rn(v[j], other);
-            }
-        }
-#pragma unroll
-        for (int j = 0; j < 8; ++j) v[j] = __fmul_rn(v[j], scale);
+        for (int j = 0; j < 8; ++j) { lo[j] = v[j]; hi[j] = v[8 + j]; }
+        const uint2 a = pack8_e4m3_c10(lo), c = pack8_e4m3_c10(hi);
+        if (off[it] >= 0) *reinterpret_cast<uint4*>(ob + off[it] * 64) = make_uint4(a.x, a.y, c.x, c.y);
     }
-    if (row_ok) *reinterpret_cast<uint2*>(out + (((int64_t)b * H + h) * S + s) * 64 + sub * 8) = pack8_e4m3_c10(v);
 }
 
 // Q / K after their projection, fused: RMS norm over all H*64 channels with an fp32 weight (bf16
@@ -993,6 +1040,33 @@ static int launch_flash_attention(bool v_rows, const void* q, const void* k, con
     return Q8K_OK;
 }
 
+// One launch over up to three [B,H,S,64] views; the caller has checked pointers and strides.
+struct PrepView { const void* x; void* out; int S; int64_t stride_b, stride_s, stride_h; int hadamard; float scale; };
+static int launch_prep_rows(const char* op, const PrepView* views, int n, int B, int H, cudaStream_t st) {
+    PrepParams p;
+    p.n = n;
+    int64_t blocks = 0;
+    for (int i = 0; i < n; ++i) {
+        const int64_t rows = (int64_t)views[i].S * H;
+        const int64_t per_b = (rows + kPrepRows - 1) / kPrepRows;
+        Q8K_REQUIRE(rows <= 0xffffff00LL && blocks + per_b * B <= 0x7fffffffLL, Q8K_ERR_TOO_LARGE, "%s: too many rows", op);
+        PrepSeg& g = p.seg[i];
+        g.x = (const __nv_bfloat16*)views[i].x;
+        g.out = (uint8_t*)views[i].out;
+        g.stride_b = views[i].stride_b; g.stride_s = views[i].stride_s; g.stride_h = views[i].stride_h;
+        g.H = (uint32_t)H; g.S = (uint32_t)views[i].S;
+        g.step_h = 32u % (uint32_t)H; g.step_s = 32u / (uint32_t)H;
+        g.blocks_per_b = (uint32_t)per_b;
+        g.first_block = (uint32_t)blocks;
+        g.scale = views[i].scale;
+        g.hadamard = views[i].hadamard;
+        blocks += per_b * B;
+    }
+    attn_prep_rows_kernel<<<(unsigned)blocks, 128, 0, st>>>(p);
+    Q8K_CUDA_OK(cudaGetLastError());
+    return Q8K_OK;
+}
+
 extern "C" int q8k_attention_cast_rows(const void* x, void* out8, int B, int H, int S, int64_t stride_b, int64_t stride_s,
                                        int64_t stride_h, void* stream) {
     const char* op = "attention_cast_rows";
@@ -1000,11 +1074,31 @@ extern "C" int q8k_attention_cast_rows(const void* x, void* out8, int B, int H, 
     Q8K_REQUIRE(B > 0 && H > 0 && S > 0, Q8K_ERR_INVALID_ARG, "%s: bad shape", op);
     Q8K_REQUIRE(stride_b % 8 == 0 && stride_s % 8 == 0 && stride_h % 8 == 0 && aligned16(x) && aligned16(out8),
                 Q8K_ERR_INVALID_ARG, "%s: strides must be multiples of 8 elements and pointers 16-byte aligned", op);
-    const int64_t rows = (int64_t)B * S * H;
-    Q8K_REQUIRE((rows + 15) / 16 <= 0x7fffffffLL, Q8K_ERR_TOO_LARGE, "%s: too many rows", op);
-    attn_prep_qk_kernel<<<(unsigned)((rows + 15) / 16), 128, 0, (cudaStream_t)stream>>>(
-        (const __nv_bfloat16*)x, (uint8_t*)out8, B, H, S, stride_b, stride_s, stride_h, 0, 1.0f);
-    Q8K_CUDA_OK(cudaGetLastError());
+    const PrepView v = {x, out8, S, stride_b, stride_s, stride_h, 0, 1.0f};
+    return launch_prep_rows(op, &v, 1, B, H, (cudaStream_t)stream);
+}
+
+static int attention_prep(const char* op, bool v_rows, const void* q, const void* k, const void* v, void* q8, void* k8,
+                          void* v8, int B, int H, int S_q, int S_kv, const int64_t (&st_q)[3], const int64_t (&st_k)[3],
+                          const int64_t (&st_v)[3], int apply_hadamard, float qk_scale, cudaStream_t st) {
+    Q8K_REQUIRE(q && k && v && q8 && k8 && v8, Q8K_ERR_INVALID_ARG, "%s: null pointer", op);
+    Q8K_REQUIRE(B > 0 && H > 0 && S_q > 0 && S_kv > 0, Q8K_ERR_INVALID_ARG, "%s: bad shape", op);
+    Q8K_REQUIRE((int64_t)B * H <= 65535, Q8K_ERR_TOO_LARGE, "%s: B*H exceeds 65535", op);
+    for (int i = 0; i < 3; ++i)
+        Q8K_REQUIRE(st_q[i] % 8 == 0 && st_k[i] % 8 == 0 && st_v[i] % 8 == 0, Q8K_ERR_INVALID_ARG,
+                    "%s: strides must be multiples of 8 elements", op);
+    Q8K_REQUIRE(aligned16(q) && aligned16(k) && aligned16(v) && aligned16(q8) && aligned16(k8) && aligned16(v8),
+                Q8K_ERR_INVALID_ARG, "%s: pointers must be 16-byte aligned", op);
+    const PrepView views[3] = {{q, q8, S_q, st_q[0], st_q[1], st_q[2], apply_hadamard, qk_scale},
+                               {k, k8, S_kv, st_k[0], st_k[1], st_k[2], apply_hadamard, qk_scale},
+                               {v, v8, S_kv, st_v[0], st_v[1], st_v[2], 0, 1.0f}};
+    if (int rc = launch_prep_rows(op, views, v_rows ? 3 : 2, B, H, st)) return rc;
+    if (!v_rows) {
+        dim3 grid((unsigned)((S_kv + 63) / 64), (unsigned)(B * H));
+        attn_prep_v_kernel<<<grid, 256, 0, st>>>((const __nv_bfloat16*)v, (uint8_t*)v8, H, S_kv, (S_kv + 15) / 16 * 16,
+                                                 st_v[0], st_v[1], st_v[2]);
+        Q8K_CUDA_OK(cudaGetLastError());
+    }
     return Q8K_OK;
 }
 
@@ -1014,35 +1108,20 @@ extern "C" int q8k_attention_prep(const void* q, const void* k, const void* v, v
                                   int64_t k_stride_b, int64_t k_stride_s, int64_t k_stride_h,
                                   int64_t v_stride_b, int64_t v_stride_s, int64_t v_stride_h,
                                   int apply_hadamard, float qk_scale, void* stream) {
-    const char* op = "attention_prep";
-    Q8K_REQUIRE(q && k && v && q8 && k8 && vt8, Q8K_ERR_INVALID_ARG, "%s: null pointer", op);
-    Q8K_REQUIRE(B > 0 && H > 0 && S_q > 0 && S_kv > 0, Q8K_ERR_INVALID_ARG, "%s: bad shape", op);
-    Q8K_REQUIRE((int64_t)B * H <= 65535, Q8K_ERR_TOO_LARGE, "%s: B*H exceeds 65535", op);
-    const int64_t all_strides[9] = {q_stride_b, q_stride_s, q_stride_h, k_stride_b, k_stride_s, k_stride_h,
-                                    v_stride_b, v_stride_s, v_stride_h};
-    for (int i = 0; i < 9; ++i)
-        Q8K_REQUIRE(all_strides[i] % 8 == 0, Q8K_ERR_INVALID_ARG, "%s: strides must be multiples of 8 elements", op);
-    Q8K_REQUIRE(aligned16(q) && aligned16(k) && aligned16(v) && aligned16(q8) && aligned16(k8) && aligned16(vt8),
-                Q8K_ERR_INVALID_ARG, "%s: pointers must be 16-byte aligned", op);
-    cudaStream_t st = (cudaStream_t)stream;
-    const int s_pad = (S_kv + 15) / 16 * 16;
-    {
-        const int64_t rows = (int64_t)B * S_q * H;
-        attn_prep_qk_kernel<<<(unsigned)((rows + 15) / 16), 128, 0, st>>>(
-            (const __nv_bfloat16*)q, (uint8_t*)q8, B, H, S_q, q_stride_b, q_stride_s, q_stride_h, apply_hadamard, qk_scale);
-    }
-    {
-        const int64_t rows = (int64_t)B * S_kv * H;
-        attn_prep_qk_kernel<<<(unsigned)((rows + 15) / 16), 128, 0, st>>>(
-            (const __nv_bfloat16*)k, (uint8_t*)k8, B, H, S_kv, k_stride_b, k_stride_s, k_stride_h, apply_hadamard, qk_scale);
-    }
-    {
-        dim3 grid((unsigned)((S_kv + 63) / 64), (unsigned)(B * H));
-        attn_prep_v_kernel<<<grid, 256, 0, st>>>((const __nv_bfloat16*)v, (uint8_t*)vt8, H, S_kv, s_pad,
-                                                 v_stride_b, v_stride_s, v_stride_h);
-    }
-    Q8K_CUDA_OK(cudaGetLastError());
-    return Q8K_OK;
+    return attention_prep("attention_prep", false, q, k, v, q8, k8, vt8, B, H, S_q, S_kv, {q_stride_b, q_stride_s, q_stride_h},
+                          {k_stride_b, k_stride_s, k_stride_h}, {v_stride_b, v_stride_s, v_stride_h}, apply_hadamard, qk_scale,
+                          (cudaStream_t)stream);
+}
+
+extern "C" int q8k_attention_prep_rows(const void* q, const void* k, const void* v, void* q8, void* k8, void* v8,
+                                       int B, int H, int S_q, int S_kv,
+                                       int64_t q_stride_b, int64_t q_stride_s, int64_t q_stride_h,
+                                       int64_t k_stride_b, int64_t k_stride_s, int64_t k_stride_h,
+                                       int64_t v_stride_b, int64_t v_stride_s, int64_t v_stride_h,
+                                       int apply_hadamard, float qk_scale, void* stream) {
+    return attention_prep("attention_prep_rows", true, q, k, v, q8, k8, v8, B, H, S_q, S_kv, {q_stride_b, q_stride_s, q_stride_h},
+                          {k_stride_b, k_stride_s, k_stride_h}, {v_stride_b, v_stride_s, v_stride_h}, apply_hadamard, qk_scale,
+                          (cudaStream_t)stream);
 }
 
 extern "C" int q8k_qk_norm_rope_prep(const void* x, int64_t x_row_stride, const float* norm_w, const float* cos_t,

@@ -241,6 +241,30 @@ __device__ __forceinline__ float warp_sum(float v) {
     return v;
 }
 
+// Walsh-Hadamard stages 0 .. log2(V)-1 over V consecutive elements: stride 1 scalar, the rest packed
+template <int V>
+__device__ __forceinline__ void butterfly_consecutive(float (&v)[V]) {
+#pragma unroll
+    for (int i = 0; i < V; i += 2) {
+        const float a = v[i], b = v[i + 1];
+        v[i] = __fadd_rn(a, b);
+        v[i + 1] = __fsub_rn(a, b);
+    }
+#pragma unroll
+    for (int st = 2; st < V; st <<= 1) {
+#pragma unroll
+        for (int h = 0; h < V / 2; h += 2) {                   // h, h+1 index two adjacent butterflies
+            const int lo = h & (st - 1);
+            const int i = ((h - lo) << 1) + lo;
+            const float2 a = make_float2(v[i], v[i + 1]);
+            const float2 b = make_float2(v[i + st], v[i + st + 1]);
+            const float2 su = fadd2(a, b), di = fsub2(a, b);
+            v[i] = su.x; v[i + 1] = su.y;
+            v[i + st] = di.x; v[i + st + 1] = di.y;
+        }
+    }
+}
+
 // tanh-GELU of the reference (csrc/gemm/q8_matmul_bias.cu:29-33).
 __device__ __forceinline__ float gelu_tanh_precise(float x) {
     const float u = 0.7978845608028654f * (x + 0.044715f * x * x * x);

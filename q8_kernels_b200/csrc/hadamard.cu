@@ -177,30 +177,6 @@ __device__ __forceinline__ void butterfly_groups(float (&v)[V]) {
     }
 }
 
-// stages 0 .. log2(V)-1 over V consecutive elements: stride 1 scalar, the rest packed
-template <int V>
-__device__ __forceinline__ void butterfly_consecutive(float (&v)[V]) {
-#pragma unroll
-    for (int i = 0; i < V; i += 2) {
-        const float a = v[i], b = v[i + 1];
-        v[i] = __fadd_rn(a, b);
-        v[i + 1] = __fsub_rn(a, b);
-    }
-#pragma unroll
-    for (int st = 2; st < V; st <<= 1) {
-#pragma unroll
-        for (int h = 0; h < V / 2; h += 2) {                   // h, h+1 index two adjacent butterflies
-            const int lo = h & (st - 1);
-            const int i = ((h - lo) << 1) + lo;
-            const float2 a = make_float2(v[i], v[i + 1]);
-            const float2 b = make_float2(v[i + st], v[i + st + 1]);
-            const float2 su = fadd2(a, b), di = fsub2(a, b);
-            v[i] = su.x; v[i + 1] = su.y;
-            v[i + st] = di.x; v[i + st + 1] = di.y;
-        }
-    }
-}
-
 // Units of whole warps walk over the rows (a grid of as many CTAs as fit the device): a row of up to 2048 elements
 // belongs to one warp or a part of one, a longer row to one CTA.  A thread has 64 values.  Per row: the raw elements
 // were copied into the unit's staging buffer by cp.async while the row before was being transformed; a thread reads

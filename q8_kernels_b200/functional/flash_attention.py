@@ -2,7 +2,7 @@
 
 For bf16 inputs with head dim 64 the reference's torch glue (transpose + pad +
 cast of V, Hadamard or cast of Q/K: five full-tensor passes) is one pre-pass
-kernel group; the attention kernel itself is the tcgen05 one.
+kernel, and V stays in rows; the attention kernel itself is the tcgen05 one.
 """
 import math
 from typing import Optional
@@ -38,8 +38,8 @@ def flash_attn_func(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, softmax_s
             kernel_scale = 1.0
         else:
             qk_scale, kernel_scale = 1.0, softmax_scale
-        q8, k8, vt8 = native.attention_prep(q, k, v, apply_qk_hadamard, qk_scale)
-        return native.flash_attention(q8, k8, vt8, kernel_scale, batch_mask, out_dtype, token_major_out)
+        q8, k8, v8 = native.attention_prep_rows(q, k, v, apply_qk_hadamard, qk_scale)
+        return native.flash_attention(q8, k8, v8, kernel_scale, batch_mask, out_dtype, token_major_out, v_rows=True)
 
     # general path, same steps as the reference
     if head_size_og % 32 != 0:

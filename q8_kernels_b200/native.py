@@ -458,6 +458,34 @@ def flash_attention_into(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, soft
               "flash_attention")
 
 
+def _attention_prep(fn, name, q, k, v, v_shape, apply_hadamard, qk_scale):
+    dev = require_cuda(q, k, v)
+    B, H, S_q, D = q.shape
+    S_kv = k.shape[2]
+    if D != 64 or k.shape[3] != 64 or v.shape[3] != 64:
+        raise Q8KernelError(f"{name}: head dim must be 64")
+    if v.shape[2] != S_kv:
+        raise Q8KernelError("v tokens != k tokens")
+    fixed = []
+    for t in (q, k, v):
+        if t.dtype != torch.bfloat16:
+            raise Q8KernelError(f"{name}: inputs must be bfloat16")
+        if t.stride(3) != 1 or any(s % 8 for s in t.stride()[:3]) or t.data_ptr() % 16:
+            t = t.contiguous()
+        fixed.append(t)
+    q, k, v = fixed
+    q8 = torch.empty((B, H, S_q, 64), dtype=E4M3, device=dev)
+    k8 = torch.empty((B, H, S_kv, 64), dtype=E4M3, device=dev)
+    v8 = torch.empty((B, H) + v_shape(S_kv), dtype=E4M3, device=dev)
+    with torch.cuda.device(dev):
+        check(fn(ptr(q), ptr(k), ptr(v), ptr(q8), ptr(k8), ptr(v8), B, H, S_q, S_kv,
+                 q.stride(0), q.stride(2), q.stride(1),
+                 k.stride(0), k.stride(2), k.stride(1),
+                 v.stride(0), v.stride(2), v.stride(1),
+                 int(bool(apply_hadamard)), float(qk_scale), stream_ptr(dev)), name)
+    return q8, k8, v8
+
+
 def attention_prep(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, apply_hadamard: bool,
                    qk_scale: float) -> Tuple[torch.Tensor, torch.Tensor, torch.Tensor]:
     """One launch group replacing the torch glue of
@@ -465,32 +493,15 @@ def attention_prep(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, apply_hada
     64: q, k, v are [B,H,S,64] tensors or views (any batch / token / head
     strides, last dim contiguous).  Returns q8, k8 [B,H,S,64] and
     vt8 [B,H,64,ceil16(S_kv)] in e4m3."""
-    dev = require_cuda(q, k, v)
-    B, H, S_q, D = q.shape
-    S_kv = k.shape[2]
-    if D != 64 or k.shape[3] != 64 or v.shape[3] != 64:
-        raise Q8KernelError("attention_prep: head dim must be 64")
-    if v.shape[2] != S_kv:
-        raise Q8KernelError("v tokens != k tokens")
-    fixed = []
-    for t in (q, k, v):
-        if t.dtype != torch.bfloat16:
-            raise Q8KernelError("attention_prep: inputs must be bfloat16")
-        if t.stride(3) != 1 or any(s % 8 for s in t.stride()[:3]) or t.data_ptr() % 16:
-            t = t.contiguous()
-        fixed.append(t)
-    q, k, v = fixed
-    s_pad = (S_kv + 15) // 16 * 16
-    q8 = torch.empty((B, H, S_q, 64), dtype=E4M3, device=dev)
-    k8 = torch.empty((B, H, S_kv, 64), dtype=E4M3, device=dev)
-    vt8 = torch.empty((B, H, 64, s_pad), dtype=E4M3, device=dev)
-    with torch.cuda.device(dev):
-        check(lib.q8k_attention_prep(ptr(q), ptr(k), ptr(v), ptr(q8), ptr(k8), ptr(vt8), B, H, S_q, S_kv,
-                                     q.stride(0), q.stride(2), q.stride(1),
-                                     k.stride(0), k.stride(2), k.stride(1),
-                                     v.stride(0), v.stride(2), v.stride(1),
-                                     int(bool(apply_hadamard)), float(qk_scale), stream_ptr(dev)), "attention_prep")
-    return q8, k8, vt8
+    return _attention_prep(lib.q8k_attention_prep, "attention_prep", q, k, v, lambda S: (64, (S + 15) // 16 * 16),
+                           apply_hadamard, qk_scale)
+
+
+def attention_prep_rows(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, apply_hadamard: bool,
+                        qk_scale: float) -> Tuple[torch.Tensor, torch.Tensor, torch.Tensor]:
+    """attention_prep with V cast to rows [B,H,S_kv,64], for ``flash_attention(v_rows=True)``: one launch."""
+    return _attention_prep(lib.q8k_attention_prep_rows, "attention_prep_rows", q, k, v, lambda S: (S, 64),
+                           apply_hadamard, qk_scale)
 
 
 def qk_norm_rope_prep(x: torch.Tensor, norm_w: torch.Tensor, freqs_cis, num_heads: int, apply_hadamard: bool,

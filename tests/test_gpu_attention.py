@@ -102,6 +102,32 @@ def test_attention_prep_bit_exact(nat, cuda_device, hadamard):
     Hp.assert_bit_equal(vt8, rv.contiguous(), "vt8")
 
 
+@pytest.mark.parametrize("B,H,Sq,Skv", [(1, 1, 1, 1), (2, 3, 43, 85), (1, 33, 4, 129), (3, 40, 31, 17), (1, 128, 2, 65)])
+@pytest.mark.parametrize("hadamard", [True, False])
+@pytest.mark.parametrize("layout", ["tokens", "heads", "batch_last"])
+def test_attention_prep_rows_every_layout(nat, cuda_device, B, H, Sq, Skv, hadamard, layout):
+    """Q, K and V rows in one launch: tails of the 128-row blocks, head counts below, at and above the 32 rows of a
+    pass, token-major, head-major and permuted views, out-of-range and NaN inputs (c10 cast)."""
+    g = Hp.gen(B * 1000 + H * 10 + Sq)
+
+    def view(S):
+        shape, perm = {"tokens": ((B, S, H, 64), (0, 2, 1, 3)), "heads": ((B, H, S, 64), (0, 1, 2, 3)),
+                       "batch_last": ((S, H, B, 64), (2, 1, 0, 3))}[layout]
+        x = torch.randn(shape, generator=g) * 3
+        x.view(-1)[:: 97] = 700.0
+        x.view(-1)[50] = float("nan")
+        return x.to(torch.bfloat16).permute(perm)
+
+    q, k, v = view(Sq), view(Skv), view(Skv)
+    scale = 0.0442 if hadamard else 1.0
+    q8, k8, v8 = nat.attention_prep_rows(q.to(cuda_device), k.to(cuda_device), v.to(cuda_device), hadamard, scale)
+    for got, x, rot in ((q8, q, hadamard), (k8, k, hadamard), (v8, v, False)):
+        ref = O.hadamard_transform(x.contiguous(), scale=scale, out_dtype=E4M3) if rot else O.c10_e4m3(x)
+        nan = torch.isnan(ref.float())
+        assert torch.equal(torch.isnan(got.cpu().float()), nan)
+        assert torch.equal(Hp.bits(got.cpu())[~nan], Hp.bits(ref.contiguous())[~nan])
+
+
 def test_self_attention_dit_shape_sampled(nat, cuda_device):
     """Config-3 shape (S = 6144, D = 64) on 2 heads; the oracle is evaluated on a
     sample of query rows (every key is still visited), the full output through
