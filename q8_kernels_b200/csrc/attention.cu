@@ -243,7 +243,7 @@ flash_attn_fp8_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
         reg_dealloc<kAttnRegsIo>();
         if (warp == 0) {
             // -------------------------------------------- TMA producer
-            if (lane == 0) {
+            if (ptx::elect_one()) {
                 auto load_q = [&](int t) {                      // query tile t of this CTA into Q buffer t & 1
                     ptx::mbar_arrive_expect_tx(q_full(t & 1), L::kQBytes);
                     ptx::tma_load_3d(smem_base + q_off(t & 1), &tmap_q, q_full(t & 1), 0, (tile0 + t * tstride) * kAttnBM, bh);
@@ -293,7 +293,7 @@ flash_attn_fp8_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
             // (if any); i+2 = P.V(i) and Q.K^T(i+2) (if any).  So phase i+1, which the softmax warps wait for in
             // the middle of step i, says that the scores of block i+1 are in TMEM AND (i >= 1) that O holds P.V
             // up to block i-1; phase nblk+1 says that O is complete.
-            if (lane == 0) {
+            if (ptx::elect_one()) {
                 constexpr uint32_t IDESC = ptx::make_idesc_e4m3(kAttnBM, kAttnBN);
                 // P.V with V as rows: B operand MN-major (bit 16); its 32-key K slices are 32 rows of 64 bytes apart
                 constexpr uint32_t IDESC_PV = V_ROWS ? (IDESC | (1u << 16)) : IDESC;

@@ -100,7 +100,7 @@ gemm_8bit_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
 
     if (warp == 0) {
         // ------------------------------------------------ TMA producer
-        if (lane == 0) {
+        if (ptx::elect_one()) {
             uint32_t it = 0;
             bool ok = true;
             for (int tile = blockIdx.x; ok && tile < p.total_tiles; tile += gridDim.x) {
@@ -133,7 +133,7 @@ gemm_8bit_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
         }
     } else if (warp == 1) {
         // ------------------------------------------------ MMA issuer
-        if (lane == 0) {
+        if (ptx::elect_one()) {
             uint32_t it = 0;
             uint32_t tile_i = 0;
             bool ok = true;

@@ -26,6 +26,21 @@ __device__ __forceinline__ unsigned long long globaltimer_ns() {
     return t;
 }
 
+// One lane of a converged warp, chosen by the hardware.  The compiler knows that exactly one thread takes the branch,
+// so the uniform operands of TMA and tcgen05 instructions are moved once; behind `lane == 0` every such instruction
+// re-derives them (four MMAs and a commit: 160 clocks against 226, N = 32).
+__device__ __forceinline__ bool elect_one() {
+    uint32_t p;
+    asm volatile(
+        "{\n\t"
+        ".reg .pred p;\n\t"
+        "elect.sync _|p, 0xffffffff;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t"
+        "}"
+        : "=r"(p));
+    return p != 0;
+}
+
 // ---------------------------------------------------------------- mbarrier
 __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
@@ -333,9 +348,12 @@ __device__ __forceinline__ void mma_i8_pair(uint32_t d_tmem, uint64_t a_desc, ui
         ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
         : "memory");
 }
-// One arrival on `cluster_bar` (in either CTA) once every MMA this thread issued before has completed.
-__device__ __forceinline__ void tcgen05_commit_pair(uint32_t cluster_bar) {
-    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(cluster_bar) : "memory");
+// One arrival on the barrier at this shared-memory offset in BOTH CTAs of the pair once every MMA this thread issued
+// before has completed.
+__device__ __forceinline__ void tcgen05_commit_both(uint32_t bar) {
+    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(bar),
+                 "h"((uint16_t)3)
+                 : "memory");
 }
 
 // ---------------------------------------------------------------- descriptors
