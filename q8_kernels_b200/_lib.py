@@ -133,7 +133,21 @@ def ptr(t: Optional[torch.Tensor]) -> Optional[int]:
 
 
 def stream_ptr(device: torch.device) -> int:
-    return torch.cuda.current_stream(device).cuda_stream
+    return torch._C._cuda_getCurrentRawStream(device.index)
+
+
+def launch(dev: torch.device, op: str, fn, *args) -> None:
+    """Call a native entry point on torch's current stream of ``dev`` (its last argument) with ``dev`` as the current
+    device, and raise if it refuses.  The device is only switched when it has to be: entering and leaving
+    ``torch.cuda.device`` and building a ``torch.cuda.Stream`` cost more host time than the launch itself."""
+    idx = dev.index
+    if torch._C._cuda_getDevice() == idx:
+        rc = fn(*args, torch._C._cuda_getCurrentRawStream(idx))
+    else:
+        with torch.cuda.device(dev):
+            rc = fn(*args, torch._C._cuda_getCurrentRawStream(idx))
+    if rc != 0:
+        check(rc, op)
 
 
 # One int32 status word per device, shared by all tensor-core launches.  The

@@ -40,8 +40,6 @@ class LTXTransformerBlock(nn.Module):
         num_ada_params = self.scale_shift_table.shape[0]
         ada_values = self.scale_shift_table[None, None] + timestep.reshape(
             hidden_states.shape[0], timestep.shape[1], num_ada_params, -1)
-        shift_msa, scale_msa, gate_msa, shift_mlp, scale_mlp, gate_mlp = ada_values.unbind(dim=2)
-
         # Fused path (same values, fewer passes over the activations): RMS norm + modulation + Hadamard +
         # quantizer in one kernel in front of attn1 and the feed-forward, and gate * out + residual in
         # the epilogue of the three output projections.  Needs bf16 activations and norms without affine
@@ -51,6 +49,8 @@ class LTXTransformerBlock(nn.Module):
                  and non_mm_precision == torch.bfloat16 and hidden_states.dim() == 3 and timestep.shape[1] == 1
                  and hidden_states.shape[-1] >= 512)
         if fused and fuse:
+            # one copy that makes each of the six [B,1,dim] modulation rows contiguous (none for batch 1)
+            shift_msa, scale_msa, gate_msa, shift_mlp, scale_mlp, gate_mlp = ada_values.permute(2, 0, 1, 3).contiguous().unbind(0)
             qt = self.ff.proj_down.weight.dtype                  # int8 or e4m3: the activations follow the weights
             nq = native.norm_modulate_quant(hidden_states, scale_msa, shift_msa, qt)
             hidden_states = self.attn1(None, freqs_cis, None, attention_mask, non_mm_precision, mm_out_dtype,
@@ -67,6 +67,7 @@ class LTXTransformerBlock(nn.Module):
             return native.mm_gate_residual(aq, down.weight.data, down.bias.data if down.bias is not None else None,
                                            as_, down.scales, gate_mlp, hidden_states)
 
+        shift_msa, scale_msa, gate_msa, shift_mlp, scale_mlp, gate_mlp = ada_values.unbind(dim=2)
         norm_hidden_states = self.norm1(hidden_states, non_mm_precision)
         norm_hidden_states = norm_hidden_states * (1 + scale_msa) + shift_msa
         attn_output = self.attn1(norm_hidden_states, freqs_cis, None, attention_mask, non_mm_precision, mm_out_dtype,

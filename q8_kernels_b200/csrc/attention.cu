@@ -1026,14 +1026,22 @@ static int launch_flash_attention(bool v_rows, const void* q, const void* k, con
         const int tiles_per_cta = (q_tiles + g_max - 1) / g_max;
         ctas_per_bh = (q_tiles + tiles_per_cta - 1) / tiles_per_cta;
     }
-    auto kern = v_rows ? (multi ? flash_attn_fp8_kernel<true, true> : flash_attn_fp8_kernel<true, false>)
-                       : (multi ? flash_attn_fp8_kernel<false, true> : flash_attn_fp8_kernel<false, false>);
-    cudaFuncAttributes fattr;
-    Q8K_CUDA_OK(cudaFuncGetAttributes(&fattr, kern));
-    Q8K_REQUIRE(fattr.numRegs >= kAttnRegsLaunch, Q8K_ERR_CUDA,
+    using Kern = void (*)(CUtensorMap, CUtensorMap, CUtensorMap, CUtensorMap, AttnParams);
+    static const Kern kernels[4] = {flash_attn_fp8_kernel<false, false>, flash_attn_fp8_kernel<false, true>,
+                                    flash_attn_fp8_kernel<true, false>, flash_attn_fp8_kernel<true, true>};
+    static std::atomic<uint64_t> smem_done[4];
+    static std::atomic<int> regs[4];
+    const int which = (v_rows ? 2 : 0) + (multi ? 1 : 0);
+    const Kern kern = kernels[which];
+    if (regs[which].load(std::memory_order_relaxed) == 0) {
+        cudaFuncAttributes fattr;
+        Q8K_CUDA_OK(cudaFuncGetAttributes(&fattr, kern));
+        regs[which].store(fattr.numRegs, std::memory_order_relaxed);
+    }
+    Q8K_REQUIRE(regs[which].load(std::memory_order_relaxed) >= kAttnRegsLaunch, Q8K_ERR_CUDA,
                 "%s: kernel was built with %d registers per thread, %d needed for the warpgroup budgets", op,
-                fattr.numRegs, kAttnRegsLaunch);
-    Q8K_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, AttnSmem::kDynamic));
+                regs[which].load(std::memory_order_relaxed), kAttnRegsLaunch);
+    if (int rc = allow_dynamic_smem((const void*)kern, AttnSmem::kDynamic, smem_done[which])) return rc;
     dim3 grid((unsigned)ctas_per_bh, (unsigned)BH);
     kern<<<grid, kAttnThreads, AttnSmem::kDynamic, (cudaStream_t)stream>>>(tq, tk, tv, to, p);
     Q8K_CUDA_OK(cudaGetLastError());

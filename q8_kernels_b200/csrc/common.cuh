@@ -10,6 +10,8 @@
 #include <stdint.h>
 #include <stdio.h>
 
+#include <atomic>
+
 #include "../../include/q8_kernels_b200.h"
 
 namespace q8k {
@@ -35,6 +37,18 @@ void set_error_detail(const char* fmt, ...);
     } while (0)
 
 int gemm_num_sms();                          // SMs of the current device (148 if it cannot be asked)
+
+// Raise a kernel's dynamic shared memory limit, once per device (the call costs about 1 us, a launch 2.5).  The setting
+// lives as long as the device's context; `done` belongs to the one kernel.
+inline int allow_dynamic_smem(const void* kern, int bytes, std::atomic<uint64_t>& done) {
+    int dev = 0;
+    Q8K_CUDA_OK(cudaGetDevice(&dev));
+    const uint64_t bit = dev < 64 ? 1ull << dev : 0ull;
+    if ((done.load(std::memory_order_relaxed) & bit) != 0) return Q8K_OK;
+    Q8K_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
+    done.fetch_or(bit, std::memory_order_relaxed);
+    return Q8K_OK;
+}
 
 inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
 

@@ -320,7 +320,8 @@ template <bool INT8, int BN, int STAGES, bool GELU, bool OUT_E4M3, bool RESID = 
 static int launch_gemm(const CUtensorMap& ta, const CUtensorMap& tb, const GemmParams& p, cudaStream_t st) {
     using L = GemmSmem<BN, STAGES>;
     auto kern = gemm_8bit_kernel<INT8, BN, STAGES, GELU, OUT_E4M3, RESID>;
-    Q8K_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, L::kDynamic));
+    static std::atomic<uint64_t> smem_done{0};
+    if (int rc = allow_dynamic_smem((const void*)kern, L::kDynamic, smem_done)) return rc;
     const int grid = p.total_tiles < gemm_num_sms() ? p.total_tiles : gemm_num_sms();
     kern<<<grid, kGemmThreads, L::kDynamic, st>>>(ta, tb, p);
     Q8K_CUDA_OK(cudaGetLastError());

@@ -485,7 +485,8 @@ static int launch_pair(const CUtensorMap& ta, const CUtensorMap& tb, const CUten
                        const PairParams& pp, cudaStream_t st) {
     using PairSmem = PairSmemT<RESID>;
     auto kern = gemm_8bit_pair_kernel<INT8, GELU, OUT_E4M3, RESID>;
-    Q8K_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, PairSmem::kDynamic));
+    static std::atomic<uint64_t> smem_done{0};
+    if (int rc = allow_dynamic_smem((const void*)kern, PairSmem::kDynamic, smem_done)) return rc;
     // how many 2-CTA clusters can be resident at once (cached per kernel variant)
     static int max_clusters = -1;
     if (max_clusters < 0) {

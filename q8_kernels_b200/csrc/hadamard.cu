@@ -567,10 +567,13 @@ template <typename Tin, typename Tout, int LOG_N, Epilogue EPI, bool NORM_MOD>
 static int launch_stream(const Tin* x, Tout* out, float* scales, int64_t rows, int dim, int64_t stride, float scale,
                          const __nv_bfloat16* ms, const __nv_bfloat16* mh, int64_t rows_per_mod, cudaStream_t st) {
     using Geo = StreamGeo<Tin, LOG_N, NORM_MOD>;
-    auto kern = dim == Geo::N ? hadamard_stream_kernel<Tin, Tout, LOG_N, EPI, NORM_MOD, true>
-                              : hadamard_stream_kernel<Tin, Tout, LOG_N, EPI, NORM_MOD, false>;
-    if (Geo::SMEM > 47 * 1024)                                 // (with the static reduction words, above the 48 KB default)
-        Q8K_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Geo::SMEM));
+    const bool full = dim == Geo::N;
+    auto kern = full ? hadamard_stream_kernel<Tin, Tout, LOG_N, EPI, NORM_MOD, true>
+                     : hadamard_stream_kernel<Tin, Tout, LOG_N, EPI, NORM_MOD, false>;
+    if (Geo::SMEM > 47 * 1024) {                               // (with the static reduction words, above the 48 KB default)
+        static std::atomic<uint64_t> smem_done[2];
+        if (int rc = allow_dynamic_smem((const void*)kern, Geo::SMEM, smem_done[full])) return rc;
+    }
     const int64_t slots = (int64_t)gemm_num_sms() * Geo::CTAS;
     constexpr int per_cta = Geo::UNITS * Geo::RPU;
     int64_t groups = 1, group_rows = rows;

@@ -16,7 +16,7 @@ import ctypes
 import torch
 
 from . import _lib
-from ._lib import Q8KernelError, check, dt, lib, ptr, require_cuda, stream_ptr
+from ._lib import Q8KernelError, dt, launch, lib, ptr, require_cuda, stream_ptr
 
 E4M3 = torch.float8_e4m3fn
 
@@ -32,8 +32,24 @@ def _rows_view(x: torch.Tensor) -> torch.Tensor:
     return x2
 
 
-def _row_stride(x2: torch.Tensor) -> int:
-    return x2.stride(0) if x2.shape[0] > 1 else x2.shape[1]
+def _rows(x: torch.Tensor):
+    """(tensor, rows, dim, row stride in elements) of [..., dim] for a kernel that takes strided rows.  A contiguous
+    tensor is passed as it is: no view is built."""
+    dim = x.shape[-1]
+    if dim and x.is_contiguous():
+        return x, x.numel() // dim, dim, dim
+    x2 = _rows_view(x)
+    rows, dim = x2.shape
+    return x2, rows, dim, x2.stride(0) if rows > 1 else dim
+
+
+def _dense_rows(x: torch.Tensor):
+    """(contiguous tensor, rows, dim) of [..., dim]."""
+    dim = x.shape[-1]
+    if dim and x.is_contiguous():
+        return x, x.numel() // dim, dim
+    x2 = x.reshape(-1, dim).contiguous()
+    return x2, x2.shape[0], dim
 
 
 # ---------------------------------------------------------------- quantizer._C
@@ -45,15 +61,12 @@ def tokenwise_quant(x: torch.Tensor, out_type: Optional[torch.dtype] = None) -> 
     out_type = torch.int8 if out_type is None else out_type
     if out_type not in (torch.int8, E4M3):
         raise Q8KernelError(f"tokenwise_quant: out_type {out_type} must be int8 or float8_e4m3fn")
-    shape = x.shape
-    x2 = _rows_view(x)
-    rows, dim = x2.shape
-    q = torch.empty((rows, dim), dtype=out_type, device=dev)
-    scales = torch.empty((rows,), dtype=torch.float32, device=dev)
-    with torch.cuda.device(dev):
-        check(lib.q8k_tokenwise_quant(ptr(x2), dt(x2.dtype), ptr(q), dt(out_type), ptr(scales), rows, dim,
-                                      _row_stride(x2), stream_ptr(dev)), "tokenwise_quant")
-    return [q.reshape(shape), scales.reshape(shape[:-1])]
+    x2, rows, dim, stride = _rows(x)
+    q = torch.empty(x.shape, dtype=out_type, device=dev)
+    scales = torch.empty(x.shape[:-1], dtype=torch.float32, device=dev)
+    launch(dev, "tokenwise_quant", lib.q8k_tokenwise_quant, ptr(x2), dt(x2.dtype), ptr(q), dt(out_type), ptr(scales),
+           rows, dim, stride)
+    return [q, scales]
 
 
 # ---------------------------------------------------------------- ops._C
@@ -65,19 +78,15 @@ def fast_hadamard_transform(x: torch.Tensor, scale: float, out_type: Optional[to
         raise Q8KernelError(f"fast_hadamard_transform: input dtype {x.dtype} must be bfloat16 or float8_e4m3fn")
     out_type = x.dtype if out_type is None else out_type
     shape = x.shape
-    x2 = _rows_view(x)
-    dim_og = x2.shape[1]
+    x2, rows, dim, stride = _rows(x)
+    dim_og = dim
     if dim_og % 8 != 0:
-        x2 = torch.nn.functional.pad(x2, (0, 8 - dim_og % 8))
-    rows, dim = x2.shape
-    out = torch.empty((rows, dim), dtype=out_type, device=dev)
-    with torch.cuda.device(dev):
-        check(lib.q8k_fast_hadamard_transform(ptr(x2), dt(x2.dtype), ptr(out), dt(out_type), rows, dim,
-                                              _row_stride(x2), float(scale), stream_ptr(dev)),
-              "fast_hadamard_transform")
-    if dim != dim_og:
-        out = out[:, :dim_og]
-    return out.reshape(shape)
+        x2 = torch.nn.functional.pad(x2.reshape(rows, dim), (0, 8 - dim_og % 8))
+        dim = stride = x2.shape[1]
+    out = torch.empty(shape if dim == dim_og else (rows, dim), dtype=out_type, device=dev)
+    launch(dev, "fast_hadamard_transform", lib.q8k_fast_hadamard_transform, ptr(x2), dt(x2.dtype), ptr(out),
+           dt(out_type), rows, dim, stride, float(scale))
+    return out if dim == dim_og else out[:, :dim_og].reshape(shape)
 
 
 def hadamard_quant(x: torch.Tensor, scale: float, out_type: Optional[torch.dtype] = None) -> List[torch.Tensor]:
@@ -86,15 +95,12 @@ def hadamard_quant(x: torch.Tensor, scale: float, out_type: Optional[torch.dtype
     q8_kernels/functional/linear.py:30-31."""
     dev = require_cuda(x)
     out_type = torch.int8 if out_type is None else out_type
-    shape = x.shape
-    x2 = _rows_view(x)
-    rows, dim = x2.shape
-    q = torch.empty((rows, dim), dtype=out_type, device=dev)
-    scales = torch.empty((rows,), dtype=torch.float32, device=dev)
-    with torch.cuda.device(dev):
-        check(lib.q8k_hadamard_quant(ptr(x2), dt(x2.dtype), ptr(q), dt(out_type), ptr(scales), rows, dim,
-                                     _row_stride(x2), float(scale), stream_ptr(dev)), "hadamard_quant")
-    return [q.reshape(shape), scales.reshape(shape[:-1])]
+    x2, rows, dim, stride = _rows(x)
+    q = torch.empty(x.shape, dtype=out_type, device=dev)
+    scales = torch.empty(x.shape[:-1], dtype=torch.float32, device=dev)
+    launch(dev, "hadamard_quant", lib.q8k_hadamard_quant, ptr(x2), dt(x2.dtype), ptr(q), dt(out_type), ptr(scales),
+           rows, dim, stride, float(scale))
+    return [q, scales]
 
 
 def norm_modulate_quant(x: torch.Tensor, mod_scale: torch.Tensor, mod_shift: torch.Tensor,
@@ -115,10 +121,8 @@ def norm_modulate_quant(x: torch.Tensor, mod_scale: torch.Tensor, mod_shift: tor
     mod_shift = mod_shift.contiguous()
     q = torch.empty((B, S, dim), dtype=out_type, device=dev)
     scales = torch.empty((B, S), dtype=torch.float32, device=dev)
-    with torch.cuda.device(dev):
-        check(lib.q8k_norm_modulate_quant(ptr(x), ptr(mod_scale), ptr(mod_shift), ptr(q), dt(out_type), ptr(scales),
-                                          B * S, dim, S, float(1.0 / math.sqrt(dim)), stream_ptr(dev)),
-              "norm_modulate_quant")
+    launch(dev, "norm_modulate_quant", lib.q8k_norm_modulate_quant, ptr(x), ptr(mod_scale), ptr(mod_shift), ptr(q),
+           dt(out_type), ptr(scales), B * S, dim, S, float(1.0 / math.sqrt(dim)))
     return [q, scales]
 
 
@@ -129,19 +133,24 @@ def rms_norm(x: torch.Tensor, weights: Optional[torch.Tensor] = None,
     if weights is not None and weights.dtype != torch.float32:
         raise Q8KernelError("rms_norm: weights must be float32")
     out_type = x.dtype if out_type is None else out_type
-    shape = x.shape
-    x2 = x.reshape(-1, shape[-1]).contiguous()
-    rows, dim = x2.shape
+    x2, rows, dim = _dense_rows(x)
     if weights is not None:
         weights = weights.contiguous()
         if weights.numel() != dim:
             raise Q8KernelError("rms_norm: weights size does not match the last dim")
-    out = torch.empty((rows, dim), dtype=out_type, device=dev)
-    rrms = torch.empty((rows,), dtype=torch.float32, device=dev)
-    with torch.cuda.device(dev):
-        check(lib.q8k_rms_norm(ptr(x2), dt(x2.dtype), ptr(weights), ptr(out), dt(out_type), ptr(rrms), rows, dim,
-                               stream_ptr(dev)), "rms_norm")
-    return [out.reshape(shape), rrms.reshape(shape[:-1])]
+    out = torch.empty(x.shape, dtype=out_type, device=dev)
+    rrms = torch.empty(x.shape[:-1], dtype=torch.float32, device=dev)
+    launch(dev, "rms_norm", lib.q8k_rms_norm, ptr(x2), dt(x2.dtype), ptr(weights), ptr(out), dt(out_type), ptr(rrms),
+           rows, dim)
+    return [out, rrms]
+
+
+def _tables(cos_freqs: torch.Tensor, sin_freqs: torch.Tensor, dim: int):
+    """The rotary tables as contiguous rows of ``dim`` (the last dim of x), and their number."""
+    if dim and cos_freqs.shape[-1] == dim and cos_freqs.is_contiguous() and sin_freqs.is_contiguous():
+        return cos_freqs, sin_freqs, cos_freqs.numel() // dim
+    c2 = cos_freqs.reshape(-1, dim).contiguous()
+    return c2, sin_freqs.reshape(-1, dim).contiguous(), c2.shape[0]
 
 
 def rope(x: torch.Tensor, cos_freqs: torch.Tensor, sin_freqs: torch.Tensor,
@@ -155,22 +164,18 @@ def rope(x: torch.Tensor, cos_freqs: torch.Tensor, sin_freqs: torch.Tensor,
         raise Q8KernelError("rope: cos and sin shapes differ")
     out_type = x.dtype if out_type is None else out_type
     shape = x.shape
-    dim = shape[-1]
-    x2 = x.reshape(-1, dim).contiguous()
-    rows = x2.shape[0]
-    c2 = cos_freqs.reshape(-1, dim).contiguous()
-    s2 = sin_freqs.reshape(-1, dim).contiguous()
-    if c2.shape[0] == rows:
+    x2, rows, dim = _dense_rows(x)
+    c2, s2, table_rows = _tables(cos_freqs, sin_freqs, dim)
+    if table_rows == rows:
         freq_rows = 0
-    elif rows % c2.shape[0] == 0 and cos_freqs.dim() == x.dim() and cos_freqs.shape[0] == 1:
-        freq_rows = c2.shape[0]
+    elif rows % table_rows == 0 and cos_freqs.dim() == x.dim() and cos_freqs.shape[0] == 1:
+        freq_rows = table_rows
     else:
         raise Q8KernelError(f"rope: table shape {tuple(cos_freqs.shape)} does not match x {tuple(shape)}")
-    out = torch.empty((rows, dim), dtype=out_type, device=dev)
-    with torch.cuda.device(dev):
-        check(lib.q8k_rope(ptr(x2), dt(x2.dtype), ptr(c2), ptr(s2), ptr(out), dt(out_type), rows, dim, freq_rows,
-                           stream_ptr(dev)), "rope")
-    return out.reshape(shape)
+    out = torch.empty(shape, dtype=out_type, device=dev)
+    launch(dev, "rope", lib.q8k_rope, ptr(x2), dt(x2.dtype), ptr(c2), ptr(s2), ptr(out), dt(out_type), rows, dim,
+           freq_rows)
+    return out
 
 
 def fma_8bit(x: torch.Tensor, y: torch.Tensor, z: torch.Tensor, scale_add: float) -> torch.Tensor:
@@ -192,9 +197,8 @@ def fma_8bit(x: torch.Tensor, y: torch.Tensor, z: torch.Tensor, scale_add: float
     y2 = y.reshape(-1, dim).contiguous()
     z2 = z.reshape(-1, dim).contiguous()
     out = torch.empty_like(x2)
-    with torch.cuda.device(dev):
-        check(lib.q8k_fma_8bit(ptr(x2), ptr(y2), dt(y2.dtype), ptr(z2), dt(z2.dtype), ptr(out), x2.shape[0], dim,
-                               y_every, z_every, float(scale_add), stream_ptr(dev)), "fma_8bit")
+    launch(dev, "fma_8bit", lib.q8k_fma_8bit, ptr(x2), ptr(y2), dt(y2.dtype), ptr(z2), dt(z2.dtype), ptr(out),
+           x2.shape[0], dim, y_every, z_every, float(scale_add))
     return out.reshape(x.shape)
 
 
@@ -205,9 +209,8 @@ def gelu_forward(x: torch.Tensor, out_type: Optional[torch.dtype] = None) -> tor
     shape = x.shape
     x2 = x.reshape(-1, shape[-1]).contiguous()
     out = torch.empty(x2.shape, dtype=out_type, device=dev)
-    with torch.cuda.device(dev):
-        check(lib.q8k_gelu_forward(ptr(x2), dt(x2.dtype), ptr(out), dt(out_type), x2.shape[0], x2.shape[1],
-                                   stream_ptr(dev)), "gelu_forward")
+    launch(dev, "gelu_forward", lib.q8k_gelu_forward, ptr(x2), dt(x2.dtype), ptr(out), dt(out_type), x2.shape[0],
+           x2.shape[1])
     return out.reshape(shape)
 
 
@@ -222,9 +225,8 @@ def gelu_backward(x: torch.Tensor, grad_output: torch.Tensor, out_type: Optional
     x2 = x.reshape(-1, shape[-1]).contiguous()
     g2 = grad_output.reshape(-1, shape[-1]).to(out_type).contiguous()
     out = torch.empty(x2.shape, dtype=out_type, device=dev)
-    with torch.cuda.device(dev):
-        check(lib.q8k_gelu_backward(ptr(x2), dt(x2.dtype), ptr(g2), ptr(out), dt(out_type), x2.shape[0], x2.shape[1],
-                                    stream_ptr(dev)), "gelu_backward")
+    launch(dev, "gelu_backward", lib.q8k_gelu_backward, ptr(x2), dt(x2.dtype), ptr(g2), ptr(out), dt(out_type),
+           x2.shape[0], x2.shape[1])
     return out.reshape(shape)
 
 
@@ -238,22 +240,18 @@ def rope_backward(grad_out: torch.Tensor, cos_freqs: torch.Tensor, sin_freqs: to
         raise Q8KernelError("rope_backward: cos and sin shapes differ")
     out_type = grad_out.dtype if out_type is None else out_type
     shape = grad_out.shape
-    dim = shape[-1]
-    g2 = grad_out.reshape(-1, dim).contiguous()
-    rows = g2.shape[0]
-    c2 = cos_freqs.reshape(-1, dim).contiguous()
-    s2 = sin_freqs.reshape(-1, dim).contiguous()
-    if c2.shape[0] == rows:
+    g2, rows, dim = _dense_rows(grad_out)
+    c2, s2, table_rows = _tables(cos_freqs, sin_freqs, dim)
+    if table_rows == rows:
         freq_rows = 0
-    elif rows % c2.shape[0] == 0 and cos_freqs.dim() == grad_out.dim() and cos_freqs.shape[0] == 1:
-        freq_rows = c2.shape[0]
+    elif rows % table_rows == 0 and cos_freqs.dim() == grad_out.dim() and cos_freqs.shape[0] == 1:
+        freq_rows = table_rows
     else:
         raise Q8KernelError(f"rope_backward: table shape {tuple(cos_freqs.shape)} does not match {tuple(shape)}")
-    out = torch.empty((rows, dim), dtype=out_type, device=dev)
-    with torch.cuda.device(dev):
-        check(lib.q8k_rope_backward(ptr(g2), dt(g2.dtype), ptr(c2), ptr(s2), ptr(out), dt(out_type), rows, dim,
-                                    freq_rows, stream_ptr(dev)), "rope_backward")
-    return out.reshape(shape)
+    out = torch.empty(shape, dtype=out_type, device=dev)
+    launch(dev, "rope_backward", lib.q8k_rope_backward, ptr(g2), dt(g2.dtype), ptr(c2), ptr(s2), ptr(out), dt(out_type),
+           rows, dim, freq_rows)
+    return out
 
 
 def rms_norm_backward(x_normed: torch.Tensor, x_norms: torch.Tensor, grad_out: torch.Tensor,
@@ -267,21 +265,19 @@ def rms_norm_backward(x_normed: torch.Tensor, x_norms: torch.Tensor, grad_out: t
         raise Q8KernelError("rms_norm_backward: grad_out and x_normed shapes differ")
     out_type = x_normed.dtype if out_type is None else out_type
     shape = x_normed.shape
-    y2 = x_normed.reshape(-1, shape[-1]).contiguous()
-    g2 = grad_out.reshape(-1, shape[-1]).to(out_type).contiguous()
-    rows, dim = y2.shape
-    r = x_norms.reshape(-1).to(torch.float32).contiguous()
+    y2, rows, dim = _dense_rows(x_normed)
+    g2 = (grad_out if grad_out.dtype == out_type else grad_out.to(out_type)).contiguous()
+    r = (x_norms if x_norms.dtype == torch.float32 else x_norms.to(torch.float32)).contiguous()
     if r.numel() != rows:
         raise Q8KernelError("rms_norm_backward: x_norms must hold one value per row")
     if weights is not None:
         weights = weights.contiguous()
         if weights.numel() != dim:
             raise Q8KernelError("rms_norm_backward: weights size does not match the last dim")
-    out = torch.empty((rows, dim), dtype=out_type, device=dev)
-    with torch.cuda.device(dev):
-        check(lib.q8k_rms_norm_backward(ptr(y2), dt(y2.dtype), ptr(r), ptr(g2), ptr(weights), ptr(out), dt(out_type),
-                                        rows, dim, stream_ptr(dev)), "rms_norm_backward")
-    return out.reshape(shape)
+    out = torch.empty(shape, dtype=out_type, device=dev)
+    launch(dev, "rms_norm_backward", lib.q8k_rms_norm_backward, ptr(y2), dt(y2.dtype), ptr(r), ptr(g2), ptr(weights),
+           ptr(out), dt(out_type), rows, dim)
+    return out
 
 
 # ---------------------------------------------------------------- gemm._C
@@ -311,9 +307,8 @@ def _gemm(fn, name, a, b, bias, a_scales, b_scales, fuse_gelu, out_type, in_dtyp
     batch = max(bs_a, bs_b)
     out_type = E4M3 if out_type is None else out_type
     out = torch.empty((batch, m, n), dtype=out_type, device=dev)
-    with torch.cuda.device(dev):
-        check(fn(ptr(a), ptr(b), ptr(bias), ptr(a_scales), ptr(b_scales), ptr(out), dt(out_type), bs_a, bs_b,
-                 m, n, k, int(bool(fuse_gelu)), ptr(_lib.status_word(dev)), stream_ptr(dev)), name)
+    launch(dev, name, fn, ptr(a), ptr(b), ptr(bias), ptr(a_scales), ptr(b_scales), ptr(out), dt(out_type), bs_a, bs_b,
+           m, n, k, int(bool(fuse_gelu)), ptr(_lib.status_word(dev)))
     return out
 
 
@@ -361,10 +356,9 @@ def mm_gate_residual(a: torch.Tensor, b: torch.Tensor, bias: Optional[torch.Tens
     a, b, resid = a.contiguous(), b.contiguous(), resid.contiguous()
     a_scales, b_scales = a_scales.contiguous(), b_scales.contiguous()
     out = torch.empty((bs_a, m, n), dtype=torch.bfloat16, device=dev)
-    with torch.cuda.device(dev):
-        check(lib.q8k_mm_gate_residual(int(a.dtype == torch.int8), ptr(a), ptr(b), ptr(bias), ptr(a_scales), ptr(b_scales),
-                                       ptr(gate), ptr(resid), rows_per_gate, ptr(out), bs_a, 1, m, n, k,
-                                       ptr(_lib.status_word(dev)), stream_ptr(dev)), "mm_gate_residual")
+    launch(dev, "mm_gate_residual", lib.q8k_mm_gate_residual, int(a.dtype == torch.int8), ptr(a), ptr(b), ptr(bias),
+           ptr(a_scales), ptr(b_scales), ptr(gate), ptr(resid), rows_per_gate, ptr(out), bs_a, 1, m, n, k,
+           ptr(_lib.status_word(dev)))
     return out
 
 
@@ -409,17 +403,14 @@ def flash_attention(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, softmax_s
     else:
         buf = torch.empty((B, H, M, 64), dtype=out_type, device=dev)
         strides = (H * M * 64, M * 64, 64)
-    with torch.cuda.device(dev):
-        if v_rows:
-            outs = (ctypes.c_void_p * 1)(buf.data_ptr())
-            check(lib.q8k_flash_attention_v_rows(ptr(q), ptr(k), ptr(v), ctypes.cast(outs, ctypes.c_void_p), 1,
-                                                 dt(out_type), B, H, M, N, *strides, float(softmax_scale),
-                                                 ptr(batch_mask), ptr(_lib.status_word(dev)), stream_ptr(dev)),
-                  "flash_attention")
-        else:
-            check(lib.q8k_flash_attention_strided(ptr(q), ptr(k), ptr(v), ptr(buf), dt(out_type), B, H, M, N, *strides,
-                                                  float(softmax_scale), ptr(batch_mask), ptr(_lib.status_word(dev)),
-                                                  stream_ptr(dev)), "flash_attention")
+    if v_rows:
+        outs = (ctypes.c_void_p * 1)(buf.data_ptr())
+        launch(dev, "flash_attention", lib.q8k_flash_attention_v_rows, ptr(q), ptr(k), ptr(v),
+               ctypes.cast(outs, ctypes.c_void_p), 1, dt(out_type), B, H, M, N, *strides, float(softmax_scale),
+               ptr(batch_mask), ptr(_lib.status_word(dev)))
+    else:
+        launch(dev, "flash_attention", lib.q8k_flash_attention_strided, ptr(q), ptr(k), ptr(v), ptr(buf), dt(out_type),
+               B, H, M, N, *strides, float(softmax_scale), ptr(batch_mask), ptr(_lib.status_word(dev)))
     return buf.transpose(1, 2) if token_major_out else buf
 
 
@@ -451,11 +442,9 @@ def flash_attention_into(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, soft
     head_off = first_head * 64 * esz
     outs = (ctypes.c_void_p * len(dest_ptrs))(*[int(a) + head_off for a in dest_ptrs])
     strides = (M * total_heads * 64, 64, total_heads * 64)
-    with torch.cuda.device(dev):
-        fn = lib.q8k_flash_attention_v_rows if v_rows else lib.q8k_flash_attention_multi_out
-        check(fn(ptr(q), ptr(k), ptr(v), ctypes.cast(outs, ctypes.c_void_p), len(dest_ptrs), dt(out_type), B, h, M, N,
-                 *strides, float(softmax_scale), ptr(batch_mask), ptr(_lib.status_word(dev)), stream_ptr(dev)),
-              "flash_attention")
+    fn = lib.q8k_flash_attention_v_rows if v_rows else lib.q8k_flash_attention_multi_out
+    launch(dev, "flash_attention", fn, ptr(q), ptr(k), ptr(v), ctypes.cast(outs, ctypes.c_void_p), len(dest_ptrs),
+           dt(out_type), B, h, M, N, *strides, float(softmax_scale), ptr(batch_mask), ptr(_lib.status_word(dev)))
 
 
 def _attention_prep(fn, name, q, k, v, v_shape, apply_hadamard, qk_scale):
@@ -477,12 +466,9 @@ def _attention_prep(fn, name, q, k, v, v_shape, apply_hadamard, qk_scale):
     q8 = torch.empty((B, H, S_q, 64), dtype=E4M3, device=dev)
     k8 = torch.empty((B, H, S_kv, 64), dtype=E4M3, device=dev)
     v8 = torch.empty((B, H) + v_shape(S_kv), dtype=E4M3, device=dev)
-    with torch.cuda.device(dev):
-        check(fn(ptr(q), ptr(k), ptr(v), ptr(q8), ptr(k8), ptr(v8), B, H, S_q, S_kv,
-                 q.stride(0), q.stride(2), q.stride(1),
-                 k.stride(0), k.stride(2), k.stride(1),
-                 v.stride(0), v.stride(2), v.stride(1),
-                 int(bool(apply_hadamard)), float(qk_scale), stream_ptr(dev)), name)
+    launch(dev, name, fn, ptr(q), ptr(k), ptr(v), ptr(q8), ptr(k8), ptr(v8), B, H, S_q, S_kv, q.stride(0), q.stride(2),
+           q.stride(1), k.stride(0), k.stride(2), k.stride(1), v.stride(0), v.stride(2), v.stride(1),
+           int(bool(apply_hadamard)), float(qk_scale))
     return q8, k8, v8
 
 
@@ -525,10 +511,8 @@ def qk_norm_rope_prep(x: torch.Tensor, norm_w: torch.Tensor, freqs_cis, num_head
             raise Q8KernelError("qk_norm_rope_prep: rotary tables must be float32 [1,S,H*64]")
         cos, sin = cos.contiguous(), sin.contiguous()
     out = torch.empty((B, num_heads, S, 64), dtype=E4M3, device=dev)
-    with torch.cuda.device(dev):
-        check(lib.q8k_qk_norm_rope_prep(ptr(x), x.stride(1), ptr(norm_w.contiguous()), ptr(cos), ptr(sin), ptr(out), B, S,
-                                        num_heads, int(bool(apply_hadamard)), float(qk_scale), stream_ptr(dev)),
-              "qk_norm_rope_prep")
+    launch(dev, "qk_norm_rope_prep", lib.q8k_qk_norm_rope_prep, ptr(x), x.stride(1), ptr(norm_w.contiguous()), ptr(cos),
+           ptr(sin), ptr(out), B, S, num_heads, int(bool(apply_hadamard)), float(qk_scale))
     return out
 
 
@@ -551,10 +535,8 @@ def kv_prep(xk: torch.Tensor, xv: torch.Tensor, norm_wk: torch.Tensor, num_heads
         raise Q8KernelError("kv_prep: the norm weight must be float32 [H*64]")
     outk = torch.empty((B, num_heads, S, 64), dtype=E4M3, device=dev)
     outv = torch.empty((B, num_heads, S, 64), dtype=E4M3, device=dev)
-    with torch.cuda.device(dev):
-        check(lib.q8k_qkv_prep(None, ptr(xk), ptr(xv), xk.stride(1), None, ptr(norm_wk.contiguous()), None, None, None,
-                               ptr(outk), ptr(outv), B, S, num_heads, int(bool(apply_hadamard)), float(qk_scale),
-                               stream_ptr(dev)), "qkv_prep")
+    launch(dev, "qkv_prep", lib.q8k_qkv_prep, None, ptr(xk), ptr(xv), xk.stride(1), None, ptr(norm_wk.contiguous()),
+           None, None, None, ptr(outk), ptr(outv), B, S, num_heads, int(bool(apply_hadamard)), float(qk_scale))
     return outk, outv
 
 
@@ -589,17 +571,15 @@ def qk_norm_rope_prep_pair(xq: torch.Tensor, xk: torch.Tensor, norm_wq: torch.Te
             raise Q8KernelError("qk_norm_rope_prep_pair: norm weights must be float32 [H*64]")
     outq = torch.empty((B, num_heads, S, 64), dtype=E4M3, device=dev)
     outk = torch.empty((B, num_heads, S, 64), dtype=E4M3, device=dev)
-    with torch.cuda.device(dev):
-        if xv is None:
-            check(lib.q8k_qk_norm_rope_prep_pair(ptr(xq), ptr(xk), xq.stride(1), ptr(norm_wq.contiguous()),
-                                                 ptr(norm_wk.contiguous()), ptr(cos), ptr(sin), ptr(outq), ptr(outk), B, S,
-                                                 num_heads, int(bool(apply_hadamard)), float(qk_scale), stream_ptr(dev)),
-                  "qk_norm_rope_prep_pair")
-            return outq, outk
-        outv = torch.empty((B, num_heads, S, 64), dtype=E4M3, device=dev)
-        check(lib.q8k_qkv_prep(ptr(xq), ptr(xk), ptr(xv), xq.stride(1), ptr(norm_wq.contiguous()),
-                               ptr(norm_wk.contiguous()), ptr(cos), ptr(sin), ptr(outq), ptr(outk), ptr(outv), B, S,
-                               num_heads, int(bool(apply_hadamard)), float(qk_scale), stream_ptr(dev)), "qkv_prep")
+    if xv is None:
+        launch(dev, "qk_norm_rope_prep_pair", lib.q8k_qk_norm_rope_prep_pair, ptr(xq), ptr(xk), xq.stride(1),
+               ptr(norm_wq.contiguous()), ptr(norm_wk.contiguous()), ptr(cos), ptr(sin), ptr(outq), ptr(outk), B, S,
+               num_heads, int(bool(apply_hadamard)), float(qk_scale))
+        return outq, outk
+    outv = torch.empty((B, num_heads, S, 64), dtype=E4M3, device=dev)
+    launch(dev, "qkv_prep", lib.q8k_qkv_prep, ptr(xq), ptr(xk), ptr(xv), xq.stride(1), ptr(norm_wq.contiguous()),
+           ptr(norm_wk.contiguous()), ptr(cos), ptr(sin), ptr(outq), ptr(outk), ptr(outv), B, S, num_heads,
+           int(bool(apply_hadamard)), float(qk_scale))
     return outq, outk, outv
 
 
@@ -613,9 +593,8 @@ def attention_prep_v(v: torch.Tensor) -> torch.Tensor:
         v = v.contiguous()
     s_pad = (S + 15) // 16 * 16
     vt8 = torch.empty((B, H, 64, s_pad), dtype=E4M3, device=dev)
-    with torch.cuda.device(dev):
-        check(lib.q8k_attention_prep_v(ptr(v), ptr(vt8), B, H, S, v.stride(0), v.stride(2), v.stride(1), stream_ptr(dev)),
-              "attention_prep_v")
+    launch(dev, "attention_prep_v", lib.q8k_attention_prep_v, ptr(v), ptr(vt8), B, H, S, v.stride(0), v.stride(2),
+           v.stride(1))
     return vt8
 
 
@@ -629,9 +608,8 @@ def attention_cast_rows(v: torch.Tensor) -> torch.Tensor:
     if v.stride(3) != 1 or any(s % 8 for s in v.stride()[:3]) or v.data_ptr() % 16:
         v = v.contiguous()
     out = torch.empty((B, H, S, 64), dtype=E4M3, device=dev)
-    with torch.cuda.device(dev):
-        check(lib.q8k_attention_cast_rows(ptr(v), ptr(out), B, H, S, v.stride(0), v.stride(2), v.stride(1),
-                                          stream_ptr(dev)), "attention_cast_rows")
+    launch(dev, "attention_cast_rows", lib.q8k_attention_cast_rows, ptr(v), ptr(out), B, H, S, v.stride(0), v.stride(2),
+           v.stride(1))
     return out
 
 
@@ -646,22 +624,21 @@ def linear(x: torch.Tensor, w: torch.Tensor, w_scales: torch.Tensor, bias: Optio
     per-device scratch buffer (q8_kernels/functional/linear.py:24-42,138-159)."""
     dev = require_cuda(x, w, w_scales, bias)
     K = x.shape[-1]
-    x2 = x.reshape(-1, K).contiguous()
-    M, N = x2.shape[0], w.shape[0]
+    x2 = x.contiguous()
+    M, N = x.numel() // K if K else 0, w.shape[0]
     need = lib.q8k_linear_workspace_bytes(M, K)
     if torch.cuda.is_current_stream_capturing():
         # a buffer allocated during capture belongs to that graph's private pool: never cache it
         ws = torch.empty(max(need, 1), dtype=torch.uint8, device=dev)
     else:
-        key = (dev.index, torch.cuda.current_stream(dev).cuda_stream)
+        key = (dev.index, stream_ptr(dev))
         ws = _workspaces.get(key)
         if ws is None or ws.numel() < need:
             ws = torch.empty(max(need, 1), dtype=torch.uint8, device=dev)
             _workspaces[key] = ws
     out_shape = (x.shape[0], x.shape[1], N) if x.dim() == 3 else (1, M, N)
     out = torch.empty(out_shape, dtype=out_type, device=dev)
-    with torch.cuda.device(dev):
-        check(lib.q8k_linear(ptr(x2), dt(x2.dtype), ptr(w), dt(w.dtype), ptr(w_scales), ptr(bias), ptr(out),
-                             dt(out_type), M, N, K, int(bool(use_hadamard)), int(bool(fuse_gelu)), ptr(ws),
-                             ws.numel(), ptr(_lib.status_word(dev)), stream_ptr(dev)), "linear")
+    launch(dev, "linear", lib.q8k_linear, ptr(x2), dt(x2.dtype), ptr(w), dt(w.dtype), ptr(w_scales), ptr(bias),
+           ptr(out), dt(out_type), M, N, K, int(bool(use_hadamard)), int(bool(fuse_gelu)), ptr(ws), ws.numel(),
+           ptr(_lib.status_word(dev)))
     return out

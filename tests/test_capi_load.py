@@ -103,3 +103,29 @@ def test_rope_table_on_cpu_matches_reference_vectors():
     Hp.assert_bit_equal(cos, G.t(d["cos"]), "cos")
     Hp.assert_bit_equal(sin, G.t(d["sin"]), "sin")
     assert torch.equal(q8.blocks.latent_grid(2, 3, 4), G.t(d["grid"]))
+
+
+def _forms():
+    """Contiguous, sliced, transposed, expanded, offset and empty tensors of one to four dims."""
+    base = torch.arange(4 * 6 * 8 * 16, dtype=torch.float32).reshape(4, 6, 8, 16)
+    yield from (base, base[0], base[0, 0], base[0, 0, 0], base[:, 1:5], base[:, :, :, :8], base[..., 8:], base.transpose(1, 2),
+                base.transpose(0, 3), base[::2], base[:, ::3], base[:1].expand(5, 6, 8, 16), base[0, 0, :1].expand(7, 16),
+                base.flatten()[4:4 + 160].view(10, 16), base[:0], base[:, :0], base[:, :, :1, ::2], base.permute(2, 0, 1, 3))
+    yield base.to(torch.bfloat16)[:, :, :, :8]
+
+
+@pytest.mark.parametrize("i", range(19))
+def test_row_arguments_describe_the_same_rows_for_every_layout(i):
+    """What a kernel is told (pointer, rows, dim, row stride) reads back as x.reshape(-1, dim), whether or not the
+    tensor takes the contiguous shortcut."""
+    from q8_kernels_b200 import native
+    x = list(_forms())[i]
+    want = x.reshape(-1, x.shape[-1])
+    t, rows, dim, stride = native._rows(x)
+    assert (rows, dim) == tuple(want.shape) and (rows <= 1 or stride >= dim)
+    got = torch.as_strided(t, (rows, dim), (stride, 1), t.storage_offset())
+    assert torch.equal(got, want)
+    t, rows, dim = native._dense_rows(x)
+    assert (rows, dim) == tuple(want.shape) and t.is_contiguous() and torch.equal(t.reshape(rows, dim), want)
+    c, s, n = native._tables(x, x.clone(), dim)
+    assert n == rows and c.is_contiguous() and s.is_contiguous() and torch.equal(c.reshape(rows, dim), want)
