@@ -1,4 +1,4 @@
-// Pieces shared by the single-CTA and the CTA-pair 8-bit GEMM kernels.
+// Pieces shared by the two 8-bit GEMM kernels.
 #pragma once
 
 #include "common.cuh"
@@ -62,8 +62,14 @@ __device__ __forceinline__ float2 epilogue_pair(uint32_t r0, uint32_t r1, float2
 
 // CTA-pair (cta_group::2) variant: 256 x 256 output tiles per cluster of two CTAs.  Returns
 // Q8K_ERR_UNSUPPORTED (without touching the error detail) when the device cannot co-schedule
-// the clusters, in which case the caller falls back to the single-CTA kernel.
+// the clusters, in which case the caller falls back to the split kernel.
 int launch_gemm_pair(bool int8, bool gelu, bool out_e4m3, bool resid, const void* a, const void* b, const GemmParams& p,
                      int bs_a, int bs_b, cudaStream_t st);
+
+// 128 x bn tiles, each owned by a cluster of sk CTAs that split K (see gemm_split.cu): bn a multiple of 16 up to 256
+// (with sk = 4 of 32), sk 1, 2 or 4 and at most the number of 128-byte K slabs.
+int launch_gemm_split(bool int8, bool gelu, bool out_e4m3, bool resid, const void* a, const void* b, const GemmParams& p,
+                      int bs_a, int bs_b, int bn, int sk, cudaStream_t st);
+inline int split_a_rows(int M) { return M >= kGemmBM ? kGemmBM : (M + 7) / 8 * 8; }   // rows of A that a tile loads
 
 }  // namespace q8k

@@ -1,19 +1,19 @@
 // CTA-pair variant of the 8-bit GEMM: a cluster of two CTAs on neighbouring SMs owns a 256 x 256
 // output tile and runs ONE tcgen05.mma (cta_group::2, M = 256, N = 256, K = 32) per K slice.
 //
-// Why: in the single-CTA kernel every MMA streams a 128-row A slab and a 256-row B slab out of the
+// Why: with one CTA per 128 x 256 tile every MMA streams a 128-row A slab and a 256-row B slab out of the
 // CTA's shared memory, and TMA writes the same 48 KB per stage into it; shared memory bandwidth is
 // what caps the main loop.  In a pair each CTA holds its own 128 rows of A and only HALF of the B
 // rows (128 of 256), so both the TMA fill and the tensor-core reads per CTA drop by a third while
 // the pair produces twice the output.
 //
-// Roles per CTA (10 warps, same as the single-CTA kernel):
+// Roles per CTA (10 warps):
 //   warp 0     TMA producer: its A rows and its half of the B rows, 32 KB per stage, 6 stages; the
 //              transaction bytes of BOTH CTAs are credited to the leader CTA's "full" barrier
 //   warp 1     TMEM allocation (both CTAs); in the leader (even rank) one thread issues the MMAs
 //              and commits to the "empty" / "accumulator full" barriers of both CTAs
-//   warps 2-9  epilogue of the CTA's own 128 rows x 256 columns (identical arithmetic to the
-//              single-CTA kernel); "accumulator free" arrivals of both CTAs go to the leader.
+//   warps 2-9  epilogue of the CTA's own 128 rows x 256 columns; "accumulator free" arrivals of both
+//              CTAs go to the leader.
 //              Output leaves through shared memory: each warp writes its 32 x 32 chunk into a
 //              swizzled staging box and one lane hands it to a TMA store, so global memory sees
 //              whole 32/64-byte row segments instead of 32 row-strided 16-byte stores per

@@ -165,3 +165,41 @@ def test_gemm_argument_errors(nat, cuda_device):
     with pytest.raises(Q8KernelError, match="Batch missmatch"):
         nat.q8_mm(torch.zeros(2, 8, 64, dtype=torch.int8, device=d), torch.zeros(3, 16, 64, dtype=torch.int8, device=d),
                   torch.ones(2, 8, device=d), torch.ones(3, 16, device=d), False, torch.bfloat16)
+
+
+@pytest.mark.parametrize("kind", ["int8", "fp8"])
+@pytest.mark.parametrize("B,M,N,K", [(1, 1, 16, 16), (1, 7, 48, 112), (2, 9, 2064, 640), (1, 77, 10240, 1040), (1, 127, 144, 4112),
+                                     (1, 128, 2048, 2048), (3, 129, 272, 272), (1, 300, 2048, 2048), (1, 512, 2064, 8208),
+                                     (2, 260, 1040, 1024), (1, 4000, 128, 512), (1, 1000, 96, 144)])
+def test_split_tiles_and_split_k(nat, cuda_device, kind, B, M, N, K):
+    """Tiles of every width, K split over 1, 2 and 4 CTAs with uneven shares, row / column / K tails, batches, and each
+    epilogue.  INT8 partial sums are exact, so only the fp32 epilogue may round differently from float64; FP8 sums are
+    fp32 in another order.  Bounds: half a bf16 step (2^-9) and, for GELU, tanh.approx (2^-11) on top of it."""
+    qd = torch.int8 if kind == "int8" else E4M3
+    g = Hp.gen(M + N + K)
+    if kind == "int8":
+        a = torch.randint(-127, 128, (B, M, K), generator=g, dtype=torch.int8)
+        w = torch.randint(-127, 128, (N, K), generator=g, dtype=torch.int8)
+    else:
+        a, w = torch.randn(B, M, K, generator=g).to(qd), torch.randn(N, K, generator=g).to(qd)
+    sa = torch.rand(B, M, generator=g) * 0.01 + 0.001
+    sw = torch.rand(N, generator=g) * 0.01 + 0.001
+    bias = torch.randn(N, generator=g) * 0.1
+    d = cuda_device
+    ad, wd, sad, swd, bd = (t.to(d) for t in (a, w, sa, sw, bias))
+    y = (ad.double() @ wd.double().T) * sad.double().unsqueeze(-1) * swd.double() + bd.double()
+    mm, mmb = (nat.q8_mm, nat.q8_mm_bias) if kind == "int8" else (nat.fp8_mm, nat.fp8_mm_bias)
+    out = mmb(ad, wd, bd, sad, swd, False, torch.bfloat16)
+    err = (out.double() - y).abs()
+    assert bool((err <= 2.0 ** -8 * y.abs() + 2e-6 * y.abs().max()).all())
+    ge = torch.nn.functional.gelu(y, approximate="tanh")
+    out = mmb(ad, wd, bd, sad, swd, True, torch.bfloat16)
+    assert bool(((out.double() - ge).abs() <= 2.0 ** -8 * ge.abs() + 2.0 ** -10 * y.abs() + 2e-6 * y.abs().max()).all())
+    out8 = mm(ad, wd, sad, swd, False, None)
+    y8 = (y - bd.double()).clamp(-448, 448)
+    assert bool(((out8.double() - y8).abs() <= 2.0 ** -3.9 * y8.abs() + 2.0 ** -9).all())
+    gate = torch.randn(B, 1, N, generator=g).to(torch.bfloat16).to(d)
+    resid = torch.randn(B, M, N, generator=g).to(torch.bfloat16).to(d)
+    lin = mmb(ad, wd, bd, sad, swd, False, torch.bfloat16)
+    fused = nat.mm_gate_residual(ad, wd, bd, sad, swd, gate, resid)
+    Hp.assert_bit_equal(fused, (gate * lin + resid).cpu(), "gate and residual in the epilogue")
