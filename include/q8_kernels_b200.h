@@ -68,6 +68,18 @@ Q8K_API const char* q8k_last_error_detail(void);
 Q8K_API int q8k_tokenwise_quant(const void* x, int x_dtype, void* q, int q_dtype, float* scales,
                         int64_t rows, int dim, int64_t x_row_stride, void* stream);
 
+/* The weight operand of the linear backward passes: x [N, K], either int8 / e4m3 with row_scales[N] or bf16
+ * (row_scales NULL), is dequantised in fp32, transposed and quantised per row of the result: q [K, N] e4m3,
+ * scales [K].  Bit-identical to q8k_tokenwise_quant of the dequantised, transposed matrix.  N and K multiples
+ * of 16.  Replaces the chain in q8_kernels/functional/linear.py:44-53,105-133,161-178.                     */
+Q8K_API int q8k_transpose_quant(const void* x, int x_dtype, const float* row_scales, void* q, float* scales,
+                        int N, int K, void* stream);
+
+/* out = bf16(hadamard(bf16(x * row_scales[row])) * scale) for int8 rows of 257 .. 16384 elements: the rotated
+ * weight of the low-rank adapter's backward pass (q8_kernels/functional/linear.py:105-133).               */
+Q8K_API int q8k_dequant_hadamard(const void* x, const float* row_scales, void* out, int64_t rows, int dim,
+                         float scale, void* stream);
+
 /* Fast Walsh-Hadamard transform of every row (zero-padded to the next power of
  * two, fp32 butterflies in ascending stride order), out = cast(y * scale).
  * x bf16|e4m3, out bf16|e4m3; dim a multiple of 8, at most 16384.

@@ -34,6 +34,8 @@ SIGNATURES = {
     "q8k_last_error_detail": (ctypes.c_char_p, []),
     "q8k_wait_selftest": (_c_int, [_c_ptr, ctypes.c_uint, _c_ptr]),
     "q8k_tokenwise_quant": (_c_int, [_c_ptr, _c_int, _c_ptr, _c_int, _c_ptr, _c_i64, _c_int, _c_i64, _c_ptr]),
+    "q8k_transpose_quant": (_c_int, [_c_ptr, _c_int, _c_ptr, _c_ptr, _c_ptr, _c_int, _c_int, _c_ptr]),
+    "q8k_dequant_hadamard": (_c_int, [_c_ptr, _c_ptr, _c_ptr, _c_i64, _c_int, _c_f32, _c_ptr]),
     "q8k_fast_hadamard_transform": (_c_int, [_c_ptr, _c_int, _c_ptr, _c_int, _c_i64, _c_int, _c_i64, _c_f32, _c_ptr]),
     "q8k_hadamard_quant": (_c_int, [_c_ptr, _c_int, _c_ptr, _c_int, _c_ptr, _c_i64, _c_int, _c_i64, _c_f32, _c_ptr]),
     "q8k_norm_modulate_quant": (_c_int, [_c_ptr, _c_ptr, _c_ptr, _c_ptr, _c_int, _c_ptr, _c_i64, _c_int, _c_i64, _c_f32,

@@ -206,6 +206,7 @@ __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wai
 // of the separate ops it replaces: n = bf16(x * rsqrt(mean x^2)); u = bf16(bf16(n * bf16(1 + s)) + h)
 // where s, h are the per-batch modulation rows (bf16 [rows / rows_per_mod, dim]).  A CTA stays inside one batch entry
 // and keeps its two modulation rows in shared memory.
+// int8 rows (Cast only) are dequantised on the way in: v = bf16(q * scales[row]), the weight of a backward pass.
 // FULL: dim is the power of two itself, so no element of a row needs a bounds test.
 
 // Raw staging: position of the 16-byte chunk c (row order) of a row whose threads own CPT chunks each, such
@@ -273,6 +274,8 @@ __global__ void __launch_bounds__(StreamGeo<Tin, LOG_N, NORM_MOD>::THREADS, Stre
 hadamard_stream_kernel(const Tin* __restrict__ x, Tout* __restrict__ out, float* __restrict__ scales, unsigned rows, int dim,
                        int64_t x_row_stride, float scale, const __nv_bfloat16* __restrict__ mod_scale,
                        const __nv_bfloat16* __restrict__ mod_shift, unsigned rows_per_mod, unsigned blocks_per_mod) {
+    constexpr bool DEQ = std::is_same_v<Tin, int8_t>;
+    static_assert(!DEQ || EPI == Epilogue::Cast, "int8 rows are only transformed, not quantised again");
     using Geo = StreamGeo<Tin, LOG_N, NORM_MOD>;
     constexpr int N = Geo::N, V = Geo::V, T = Geo::T, UNIT = Geo::UNIT, RPU = Geo::RPU, LOG_V = Geo::LOG_V;
     constexpr int B1 = Geo::B1, B2 = Geo::B2;
@@ -359,7 +362,15 @@ hadamard_stream_kernel(const Tin* __restrict__ x, Tout* __restrict__ out, float*
 #pragma unroll
                     for (int i = 0; i < 4; ++i) {
                         float f[4];
-                        e4m3x4_to_float(w[i], f);
+                        if constexpr (DEQ) {
+                            const float rs = row_ok ? scales[row] : 0.f;
+#pragma unroll
+                            for (int j = 0; j < 4; ++j) f[j] = __fmul_rn((float)(int8_t)(w[i] >> (8 * j)), rs);
+                            round_through_bf16x2(f[0], f[1]);
+                            round_through_bf16x2(f[2], f[3]);
+                        } else {
+                            e4m3x4_to_float(w[i], f);
+                        }
 #pragma unroll
                         for (int j = 0; j < 4; ++j) v[k * 8 + i * 4 + j] = f[j];
                     }
@@ -668,6 +679,25 @@ extern "C" int q8k_fast_hadamard_transform(const void* x, int x_dtype, void* out
     if (x_dtype == Q8K_DT_E4M3 && out_dtype == Q8K_DT_BF16) return launch_hadamard<e4m3_t, __nv_bfloat16, C>(x, out, nullptr, rows, dim, x_row_stride, scale, st, op);
     if (x_dtype == Q8K_DT_E4M3 && out_dtype == Q8K_DT_E4M3) return launch_hadamard<e4m3_t, e4m3_t, C>(x, out, nullptr, rows, dim, x_row_stride, scale, st, op);
     set_error_detail("%s: output dtype %d is not bf16 or e4m3", op, out_dtype);
+    return Q8K_ERR_UNSUPPORTED;
+}
+
+extern "C" int q8k_dequant_hadamard(const void* x, const float* row_scales, void* out, int64_t rows, int dim, float scale,
+                                    void* stream) {
+    const char* op = "dequant_hadamard";
+    Q8K_REQUIRE(rows >= 0 && rows <= 0x7fffffffLL, Q8K_ERR_INVALID_ARG, "%s: rows %lld out of range", op, (long long)rows);
+    Q8K_REQUIRE(dim > 256 && dim <= 16384 && dim % 8 == 0, Q8K_ERR_UNSUPPORTED, "%s: dim %d not a multiple of 8 in (256, 16384]", op, dim);
+    if (rows == 0) return Q8K_OK;
+    Q8K_REQUIRE(x && row_scales && out && aligned16(x) && aligned16(out), Q8K_ERR_INVALID_ARG, "%s: null or misaligned pointer", op);
+    float* rs = const_cast<float*>(row_scales);                // read only: the kernel's scales argument is an output otherwise
+    const int8_t* xi = (const int8_t*)x;
+    __nv_bfloat16* o = (__nv_bfloat16*)out;
+    cudaStream_t st = (cudaStream_t)stream;
+    int log_n = 9;
+    while ((1 << log_n) < dim) ++log_n;
+#define Q8K_DH(LN) case LN: return launch_stream<int8_t, __nv_bfloat16, LN, Epilogue::Cast, false>(xi, o, rs, rows, dim, dim, scale, nullptr, nullptr, 1, st)
+    switch (log_n) { Q8K_DH(9); Q8K_DH(10); Q8K_DH(11); Q8K_DH(12); Q8K_DH(13); Q8K_DH(14); }
+#undef Q8K_DH
     return Q8K_ERR_UNSUPPORTED;
 }
 

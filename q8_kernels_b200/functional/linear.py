@@ -117,6 +117,17 @@ def _dequant_t(b: torch.Tensor, scale_b: torch.Tensor, dtype: torch.dtype) -> to
     return (b.to(dtype) * scale_b[:, None]).T
 
 
+def _weight_operand(b: torch.Tensor, scale_b: torch.Tensor, dtype: torch.dtype):
+    """``quantize_fp8(_dequant_t(b, scale_b, dtype).contiguous())``: for a [N,K] weight with fp32 row scales in one
+    kernel (its fp32 products do not depend on ``dtype``: every 8-bit value is exact in 16 bits).  The bounds are those
+    of the two kernels: multiples of 16, and rows that the row quantizer takes."""
+    if (b.dim() == 2 and b.dtype in (torch.int8, E4M3) and is_16bit(dtype) and scale_b.dtype == torch.float32
+            and scale_b.dim() == 1 and b.shape[0] % 16 == 0 and b.shape[1] % 16 == 0 and 0 < b.shape[0] <= 16384
+            and b.shape[1] > 0):
+        return native.transpose_quant(b, scale_b)
+    return quantize_fp8(_dequant_t(b, scale_b, dtype).contiguous())
+
+
 class Q8LinearFunc(torch.autograd.Function):
     """q8_kernels/functional/linear.py:24-53."""
 
@@ -132,7 +143,7 @@ class Q8LinearFunc(torch.autograd.Function):
     def backward(ctx, grad_output):
         b, scale_b = ctx.saved_tensors
         g8, gs = quantize_fp8(grad_output.contiguous())
-        w8, ws = quantize_fp8(_dequant_t(b, scale_b, ctx.out_dtype).contiguous())
+        w8, ws = _weight_operand(b, scale_b, ctx.out_dtype)
         grad_x = hadamard_transform(native.fp8_mm(g8, w8, gs, ws, False, ctx.out_dtype))
         return grad_x, None, None, None, None, None, None
 
@@ -154,10 +165,12 @@ class FP8LinearFunc(torch.autograd.Function):
     def backward(ctx, grad_output):
         b, scale_b = ctx.saved_tensors
         g8, gs = quantize_fp8(grad_output.contiguous())
-        w = _dequant_t(b, scale_b, ctx.out_dtype)
-        # the reference rotates and THEN transposes here (linear.py:165), which only type-checks for
-        # square weights; kept as it is
-        w8, ws = quantize_fp8((hadamard_transform(w.contiguous()).T if ctx.use_hadamard else w).contiguous())
+        if ctx.use_hadamard:
+            # the reference rotates and THEN transposes here (linear.py:165), which only type-checks for
+            # square weights; kept as it is
+            w8, ws = quantize_fp8(hadamard_transform(_dequant_t(b, scale_b, ctx.out_dtype).contiguous()).T.contiguous())
+        else:
+            w8, ws = _weight_operand(b, scale_b, ctx.out_dtype)
         grad_x = native.fp8_mm(g8, w8, gs, ws, False, ctx.out_dtype)
         return grad_x, None, None, None, None, None, None
 
@@ -200,11 +213,16 @@ class Q8LinearLora(torch.autograd.Function):
         if ctx.fuse_gelu:
             grad_output = native.gelu_backward(o, grad_output, out_dtype)
         grad_out_lora_b = grad_output @ lora_b                                  # [.., s, d] @ [d, r]
-        w = (b * scale_b[:, None]).to(out_dtype)
         if not ctx.use_hadamard:
             raise NotImplementedError("q8_linear_lora backward: only use_hadamard=True is defined "
                                       "(the reference's other branch reads an unset variable)")
-        w8, ws = quantize_fp8(hadamard_transform(w).T.contiguous())
+        if (out_dtype == torch.bfloat16 and b.dim() == 2 and scale_b.dtype == torch.float32 and scale_b.dim() == 1
+                and b.shape[0] % 16 == 0 and 0 < b.shape[0] <= 16384 and b.shape[1] % 16 == 0 and 256 < b.shape[1] <= 16384):
+            # dequantise + rotate, then transpose + quantise: two kernels, same bits as the chain below
+            w8, ws = native.transpose_quant(native.dequant_hadamard(b, scale_b, 1 / math.sqrt(b.shape[1])), None)
+        else:
+            w = (b * scale_b[:, None]).to(out_dtype)
+            w8, ws = quantize_fp8(hadamard_transform(w).T.contiguous())
         g8, gs = quantize_fp8(grad_output.contiguous())
         grad_x = native.fp8_mm(g8, w8, gs, ws, False, out_dtype).reshape(a.shape) + grad_out_lora_b @ lora_a
         grad_lora_a = grad_out_lora_b.transpose(-1, -2) @ a                     # [.., r, s] @ [.., s, h]

@@ -69,6 +69,37 @@ def tokenwise_quant(x: torch.Tensor, out_type: Optional[torch.dtype] = None) -> 
     return [q, scales]
 
 
+def transpose_quant(x: torch.Tensor, row_scales: Optional[torch.Tensor]) -> List[torch.Tensor]:
+    """``tokenwise_quant((x * row_scales[:, None]).T.contiguous(), e4m3)`` in one pass, bit-identical: the weight
+    operand of the linear backward passes.  x [N,K] int8 / e4m3 with fp32 ``row_scales`` [N], or bf16 with None;
+    returns ``[q, scales]`` with q e4m3 [K,N] and fp32 scales [K].  N and K must be multiples of 16."""
+    dev = require_cuda(x, row_scales)
+    if x.dim() != 2:
+        raise Q8KernelError("transpose_quant: x must be [N,K]")
+    if row_scales is not None and (row_scales.dtype != torch.float32 or row_scales.numel() != x.shape[0]):
+        raise Q8KernelError("transpose_quant: row_scales must be float32 [N]")
+    n, k = x.shape
+    x = x.contiguous()
+    row_scales = None if row_scales is None else row_scales.contiguous()
+    q = torch.empty((k, n), dtype=E4M3, device=dev)
+    scales = torch.empty((k,), dtype=torch.float32, device=dev)
+    launch(dev, "transpose_quant", lib.q8k_transpose_quant, ptr(x), dt(x.dtype), ptr(row_scales), ptr(q), ptr(scales), n, k)
+    return [q, scales]
+
+
+def dequant_hadamard(x: torch.Tensor, row_scales: torch.Tensor, scale: float) -> torch.Tensor:
+    """``fast_hadamard_transform((x * row_scales[:, None]).to(bfloat16), scale)`` for int8 x [N,K] with fp32
+    ``row_scales`` [N] and 256 < K <= 16384 in one pass, bit-identical."""
+    dev = require_cuda(x, row_scales)
+    if x.dtype != torch.int8 or x.dim() != 2 or row_scales.dtype != torch.float32 or row_scales.numel() != x.shape[0]:
+        raise Q8KernelError("dequant_hadamard: x must be int8 [N,K] with float32 row_scales [N]")
+    x, row_scales = x.contiguous(), row_scales.contiguous()
+    out = torch.empty(x.shape, dtype=torch.bfloat16, device=dev)
+    launch(dev, "dequant_hadamard", lib.q8k_dequant_hadamard, ptr(x), ptr(row_scales), ptr(out), x.shape[0], x.shape[1],
+           float(scale))
+    return out
+
+
 # ---------------------------------------------------------------- ops._C
 
 def fast_hadamard_transform(x: torch.Tensor, scale: float, out_type: Optional[torch.dtype] = None) -> torch.Tensor:

@@ -285,3 +285,35 @@ def test_autograd_rules_use_the_backward_kernels(nat, cuda_device):
     rot = torch.stack((-t[..., 1], t[..., 0]), dim=-1).reshape(1, 16, dim)
     (x2f * cos + rot * sin).backward(g.view(1, 16, dim).float())
     assert Hp.rel_fro(x2.grad.float(), x2f.grad) < 5e-3
+
+
+@pytest.mark.parametrize("N,K", [(16, 16), (48, 272), (1024, 512), (1040, 2064), (2048, 2048), (4112, 528), (8192, 1024)])
+@pytest.mark.parametrize("kind", ["int8", "e4m3", "bf16"])
+def test_transpose_quant_equals_the_op_chain(nat, cuda_device, N, K, kind):
+    """One pass against dequantise, transpose, row quantizer: the same bytes, with a zero column, tiny and large ones."""
+    g = Hp.gen(N + K)
+    w = torch.randn(N, K, generator=g)
+    w[:, 0] = 0
+    w[:, 1] *= 1e-30 if kind == "bf16" else 1
+    sc = (torch.rand(N, generator=g) * 0.1 + 1e-3).to(cuda_device)
+    if kind == "int8":
+        x = (w * 40).round().clamp(-127, 127).to(torch.int8).to(cuda_device)
+    else:
+        x = w.to(E4M3 if kind == "e4m3" else torch.bfloat16).to(cuda_device)
+    if kind == "bf16":
+        q, s = nat.transpose_quant(x, None)
+        q_ref, s_ref = nat.tokenwise_quant(x.T.contiguous(), E4M3)
+    else:
+        q, s = nat.transpose_quant(x, sc)
+        q_ref, s_ref = nat.tokenwise_quant((x.to(torch.bfloat16) * sc[:, None]).T.contiguous(), E4M3)
+    Hp.assert_bit_equal(q, q_ref.cpu(), "bytes")
+    Hp.assert_bit_equal(s, s_ref.cpu(), "scales")
+
+
+@pytest.mark.parametrize("N,K", [(3, 512), (9475, 264), (700, 2048), (33, 1544), (5, 8192), (2, 16384)])
+def test_dequant_hadamard_equals_the_op_chain(nat, cuda_device, N, K):
+    g = Hp.gen(N + K)
+    x = torch.randint(-128, 128, (N, K), generator=g, dtype=torch.int8).to(cuda_device)
+    sc = (torch.rand(N, generator=g) * 0.1 + 1e-3).to(cuda_device)
+    ref = nat.fast_hadamard_transform((x * sc[:, None]).to(torch.bfloat16), 1 / math.sqrt(K), None)
+    Hp.assert_bit_equal(nat.dequant_hadamard(x, sc, 1 / math.sqrt(K)), ref.cpu(), "rotated weight")
