@@ -50,7 +50,34 @@ inline int allow_dynamic_smem(const void* kern, int bytes, std::atomic<uint64_t>
     return Q8K_OK;
 }
 
+// Launch as a programmatic dependent of whatever runs before it on the stream: the kernel may become resident while its
+// predecessor drains, so the launch latency and everything it does before pdl_wait() are hidden.  The kernel must call
+// pdl_wait() in every thread before it touches global memory.  cluster > 1: CTAs per cluster along x.
+template <typename... KArgs, typename... Args>
+inline cudaError_t launch_dependent(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, int cluster,
+                                    Args... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = cluster; attr[1].val.clusterDim.y = 1; attr[1].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = cluster > 1 ? 2 : 1;
+    return cudaLaunchKernelEx(&cfg, kern, KArgs(args)...);
+}
+
 inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
+
+// ---------------------------------------------------------------- programmatic dependent launch
+// Wait until the kernels this one depends on have completed and their writes are visible (at once when it was launched
+// without the attribute), then let the next kernel on the stream become resident as soon as every CTA has got here.
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 // ---------------------------------------------------------------- element types
 struct e4m3_t { uint8_t bits; };

@@ -86,6 +86,7 @@ gemm_8bit_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
     extern __shared__ __align__(1024) uint8_t smem[];
     const uint32_t smem_base = ptx::smem_u32(smem);
     if (smem_base & 1023u) {                                   // same offset in both CTAs: both leave
+        pdl_wait();
         if (threadIdx.x == 0 && p.status != nullptr) atomicExch(p.status, Q8K_STATUS_TIMEOUT | (11 << 8));
         return;
     }
@@ -108,19 +109,6 @@ gemm_8bit_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
     const int warp = threadIdx.x >> 5;
     const int lane = threadIdx.x & 31;
     const int k_iters = (p.K + kGemmBK - 1) / kGemmBK;
-
-    // A launch that follows a failed one on the same status word does nothing.  The leader reads
-    // the word and hands its decision to the peer, so the two CTAs of a pair always agree.
-    volatile int* prior_failure = reinterpret_cast<volatile int*>(smem + L::kPriorOffset);
-    if (threadIdx.x == 0 && leader) {
-        const int v = p.status != nullptr ? *reinterpret_cast<volatile int*>(p.status) : 0;
-        *prior_failure = v;
-        asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(ptx::mapa_shared(smem_base + L::kPriorOffset, 1)), "r"(v)
-                     : "memory");
-    }
-    ptx::cluster_sync_all();
-    const bool skip = *prior_failure != 0;
-    if (skip) return;
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < kPairStages; ++s) {
@@ -149,17 +137,30 @@ gemm_8bit_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
         ptx::tmem_alloc_pair<kPairTmemCols>(ptx::smem_u32(const_cast<uint32_t*>(tmem_ptr_smem)));
         ptx::tmem_relinquish_alloc_permit_pair();
     }
+    pdl_wait();                                                // everything above overlaps the kernel before
+    // A launch that follows a failed one on the same status word does nothing.  The leader reads
+    // the word and hands its decision to the peer, so the two CTAs of a pair always agree.
+    volatile int* prior_failure = reinterpret_cast<volatile int*>(smem + L::kPriorOffset);
+    if (threadIdx.x == 0 && leader) {
+        const int v = p.status != nullptr ? *reinterpret_cast<volatile int*>(p.status) : 0;
+        *prior_failure = v;
+        asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(ptx::mapa_shared(smem_base + L::kPriorOffset, 1)), "r"(v)
+                     : "memory");
+    }
     ptx::tcgen05_fence_before_sync();
     __syncthreads();
     ptx::cluster_sync_all();                                   // both CTAs' barriers exist before anyone signals across
     ptx::tcgen05_fence_after_sync();
+    pdl_release();                                             // this CTA holds its TMEM: the next kernel may move in behind it
+    const bool skip = *prior_failure != 0;
     const uint32_t tmem_base = *tmem_ptr_smem;
 
     // barriers of the leader CTA, as seen from this CTA
     const uint32_t leader_full0 = ptx::mapa_shared(full_bar(0), 0);
     auto leader_tmem_empty_bar = [&](int a) { return ptx::mapa_shared(tmem_empty_bar(a), 0); };
 
-    if (warp == 0) {
+    if (skip) {
+    } else if (warp == 0) {
         // ------------------------------------------------ TMA producer (both CTAs)
         if (ptx::elect_one()) {
             int s = 0;
@@ -505,8 +506,7 @@ static int launch_pair(const CUtensorMap& ta, const CUtensorMap& tb, const CUten
     }
     if (max_clusters < 8) return Q8K_ERR_UNSUPPORTED;
     const int clusters = pp.total_tiles2 < max_clusters ? pp.total_tiles2 : max_clusters;
-    kern<<<2 * clusters, kGemmThreads, PairSmem::kDynamic, st>>>(ta, tb, tc, tr, pp);
-    Q8K_CUDA_OK(cudaGetLastError());
+    Q8K_CUDA_OK(launch_dependent(kern, 2 * clusters, kGemmThreads, PairSmem::kDynamic, st, 1, ta, tb, tc, tr, pp));
     return Q8K_OK;
 }
 

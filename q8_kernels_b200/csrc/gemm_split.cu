@@ -141,7 +141,6 @@ gemm_8bit_split_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_
     const int n0 = n_blk * bn;
 
     if (threadIdx.x == 0) {
-        prior_failure = p.status != nullptr ? *reinterpret_cast<volatile int*>(p.status) : 0;
         for (int s = 0; s < stages; ++s) {
             ptx::mbar_init(full_bar(s), 1);
             ptx::mbar_init(empty_bar(s), 1);
@@ -157,9 +156,12 @@ gemm_8bit_split_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_
         split_tmem_any(bn, true, ptx::smem_u32(const_cast<uint32_t*>(tmem_ptr_smem)));
         ptx::tmem_relinquish_alloc_permit();
     }
+    pdl_wait();                                                // everything above overlaps the kernel before
+    if (threadIdx.x == 0) prior_failure = p.status != nullptr ? *reinterpret_cast<volatile int*>(p.status) : 0;
     ptx::tcgen05_fence_before_sync();
     __syncthreads();
     ptx::tcgen05_fence_after_sync();
+    pdl_release();                                             // this CTA holds its TMEM: the next kernel may move in behind it
     const uint32_t tmem_base = *tmem_ptr_smem;
     bool ok = prior_failure == 0;
 
@@ -310,17 +312,7 @@ static int launch_split(const CUtensorMap& ta, const CUtensorMap& tb, const Spli
     auto kern = gemm_8bit_split_kernel<INT8, GELU, OUT_E4M3, RESID>;
     static std::atomic<uint64_t> smem_done{0};
     if (int rc = allow_dynamic_smem((const void*)kern, 226 * 1024, smem_done)) return rc;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)sp.g.total_tiles * (unsigned)sp.sk);
-    cfg.blockDim = dim3(kGemmThreads);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = st;
-    cudaLaunchAttribute attr;
-    attr.id = cudaLaunchAttributeClusterDimension;
-    attr.val.clusterDim.x = sp.sk; attr.val.clusterDim.y = 1; attr.val.clusterDim.z = 1;
-    cfg.attrs = &attr;
-    cfg.numAttrs = sp.sk > 1 ? 1 : 0;
-    Q8K_CUDA_OK(cudaLaunchKernelEx(&cfg, kern, ta, tb, sp));
+    Q8K_CUDA_OK(launch_dependent(kern, (unsigned)sp.g.total_tiles * (unsigned)sp.sk, kGemmThreads, smem, st, sp.sk, ta, tb, sp));
     return Q8K_OK;
 }
 

@@ -321,6 +321,8 @@ hadamard_stream_kernel(const Tin* __restrict__ x, Tout* __restrict__ out, float*
         }
         cp_async_commit();
     };
+    pdl_wait();
+    pdl_release();
     load_rows(rel);
 
     __nv_bfloat16* mod_smem = reinterpret_cast<__nv_bfloat16*>(stream_smem + Geo::UNITS * (Geo::RAW + Geo::XCH));
@@ -595,9 +597,8 @@ static int launch_stream(const Tin* x, Tout* out, float* scales, int64_t rows, i
     const int64_t need = (group_rows + per_cta - 1) / per_cta;
     int64_t blocks = slots / groups < 1 ? 1 : slots / groups;
     if (blocks > need) blocks = need;
-    kern<<<(unsigned)(blocks * groups), Geo::THREADS, Geo::SMEM, st>>>(x, out, scales, (unsigned)rows, dim, stride, scale, ms, mh,
-                                                                      (unsigned)group_rows, (unsigned)blocks);
-    Q8K_CUDA_OK(cudaGetLastError());
+    Q8K_CUDA_OK(launch_dependent(kern, (unsigned)(blocks * groups), Geo::THREADS, Geo::SMEM, st, 1, x, out, scales, (unsigned)rows,
+                                 dim, stride, scale, ms, mh, (unsigned)group_rows, (unsigned)blocks));
     return Q8K_OK;
 }
 

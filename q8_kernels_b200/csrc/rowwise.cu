@@ -57,6 +57,8 @@ __global__ void __launch_bounds__(T)
 tokenwise_quant_kernel(const Tin* __restrict__ x, Tout* __restrict__ q, float* __restrict__ scales,
                        int dim, int64_t x_row_stride) {
     __shared__ float red[32];
+    pdl_wait();
+    pdl_release();
     const int64_t row = blockIdx.x;
     const Tin* xr = x + row * x_row_stride;
     Tout* qr = q + row * (int64_t)dim;
@@ -439,8 +441,8 @@ static int launch_quant(const void* x, void* q, float* scales, int64_t rows, int
                         int64_t stride, cudaStream_t st) {
     const int items = dim / kItem;
 #define Q8K_Q_LAUNCH(ITEMS, T)                                                                  \
-    tokenwise_quant_kernel<Tin, Tout, ITEMS, T><<<(unsigned)rows, T, 0, st>>>(                   \
-        (const Tin*)x, (Tout*)q, scales, dim, stride)
+    Q8K_CUDA_OK(launch_dependent(tokenwise_quant_kernel<Tin, Tout, ITEMS, T>, (unsigned)rows, T, 0, st, 1,     \
+                                 (const Tin*)x, (Tout*)q, scales, dim, stride))
     if (items <= 32)        Q8K_Q_LAUNCH(1, 32);
     else if (items <= 128)  Q8K_Q_LAUNCH(1, 128);
     else if (items <= 256)  Q8K_Q_LAUNCH(2, 128);
