@@ -8,7 +8,7 @@
 // or e4m3 (saturating).
 //
 // This file checks the arguments and chooses between the two kernels: 256 x 256 tiles on CTA pairs (gemm_pair.cu) and
-// 128 x bn tiles with K split over clusters (gemm_split.cu).
+// 128 x bn tiles, for int8 with K split over clusters (gemm_split.cu).
 
 #include "gemm_common.cuh"
 
@@ -35,18 +35,21 @@ int gemm_num_sms() {
 //          threads) and its bytes at 140 GB/s (one SM's L2 port; 1.7 x the bytes where K is not a multiple of 128 and
 //          rows straddle cache lines), times the CTAs of the busiest SM, and 1.5 for every CTA beyond the first there; 3.85e-5 bn^2 for the epilogue; the exchange of a K split; 0.06 per MB of weights
 //   pair:  6.5 + 0.31 per slab and wave of 74 tiles
-// Examples (pair or 128 x 128 tiles before -> now): FP8 M = 128, N = K = 2048 10.3 -> 7.2 (bn 32, sk 2);  M = 77, N =
-// 10240, K = 4096 15.7 -> 12.5 (bn 80);  M = 128, N = 2048, K = 8192 23.7 -> 10.1 (bn 64, sk 4);  M = 1024, N = 2048,
-// K = 8192 26.0 -> 19.7 (bn 128).  At N = K = 2048 the line to the pair kernel lies between M = 1024 (11.8 -> 9.7) and
-// M = 2048 (12.6 against 14.9).
+// Examples, int8 (pair or 128 x 128 tiles before -> now): M = 128, N = K = 2048 9.5 -> 5.2 (bn 32);  M = 77, N = 10240,
+// K = 4096 15.4 -> 11.6 (bn 80);  M = 128, N = 2048, K = 8192 23.1 -> 9.0 (bn 64, sk 4);  M = 1024, N = 2048, K = 8192
+// 26.2 -> 18.0 (bn 128).  At N = K = 2048 the line to the pair kernel lies between M = 1024 (12.2 -> 8.4) and M = 2048
+// (12.6 against 14.9).
+// Only int8 splits K: its partial sums are exact.  fp32 partials would round in another order than one accumulator,
+// and an fp8 row would then have other bits in a call with other M or N (it has the same in every call, and stacked
+// weights give the bits of the separate ones).
 struct SplitChoice { bool use; int bn, sk; };
-static SplitChoice choose_split(int M, int N, int K, int batch, int sms) {
+static SplitChoice choose_split(bool int8, int M, int N, int K, int batch, int sms) {
     const int iters = (K + kGemmBK - 1) / kGemmBK;
     const double m_tiles = (double)((M + kGemmBM - 1) / kGemmBM) * batch;
     const int a_rows = split_a_rows(M);
     SplitChoice c = {true, 128, 1};
     double best = 1e30;
-    for (int sk = 1; sk <= 4; sk *= 2) {
+    for (int sk = 1; sk <= (int8 ? 4 : 1); sk *= 2) {
         if (iters < 2 * sk && sk > 1) break;
         for (int bn = 32; bn <= 256; bn += sk == 4 ? 32 : 16) {
             if (bn > 32 && bn - 16 >= N) break;
@@ -107,7 +110,7 @@ static int gemm_8bit(bool int8, const void* a, const void* b, const float* bias,
         Q8K_REQUIRE(!gelu && !e4m3, Q8K_ERR_UNSUPPORTED, "%s: the gate/residual tail needs a bf16 output without GELU", op);
         Q8K_REQUIRE(aligned16(resid) && aligned16(gate), Q8K_ERR_INVALID_ARG, "%s: gate and residual must be 16-byte aligned", op);
     }
-    const SplitChoice choice = choose_split(M, N, K, batch, gemm_num_sms());
+    const SplitChoice choice = choose_split(int8, M, N, K, batch, gemm_num_sms());
     if (!choice.use) {
         const int rc = launch_gemm_pair(int8, gelu, e4m3, fuse_resid, a, b, p, bs_a, bs_b, st);
         if (rc != Q8K_ERR_UNSUPPORTED) return rc;              // (the device cannot co-schedule the pairs)

@@ -67,7 +67,7 @@ int launch_gemm_pair(bool int8, bool gelu, bool out_e4m3, bool resid, const void
                      int bs_a, int bs_b, cudaStream_t st);
 
 // 128 x bn tiles, each owned by a cluster of sk CTAs that split K (see gemm_split.cu): bn a multiple of 16 up to 256
-// (with sk = 4 of 32), sk 1, 2 or 4 and at most the number of 128-byte K slabs.
+// (with sk = 4 of 32), sk 1, 2 or 4 (fp8: 1) and at most the number of 128-byte K slabs.
 int launch_gemm_split(bool int8, bool gelu, bool out_e4m3, bool resid, const void* a, const void* b, const GemmParams& p,
                       int bs_a, int bs_b, int bn, int sk, cudaStream_t st);
 inline int split_a_rows(int M) { return M >= kGemmBM ? kGemmBM : (M + 7) / 8 * 8; }   // rows of A that a tile loads

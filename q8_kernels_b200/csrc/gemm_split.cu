@@ -1,5 +1,5 @@
 // 8-bit GEMM for problems that 256 x 256 pair tiles cannot spread over the device: 128 x bn output tiles,
-// optionally with the K range split over the CTAs of a cluster.
+// for int8 optionally with the K range split over the CTAs of a cluster.
 //
 //   C[b] = act((A[b] . B[b]^T) * (sa[m] * sb[n]) + bias[n])      (operands and epilogue as in gemm_pair.cu)
 //
@@ -7,8 +7,9 @@
 // through one SM's L2 port (about 91 GB/s of TMA traffic), and the rest of the device idles.  Here the tile width
 // is chosen so that the tiles fill the device once, and where that is not enough a cluster of sk CTAs owns one
 // tile: CTA r accumulates its share of K in TMEM, then the partial tiles are exchanged through distributed shared
-// memory (every CTA receives all sk partials of its bn / sk columns), summed in rank order and finished by the CTA
-// that owns the columns.  The sum of the int32 partials is exact; the fp32 partials are added in a fixed order.
+// memory (every CTA receives all sk partials of its bn / sk columns), summed and finished by the CTA that owns the
+// columns.  The sum of the int32 partials is exact.  fp8 keeps one fp32 accumulator per element (sk = 1), so that its
+// bits do not depend on the split, i.e. on the other rows and columns of the call.
 //
 // One tile per CTA.  Roles (10 warps):
 //   warp 0     TMA producer (plain loads, no multicast; of A only the rows that exist)
@@ -18,9 +19,9 @@
 // cluster barriers, so the CTAs of a cluster need not agree.
 //
 // Bound by the latency of one short main loop: launch, set-up and drain take about 4 us, a 128-byte K slab 0.165 us.
-// Measured (CUDA graph, weights from HBM; the 128 x 128-tile kernel or the pair kernel before): FP8 M = 128, N = K = 2048
-// 10.3 -> 7.2 us, M = 77, N = 10240, K = 4096 15.7 -> 12.5 us (42 MB of weights: 0.52 of the copy rate), M = 128,
-// N = 2048, K = 8192 23.7 -> 10.1 us, M = 512, N = 2048, K = 8192 25.1 -> 15.3 us.  Tried: independent accumulators for
+// Measured (CUDA graph, weights from HBM; the 128 x 128-tile kernel or the pair kernel before): int8 M = 128, N = K = 2048
+// 9.5 -> 5.2 us (bn 32), M = 77, N = 10240, K = 4096 15.4 -> 11.6 us (42 MB of weights: 0.55 of the copy rate), M = 128,
+// N = 2048, K = 8192 23.1 -> 9.0 us (bn 64, sk 4), M = 512 26.0 -> 13.7 us (bn 128, sk 2).  Tried: independent accumulators for
 // the four MMAs of a slab (no difference), clusters of eight (the exchange costs 5 us).  Where the line to the pair
 // kernel lies: choose_split in gemm.cu.
 
@@ -42,7 +43,7 @@ struct SplitSmem {                           // behind the operand ring, whose l
 struct SplitParams {
     GemmParams g;
     uint32_t idesc;
-    int bn, sk;                              // tile columns (a multiple of 16, with sk = 4 of 32); CTAs per tile
+    int bn, sk;                              // tile columns (a multiple of 16, with sk = 4 of 32); CTAs per tile (fp8: 1)
     int stages;
     int stage_bytes;                         // 16 KB of A and bn rows of B
     int load_bytes;                          // what one stage's TMA boxes bring
@@ -112,7 +113,7 @@ gemm_8bit_split_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_
                        const __grid_constant__ SplitParams sp) {
     using L = SplitSmem;
     const GemmParams& p = sp.g;
-    const int bn = sp.bn, sk = sp.sk, stages = sp.stages;
+    const int bn = sp.bn, sk = INT8 ? sp.sk : 1, stages = sp.stages;
 
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -282,8 +283,7 @@ gemm_8bit_split_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_
 #pragma unroll
                         for (int j = 0; j < 4; ++j) {
                             if (r == 0) acc[4 * q + j] = v[j];
-                            else if (INT8) acc[4 * q + j] += v[j];
-                            else acc[4 * q + j] = __float_as_uint(__fadd_rn(__uint_as_float(acc[4 * q + j]), __uint_as_float(v[j])));
+                            else acc[4 * q + j] += v[j];
                         }
                     }
                 }

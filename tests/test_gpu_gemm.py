@@ -203,3 +203,24 @@ def test_split_tiles_and_split_k(nat, cuda_device, kind, B, M, N, K):
     lin = mmb(ad, wd, bd, sad, swd, False, torch.bfloat16)
     fused = nat.mm_gate_residual(ad, wd, bd, sad, swd, gate, resid)
     Hp.assert_bit_equal(fused, (gate * lin + resid).cpu(), "gate and residual in the epilogue")
+
+
+@pytest.mark.parametrize("N,K", [(2048, 8192), (944, 4240), (2064, 4096), (4096, 1024)])
+def test_fp8_row_has_the_same_bits_in_every_call(nat, cuda_device, N, K):
+    """One fp32 accumulator per element, whatever tiles the call's M and N choose: a row alone, among others or in a
+    batch, and a column of separate or stacked weights, have the same bits."""
+    g = Hp.gen(N + K)
+    d = cuda_device
+    a = torch.randn(1100, K, generator=g).to(E4M3).to(d)
+    w = torch.randn(N, K, generator=g).to(E4M3).to(d)
+    sa = (torch.rand(1100, generator=g) * 0.01 + 0.001).to(d)
+    sw = (torch.rand(N, generator=g) * 0.01 + 0.001).to(d)
+    full = nat.fp8_mm(a, w, sa, sw, False, torch.bfloat16)[0].cpu()
+    for m in (1, 36, 128, 256, 512, 1024):
+        Hp.assert_bit_equal(nat.fp8_mm(a[:m], w, sa[:m], sw, False, torch.bfloat16)[0], full[:m], f"{m} rows")
+    for n in (16, 464, N // 32 * 16):
+        for m in (128, 300):
+            Hp.assert_bit_equal(nat.fp8_mm(a[:m], w[:n], sa[:m], sw[:n], False, torch.bfloat16)[0], full[:m, :n].contiguous(),
+                                f"{m} rows, {n} columns")
+    batch = nat.fp8_mm(a[:96].view(3, 32, K), w, sa[:96].view(3, 32), sw, False, torch.bfloat16)
+    Hp.assert_bit_equal(batch.reshape(96, N), full[:96], "a batch")
