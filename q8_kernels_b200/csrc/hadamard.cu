@@ -182,7 +182,8 @@ __device__ __forceinline__ void butterfly_groups(float (&v)[V]) {
 // were copied into the unit's staging buffer by cp.async while the row before was being transformed; a thread reads
 // its 64 consecutive elements, does stages 0-5 in registers, and the remaining stages after one exchange through
 // shared memory (two above 2048).  The first exchange never leaves a warp and the staged elements are read by the
-// warp that copied them, so rows of up to 2048 elements need no block barrier at all and longer ones two.
+// warp that copied them, so rows of up to 2048 elements need no block barrier at all and longer ones two (three with
+// norm + modulation: the mean square is summed over the CTA).
 //
 // Bound by instruction issue and the FMA pipe (add/sub.f32x2 issue every second clock: 11 stages are 11 clocks per
 // element and scheduler), no longer by barriers and shared memory: 8 bytes per element of exchange (16 above 2048)
@@ -293,7 +294,9 @@ hadamard_stream_kernel(const Tin* __restrict__ x, Tout* __restrict__ out, float*
     constexpr int W = T < 32 ? T : 32;                         // threads of a row within one warp: they copy what they read
 
     extern __shared__ __align__(16) char stream_smem[];
-    __shared__ float red[8];
+    // two reductions of a row over the CTA's warps, an array each: a warp may be a row ahead when a slower one reads
+    __shared__ float red_ss[8], red_max[8];
+    static_assert(T <= 32 || B2 > 0, "the second exchange's barrier separates each array's reads from its next writes");
     const int tu = threadIdx.x % UNIT;
     const int unit = threadIdx.x / UNIT;
     const int t = tu % T;
@@ -403,11 +406,11 @@ hadamard_stream_kernel(const Tin* __restrict__ x, Tout* __restrict__ out, float*
 #pragma unroll
             for (int m = 1; m < W; m <<= 1) ss += __shfl_xor_sync(0xffffffffu, ss, m);
             if constexpr (T > 32) {
-                if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = ss;
+                if ((threadIdx.x & 31) == 0) red_ss[threadIdx.x >> 5] = ss;
                 __syncthreads();
-                ss = red[0];
+                ss = red_ss[0];
 #pragma unroll
-                for (int k = 1; k < T / 32; ++k) ss += red[k];
+                for (int k = 1; k < T / 32; ++k) ss += red_ss[k];
             }
             const float rr = rsqrtf(ss * (1.0f / (float)dim));
 #pragma unroll
@@ -515,11 +518,11 @@ hadamard_stream_kernel(const Tin* __restrict__ x, Tout* __restrict__ out, float*
 #pragma unroll
             for (int m = 1; m < (T < 32 ? T : 32); m <<= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, m));
             if constexpr (T > 32) {
-                if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = amax;
+                if ((threadIdx.x & 31) == 0) red_max[threadIdx.x >> 5] = amax;
                 __syncthreads();
-                amax = red[0];
+                amax = red_max[0];
 #pragma unroll
-                for (int k = 1; k < T / 32; ++k) amax = fmaxf(amax, red[k]);
+                for (int k = 1; k < T / 32; ++k) amax = fmaxf(amax, red_max[k]);
             }
             const float qmax = std::is_same_v<Tout, int8_t> ? 127.0f : 448.0f;
             const float qscale = __fdiv_rn(qmax, amax);

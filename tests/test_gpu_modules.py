@@ -209,6 +209,27 @@ def test_norm_modulate_quant_groups_and_turns(q8, cuda_device, B, S, C):
     assert torch.allclose(s, sd, rtol=1e-2)
 
 
+@pytest.mark.parametrize("C", [2064, 4096, 6000, 8192])
+@pytest.mark.parametrize("q_dtype", [torch.int8, E4M3])
+def test_norm_modulate_quant_turns_of_long_rows_do_not_meet(q8, cuda_device, C, q_dtype):
+    """Above 2048 channels a row belongs to a CTA of several warps: dozens of rows per CTA in one call give the bytes of
+    calls that are small enough for one row per CTA."""
+    d = cuda_device
+    rows, few = 20000, 250
+    g = torch.Generator(device=d).manual_seed(C)
+    x = torch.randn(1, rows, C, generator=g, device=d) * torch.rand(1, rows, 1, generator=g, device=d).exp2().pow(8)
+    x[..., : C // 2] *= 4                                        # the warps of a row see different maxima
+    x = x.to(torch.bfloat16)
+    sc = torch.randn(1, 1, C, generator=g, device=d).to(torch.bfloat16)
+    sh = (torch.randn(1, 1, C, generator=g, device=d) * 10).to(torch.bfloat16)
+    parts = [q8.native.norm_modulate_quant(x[:, i:i + few], sc, sh, q_dtype) for i in range(0, rows, few)]
+    q_ref, s_ref = (torch.cat([p[k] for p in parts], dim=1) for k in (0, 1))
+    for _ in range(3):
+        q, s = q8.native.norm_modulate_quant(x, sc, sh, q_dtype)
+        assert torch.equal(q.view(torch.uint8), q_ref.view(torch.uint8)), "bytes"
+        assert torch.equal(s, s_ref), "scales"
+
+
 @pytest.mark.parametrize("kind", ["int8", "fp8"])
 @pytest.mark.parametrize("with_gate", [True, False])
 @pytest.mark.parametrize("M,N,K", [(200, 512, 256), (384, 2048, 2048), (96, 128, 128), (300, 272, 192), (515, 1040, 320)])
