@@ -39,6 +39,12 @@ int gemm_num_sms() {
 // K = 4096 15.4 -> 11.6 (bn 80);  M = 128, N = 2048, K = 8192 23.1 -> 9.0 (bn 64, sk 4);  M = 1024, N = 2048, K = 8192
 // 26.2 -> 18.0 (bn 128).  At N = K = 2048 the line to the pair kernel lies between M = 1024 (12.2 -> 8.4) and M = 2048
 // (12.6 against 14.9).
+// Half of a pair tile is padding where M or N is at most 128, so there the split kernel is the rule; but one tile per CTA
+// pays its set-up for every tile, and from three rounds of pair tiles on the persistent pair kernel is faster all the same
+// (int8, pair against split): N = 128, K = 1024 M = 24576 11.5 against 11.4, M = 49152 15.7 against 20.9, M = 196608 45.3
+// against 60.9;  N = 64, K = 512, M = 98304 17.4 against 18.9;  N = 16 28.2 against 23.8 (K = 1024, M = 98304: split).
+// With weights of their own per batch entry: 32 x (M = 100, N = 4096, K = 1024) 33.5 against 37.5, 32 x (M = 128, N = 2048,
+// K = 128) 14.4 against 10.8 (split).  M <= 128 rows on shared weights: split (N = 65536, K = 1024, M = 77 22.0 against 18.5).
 // Only int8 splits K: its partial sums are exact.  fp32 partials would round in another order than one accumulator,
 // and an fp8 row would then have other bits in a call with other M or N (it has the same in every call, and stacked
 // weights give the bits of the separate ones).
@@ -63,11 +69,10 @@ static SplitChoice choose_split(bool int8, int M, int N, int K, int batch, int s
         }
     }
     best += 0.06e-6 * N * K;
-    if (M > kGemmBM && N > 128) {
-        const double tiles = (double)((M + 255) / 256) * ((N + 255) / 256) * batch;
-        const double waves = (double)(int64_t)((tiles + sms / 2 - 1) / (sms / 2));
-        c.use = best < 0.95 * (6.5 + 0.31 * iters * waves);
-    }
+    const double tiles = (double)((M + 255) / 256) * ((N + 255) / 256) * batch;
+    const double waves = (double)(int64_t)((tiles + sms / 2 - 1) / (sms / 2));
+    if (M > kGemmBM && N > 128) c.use = best < 0.95 * (6.5 + 0.31 * iters * waves);
+    else c.use = waves < 3 || !((N >= 64 && N <= 128) || (batch > 1 && M >= 64 && iters >= 8));
     return c;
 }
 
@@ -85,10 +90,14 @@ static int gemm_8bit(bool int8, const void* a, const void* b, const float* bias,
                 "%s: a, b and out must be 16-byte aligned", op);
     Q8K_REQUIRE(out_dtype == Q8K_DT_BF16 || out_dtype == Q8K_DT_E4M3, Q8K_ERR_UNSUPPORTED,
                 "%s: output dtype %d is not bf16 or e4m3", op, out_dtype);
-    const int batch = bs_a > bs_b ? bs_a : bs_b;
     Q8K_REQUIRE((int64_t)bs_a * M <= 0x7fffffffLL && (int64_t)bs_b * N <= 0x7fffffffLL, Q8K_ERR_TOO_LARGE,
                 "%s: batch * rows exceeds 2^31", op);
     if (M == 0) return Q8K_OK;
+    if (bs_b == 1) {                                           // shared weights: the batch is more rows of one product
+        M *= bs_a;
+        bs_a = 1;
+    }
+    const int batch = bs_a > bs_b ? bs_a : bs_b;
 
     GemmParams p;
     p.a_scales = a_scales;

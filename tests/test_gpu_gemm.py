@@ -224,3 +224,37 @@ def test_fp8_row_has_the_same_bits_in_every_call(nat, cuda_device, N, K):
                                 f"{m} rows, {n} columns")
     batch = nat.fp8_mm(a[:96].view(3, 32, K), w, sa[:96].view(3, 32), sw, False, torch.bfloat16)
     Hp.assert_bit_equal(batch.reshape(96, N), full[:96], "a batch")
+
+
+@pytest.mark.parametrize("kind", ["int8", "fp8"])
+@pytest.mark.parametrize("B,Bw,M,N,K", [(1, 1, 37900, 64, 144), (1, 1, 38000, 128, 272), (40, 40, 100, 1040, 1040),
+                                        (160, 160, 128, 128, 1024), (7, 1, 77, 272, 400), (300, 1, 3, 144, 64), (1, 3, 33, 96, 208)])
+def test_padded_pair_tiles_and_folded_batches(nat, cuda_device, kind, B, Bw, M, N, K):
+    """Pair tiles half of which is padding (three rounds of them, N or M at most 128), a batch on shared weights as rows
+    of one product (tiles that straddle batch entries and their gate rows), one activation on a batch of weights.
+    Bounds as in test_split_tiles_and_split_k, without GELU."""
+    qd = torch.int8 if kind == "int8" else E4M3
+    d = cuda_device
+    g = torch.Generator(device=d).manual_seed(M + N + K)
+
+    def mk(*s):
+        x = torch.randint(-127, 128, s, generator=g, device=d) if kind == "int8" else torch.randn(s, generator=g, device=d)
+        return x.to(qd)
+
+    a, w = mk(B, M, K), mk(*((Bw, N, K) if Bw > 1 else (N, K)))
+    sa = torch.rand(B, M, generator=g, device=d) * 0.01 + 0.001
+    sw = torch.rand(*((Bw, N) if Bw > 1 else (N,)), generator=g, device=d) * 0.01 + 0.001
+    bias = torch.randn(N, generator=g, device=d) * 0.1
+    mmb = nat.q8_mm_bias if kind == "int8" else nat.fp8_mm_bias
+    out = mmb(a, w, bias, sa, sw, False, torch.bfloat16)
+    assert out.shape == (max(B, Bw), M, N)
+    for i in range(0, max(B, Bw), max(1, max(B, Bw) // 8)):
+        ai, si = a[min(i, B - 1)], sa[min(i, B - 1)]
+        wi, swi = (w[i], sw[i]) if Bw > 1 else (w, sw)
+        y = (ai.double() @ wi.double().T) * si.double().unsqueeze(-1) * swi.double() + bias.double()
+        assert bool(((out[i].double() - y).abs() <= 2.0 ** -8 * y.abs() + 2e-6 * y.abs().max()).all())
+    if Bw == 1:
+        gate = torch.randn(B, 1, N, generator=g, device=d).to(torch.bfloat16)
+        resid = torch.randn(B, M, N, generator=g, device=d).to(torch.bfloat16)
+        fused = nat.mm_gate_residual(a, w, bias, sa, sw, gate, resid)
+        Hp.assert_bit_equal(fused, gate * out + resid, "gate and residual in the epilogue")
