@@ -317,3 +317,21 @@ def test_dequant_hadamard_equals_the_op_chain(nat, cuda_device, N, K):
     sc = (torch.rand(N, generator=g) * 0.1 + 1e-3).to(cuda_device)
     ref = nat.fast_hadamard_transform((x * sc[:, None]).to(torch.bfloat16), 1 / math.sqrt(K), None)
     Hp.assert_bit_equal(nat.dequant_hadamard(x, sc, 1 / math.sqrt(K)), ref.cpu(), "rotated weight")
+
+
+@pytest.mark.parametrize("N,K,fused", [(4096, 16, True), (4112, 128, False), (8192, 64, False), (8192, 144, True), (16384, 112, False),
+                                       (48, 272, True)])
+def test_weight_operand_routes(nat, cuda_device, monkeypatch, N, K, fused):
+    """Long weights with few columns take the op chain, the others the transposing kernel: the same bytes on both."""
+    from q8_kernels_b200.functional import linear as L
+    g = Hp.gen(N + K)
+    b = torch.randint(-127, 128, (N, K), generator=g, dtype=torch.int8).to(cuda_device)
+    s = (torch.rand(N, generator=g) * 0.1 + 1e-3).to(cuda_device)
+    calls = []
+    kernel = nat.transpose_quant
+    monkeypatch.setattr(nat, "transpose_quant", lambda *a: (calls.append(1), kernel(*a))[1])
+    q, sc = L._weight_operand(b, s, torch.bfloat16)
+    assert bool(calls) == fused
+    q_ref, s_ref = nat.tokenwise_quant((b.to(torch.bfloat16) * s[:, None]).T.contiguous(), E4M3)
+    Hp.assert_bit_equal(q, q_ref.cpu(), "bytes")
+    Hp.assert_bit_equal(sc, s_ref.cpu(), "scales")
