@@ -455,15 +455,25 @@ hadamard_stream_kernel(const Tin* __restrict__ x, Tout* __restrict__ out, float*
             v[i] = m.x; v[i + 1] = m.y;
         }
         Tout* outr = out + (int64_t)row * dim;
+        // Group j of this thread starts at element e0 + (j << LOW), inside the row if (j << LOW) < lim.  The asm keeps the
+        // compiler from holding up to 32 such comparisons in registers across the rows (168 of them, or spills).
+        const int e0 = LF::elem(t, 0);
+        int lim = dim - e0;
+        if constexpr (!FULL) asm volatile("" : "+r"(lim));
+        auto in_row = [&](int j) { return FULL || (j << LF::LOW) < lim; };
+        // Of 32 groups, eight at a time whose elements all lie beyond dim are neither rounded, reduced nor quantised.
+        // Measured, 6144 x 1536 (neither of the two before -> now): int8 rows 16.7 -> 14.0 us, e4m3 rows 12.9 -> 12.6 us;
+        // 6144 x 1544, where nothing can be skipped: 16.9 -> 15.3 us.
+        constexpr int SKIP = !FULL && LF::G == 32 ? 8 : LF::G;
+        auto any_in_row = [&](int j) { return SKIP == LF::G || (j << LF::LOW) < dim; };
         if constexpr (EPI == Epilogue::Cast) {
             if constexpr (std::is_same_v<Tout, __nv_bfloat16>) {
 #pragma unroll
                 for (int j = 0; j < LF::G; ++j) {
-                    const int e = LF::elem(t, j);
                     float o[C];
 #pragma unroll
                     for (int i = 0; i < C; ++i) o[i] = v[j * C + i];
-                    if (row_ok && (FULL || e < dim)) store_elems<Tout, C>(outr + e, o);
+                    if (row_ok && in_row(j)) store_elems<Tout, C>(outr + e0 + (j << LF::LOW), o);
                 }
             } else {
                 static_assert(std::is_same_v<Tout, e4m3_t>, "cast to bf16 or e4m3");
@@ -476,9 +486,9 @@ hadamard_stream_kernel(const Tin* __restrict__ x, Tout* __restrict__ out, float*
                     u.w = pack8_e4m3_c10(o);
 #pragma unroll
                     for (int g = 0; g < 8 / C; ++g) {
-                        const int e = LF::elem(t, f / C + g);
-                        if (row_ok && (FULL || e < dim))
-                            *reinterpret_cast<typename ByteVec<C>::type*>(reinterpret_cast<uint8_t*>(outr) + e) = u.b[g];
+                        const int j = f / C + g;
+                        if (row_ok && in_row(j))
+                            *reinterpret_cast<typename ByteVec<C>::type*>(reinterpret_cast<uint8_t*>(outr) + e0 + (j << LF::LOW)) = u.b[g];
                     }
                 }
             }
@@ -490,28 +500,38 @@ hadamard_stream_kernel(const Tin* __restrict__ x, Tout* __restrict__ out, float*
             if constexpr (IN8) {
                 __half2 m2 = __floats2half2_rn(0.f, 0.f);
 #pragma unroll
-                for (int f = 0; f < V; f += 8) {
-                    float o[8];
+                for (int jc = 0; jc < LF::G; jc += SKIP) {
+                    if (any_in_row(jc)) {
 #pragma unroll
-                    for (int i = 0; i < 8; ++i) o[i] = v[f + i];
-                    const uint2 w = pack8_e4m3_c10(o);
-                    pk[f / 4] = w.x;
-                    pk[f / 4 + 1] = w.y;
+                        for (int f = jc * C; f < (jc + SKIP) * C; f += 8) {
+                            float o[8];
 #pragma unroll
-                    for (int g = 0; g < 4; ++g) {
-                        const uint32_t ww = g < 2 ? w.x : w.y;
-                        const __half2_raw h = __nv_cvt_fp8x2_to_halfraw2((__nv_fp8x2_storage_t)(g & 1 ? ww >> 16 : ww & 0xffffu), __NV_E4M3);
-                        if (FULL || LF::elem(t, (f + 2 * g) / C) < dim) m2 = __hmax2(m2, __habs2(__half2(h)));
+                            for (int i = 0; i < 8; ++i) o[i] = v[f + i];
+                            const uint2 w = pack8_e4m3_c10(o);
+                            pk[f / 4] = w.x;
+                            pk[f / 4 + 1] = w.y;
+#pragma unroll
+                            for (int g = 0; g < 4; ++g) {
+                                const uint32_t ww = g < 2 ? w.x : w.y;
+                                const __half2_raw h = __nv_cvt_fp8x2_to_halfraw2((__nv_fp8x2_storage_t)(g & 1 ? ww >> 16 : ww & 0xffffu), __NV_E4M3);
+                                if (in_row((f + 2 * g) / C)) m2 = __hmax2(m2, __habs2(__half2(h)));
+                            }
+                        }
                     }
                 }
                 amax = fmaxf(__low2float(m2), __high2float(m2));
             } else {
                 __nv_bfloat162 m2 = __floats2bfloat162_rn(0.f, 0.f);
 #pragma unroll
-                for (int f = 0; f < V; f += 2) {
-                    const __nv_bfloat162 w = __floats2bfloat162_rn(v[f], v[f + 1]);
-                    pk[f / 2] = *reinterpret_cast<const uint32_t*>(&w);
-                    if (FULL || LF::elem(t, f / C) < dim) m2 = __hmax2(m2, __habs2(w));
+                for (int jc = 0; jc < LF::G; jc += SKIP) {
+                    if (any_in_row(jc)) {
+#pragma unroll
+                        for (int f = jc * C; f < (jc + SKIP) * C; f += 2) {
+                            const __nv_bfloat162 w = __floats2bfloat162_rn(v[f], v[f + 1]);
+                            pk[f / 2] = *reinterpret_cast<const uint32_t*>(&w);
+                            if (in_row(f / C)) m2 = __hmax2(m2, __habs2(w));
+                        }
+                    }
                 }
                 amax = fmaxf(__low2float(m2), __high2float(m2));
             }
@@ -531,46 +551,50 @@ hadamard_stream_kernel(const Tin* __restrict__ x, Tout* __restrict__ out, float*
             const float2 q2 = make_float2(qmul, qmul);
             constexpr int P = C < 4 ? C : 4;                   // values per packing step
 #pragma unroll
-            for (int j = 0; j < LF::G; ++j) {
-                const int e = LF::elem(t, j);
-                union { typename ByteVec<C>::type b; uint32_t w[C >= 4 ? C / 4 : 1]; } u;
+            for (int jc = 0; jc < LF::G; jc += SKIP) {
+                if (any_in_row(jc)) {
 #pragma unroll
-                for (int i = 0; i < C; i += P) {
-                    float y[4];
+                    for (int j = jc; j < jc + SKIP; ++j) {
+                        union { typename ByteVec<C>::type b; uint32_t w[C >= 4 ? C / 4 : 1]; } u;
 #pragma unroll
-                    for (int h = 0; h < P; h += 2) {
-                        const int f = j * C + i + h;
-                        float2 a;
-                        if constexpr (IN8) {
-                            const uint32_t ww = pk[f / 4];
-                            const __half2_raw hr = __nv_cvt_fp8x2_to_halfraw2((__nv_fp8x2_storage_t)(f & 2 ? ww >> 16 : ww & 0xffffu), __NV_E4M3);
-                            a = __half22float2(__half2(hr));
-                        } else {
-                            a = make_float2(__uint_as_float(pk[f / 2] << 16), __uint_as_float(pk[f / 2] & 0xffff0000u));
+                        for (int i = 0; i < C; i += P) {
+                            float y[4];
+#pragma unroll
+                            for (int h = 0; h < P; h += 2) {
+                                const int f = j * C + i + h;
+                                float2 a;
+                                if constexpr (IN8) {
+                                    const uint32_t ww = pk[f / 4];
+                                    const __half2_raw hr = __nv_cvt_fp8x2_to_halfraw2((__nv_fp8x2_storage_t)(f & 2 ? ww >> 16 : ww & 0xffffu), __NV_E4M3);
+                                    a = __half22float2(__half2(hr));
+                                } else {
+                                    a = make_float2(__uint_as_float(pk[f / 2] << 16), __uint_as_float(pk[f / 2] & 0xffff0000u));
+                                }
+                                a = fmul2(a, q2);
+                                // round half away from zero (C round()) of |y| < 2^22: adding the largest float below 0.5 with
+                                // y's sign and truncating gives floor(|y| + 0.5) for every fp32 y, ties included
+                                if constexpr (std::is_same_v<Tout, int8_t>)
+                                    a = fadd2(a, make_float2(copysignf(0.49999997f, a.x), copysignf(0.49999997f, a.y)));
+                                y[h] = a.x;
+                                y[h + 1] = a.y;
+                            }
+                            uint32_t w;
+                            if constexpr (std::is_same_v<Tout, int8_t>) {
+                                w = __byte_perm((uint32_t)__float2int_rz(y[0]), (uint32_t)__float2int_rz(y[1]), 0x0040);
+                                if constexpr (P == 4)
+                                    w = __byte_perm(w, __byte_perm((uint32_t)__float2int_rz(y[2]), (uint32_t)__float2int_rz(y[3]), 0x0040), 0x5410);
+                            } else {
+                                // |y| <= 448 (1 + 2^-23) for finite rows, where the saturating cast and the c10 cast (overflow ->
+                                // NaN beyond 464) agree; a NaN stays a NaN in both
+                                w = (uint32_t)float2_to_e4m3x2_sat(y[0], y[1]);
+                                if constexpr (P == 4) w |= (uint32_t)float2_to_e4m3x2_sat(y[2], y[3]) << 16;
+                            }
+                            u.w[i / 4] = w;
                         }
-                        a = fmul2(a, q2);
-                        // round half away from zero (C round()) of |y| < 2^22: adding the largest float below 0.5 with
-                        // y's sign and truncating gives floor(|y| + 0.5) for every fp32 y, ties included
-                        if constexpr (std::is_same_v<Tout, int8_t>)
-                            a = fadd2(a, make_float2(copysignf(0.49999997f, a.x), copysignf(0.49999997f, a.y)));
-                        y[h] = a.x;
-                        y[h + 1] = a.y;
+                        if (row_ok && in_row(j))
+                            *reinterpret_cast<typename ByteVec<C>::type*>(reinterpret_cast<uint8_t*>(outr) + e0 + (j << LF::LOW)) = u.b;
                     }
-                    uint32_t w;
-                    if constexpr (std::is_same_v<Tout, int8_t>) {
-                        w = __byte_perm((uint32_t)__float2int_rz(y[0]), (uint32_t)__float2int_rz(y[1]), 0x0040);
-                        if constexpr (P == 4)
-                            w = __byte_perm(w, __byte_perm((uint32_t)__float2int_rz(y[2]), (uint32_t)__float2int_rz(y[3]), 0x0040), 0x5410);
-                    } else {
-                        // |y| <= 448 (1 + 2^-23) for finite rows, where the saturating cast and the c10 cast (overflow ->
-                        // NaN beyond 464) agree; a NaN stays a NaN in both
-                        w = (uint32_t)float2_to_e4m3x2_sat(y[0], y[1]);
-                        if constexpr (P == 4) w |= (uint32_t)float2_to_e4m3x2_sat(y[2], y[3]) << 16;
-                    }
-                    u.w[i / 4] = w;
                 }
-                if (row_ok && (FULL || e < dim))
-                    *reinterpret_cast<typename ByteVec<C>::type*>(reinterpret_cast<uint8_t*>(outr) + e) = u.b;
             }
         }
         // the other warps have read the exchange before it is overwritten (with a quantizer: the absmax barrier)

@@ -189,7 +189,7 @@ def test_norm_modulate_quant_matches_unfused_chain(q8, cuda_device):
     assert ((q.int() - qd.int()).abs() != 0).float().mean().item() < 0.01
 
 
-@pytest.mark.parametrize("B,S,C", [(3, 5, 512), (1, 4801, 1024), (2, 901, 2048), (2, 901, 1552), (5, 33, 4096), (3, 201, 8192),
+@pytest.mark.parametrize("B,S,C", [(3, 5, 512), (1, 4801, 1024), (2, 901, 2048), (2, 901, 1552), (2, 901, 1536), (5, 33, 4096), (3, 201, 8192),
                                    (700, 1, 2048)])
 def test_norm_modulate_quant_groups_and_turns(q8, cuda_device, B, S, C):
     """Every batch entry keeps to its own modulation rows, over group tails, several turns of a CTA, ragged dims and

@@ -134,6 +134,23 @@ def test_long_rows_stream_through_a_full_grid(nat, cuda_device, rows, dim):
     Hp.assert_bit_equal(sc, s_ref, "e4m3 in, scales")
 
 
+@pytest.mark.parametrize("dim", [1032, 1280, 1536, 1544, 1800, 2040])
+def test_rows_that_end_inside_a_group_of_eight_runs(nat, cuda_device, dim):
+    """Between 1024 and 2048 elements whole groups beyond the row are skipped: rows that end on, just behind and between
+    the 512-element groups, quantised and cast, from bf16 and e4m3."""
+    s = 1.0 / math.sqrt(dim)
+    x = Hp.activations(37, dim, seed=dim, outliers=True)
+    x8 = O.c10_e4m3(x.float() * 0.05)
+    for src in (x, x8):
+        h_ref = O.hadamard_transform(src, scale=s)
+        Hp.assert_bit_equal(nat.fast_hadamard_transform(src.to(cuda_device), s, None), h_ref, "cast")
+        for qt in (torch.int8, E4M3):
+            q_ref, s_ref = O.tokenwise_quant(h_ref, qt)
+            q, sc = nat.hadamard_quant(src.to(cuda_device), s, qt)
+            Hp.assert_bit_equal(q, q_ref, f"rows {src.dtype} {qt}")
+            Hp.assert_bit_equal(sc, s_ref, f"scales {src.dtype} {qt}")
+
+
 def test_fused_hadamard_quant_e4m3_input(nat, cuda_device):
     # the e4m3 attention output feeding to_out: intermediate is rounded to e4m3 (c10 cast)
     x8 = O.c10_e4m3(torch.randn(20, 2048, generator=Hp.gen(8)) * 0.5)
