@@ -264,7 +264,8 @@ struct StreamGeo {
     static constexpr int XROW = (N / 4 + N / 64 + (PAD8 ? N / 32 : 0)) * 16;
     static constexpr int XCH = RPU * XROW;
     static constexpr int MOD = NORM_MOD ? 2 * N * 2 : 0;       // bytes per CTA: 1 + scale and shift rows (bf16)
-    static constexpr int SMEM = UNITS * (RAW + XCH) + MOD;
+    static constexpr int smem(int units) { return units * (RAW + XCH) + MOD; }
+    static constexpr int SMEM = smem(UNITS);
     static constexpr int BY_SMEM = (228 * 1024) / (SMEM + 1024);
     static constexpr int BY_REGS = 65536 / (THREADS * 128);
     static constexpr int CTAS = BY_SMEM < BY_REGS ? BY_SMEM : BY_REGS;
@@ -302,14 +303,15 @@ hadamard_stream_kernel(const Tin* __restrict__ x, Tout* __restrict__ out, float*
     const int t = tu % T;
     const int r_in = tu / T;
     char* raw = stream_smem + unit * Geo::RAW + r_in * (N * (int)sizeof(Tin));
-    char* xch = stream_smem + Geo::UNITS * Geo::RAW + unit * Geo::XCH + r_in * Geo::XROW;
+    const int units = NORM_MOD && Geo::UNITS > 1 ? (int)blockDim.x / UNIT : Geo::UNITS;
+    char* xch = stream_smem + units * Geo::RAW + unit * Geo::XCH + r_in * Geo::XROW;
     const uint32_t raw_addr = (uint32_t)__cvta_generic_to_shared(raw);
     const unsigned mod = NORM_MOD ? blockIdx.x / blocks_per_mod : 0u;
     const unsigned blk = NORM_MOD ? blockIdx.x - mod * blocks_per_mod : blockIdx.x;
     const unsigned first = mod * rows_per_mod;
     const unsigned count = NORM_MOD ? (rows - first < rows_per_mod ? rows - first : rows_per_mod) : rows;   // rows of this group
-    const unsigned step = (NORM_MOD ? blocks_per_mod : gridDim.x) * (unsigned)(Geo::UNITS * RPU);
-    unsigned rel = (blk * (unsigned)Geo::UNITS + (unsigned)unit) * (unsigned)RPU;   // first row of this unit, relative to the group
+    const unsigned step = (NORM_MOD ? blocks_per_mod : gridDim.x) * (unsigned)(units * RPU);
+    unsigned rel = (blk * (unsigned)units + (unsigned)unit) * (unsigned)RPU;   // first row of this unit, relative to the group
 
     auto load_rows = [&](unsigned rel0) {
         const bool ok = rel0 + r_in < count;
@@ -328,27 +330,31 @@ hadamard_stream_kernel(const Tin* __restrict__ x, Tout* __restrict__ out, float*
     pdl_release();
     load_rows(rel);
 
-    __nv_bfloat16* mod_smem = reinterpret_cast<__nv_bfloat16*>(stream_smem + Geo::UNITS * (Geo::RAW + Geo::XCH));
+    __nv_bfloat16* mod_smem = reinterpret_cast<__nv_bfloat16*>(stream_smem + units * (Geo::RAW + Geo::XCH));
     if constexpr (NORM_MOD) {
         // 1 + scale and shift rows of this CTA's batch entry, staged like the raw rows (bf16: CPT = V / 8)
         const __nv_bfloat16* sc = mod_scale + (int64_t)mod * dim;
         const __nv_bfloat16* sh = mod_shift + (int64_t)mod * dim;
         const __nv_bfloat162 one2 = __floats2bfloat162_rn(1.0f, 1.0f);
-        for (int c = threadIdx.x; c < N / 8; c += Geo::THREADS) {
-            uint4 s8 = make_uint4(0, 0, 0, 0), h8 = make_uint4(0, 0, 0, 0);
-            if (FULL || c * 8 < dim) {
-                s8 = *reinterpret_cast<const uint4*>(sc + c * 8);
-                h8 = *reinterpret_cast<const uint4*>(sh + c * 8);
-            }
-            uint32_t* w = &s8.x;
+        auto load_mod = [&](int stride) {
+            for (int c = threadIdx.x; c < N / 8; c += stride) {
+                uint4 s8 = make_uint4(0, 0, 0, 0), h8 = make_uint4(0, 0, 0, 0);
+                if (FULL || c * 8 < dim) {
+                    s8 = *reinterpret_cast<const uint4*>(sc + c * 8);
+                    h8 = *reinterpret_cast<const uint4*>(sh + c * 8);
+                }
+                uint32_t* w = &s8.x;
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                const __nv_bfloat162 m1 = __hadd2_rn(one2, *reinterpret_cast<const __nv_bfloat162*>(w + j));
-                w[j] = *reinterpret_cast<const uint32_t*>(&m1);
+                for (int j = 0; j < 4; ++j) {
+                    const __nv_bfloat162 m1 = __hadd2_rn(one2, *reinterpret_cast<const __nv_bfloat162*>(w + j));
+                    w[j] = *reinterpret_cast<const uint32_t*>(&m1);
+                }
+                reinterpret_cast<uint4*>(mod_smem)[raw_pos<CPT>(c)] = s8;
+                reinterpret_cast<uint4*>(mod_smem + N)[raw_pos<CPT>(c)] = h8;
             }
-            reinterpret_cast<uint4*>(mod_smem)[raw_pos<CPT>(c)] = s8;
-            reinterpret_cast<uint4*>(mod_smem + N)[raw_pos<CPT>(c)] = h8;
-        }
+        };
+        if (units == Geo::UNITS) load_mod(Geo::THREADS);       // a constant stride: all loads at once
+        else load_mod(units * UNIT);
         __syncthreads();
     }
 
@@ -624,7 +630,12 @@ static int launch_stream(const Tin* x, Tout* out, float* scales, int64_t rows, i
     const int64_t need = (group_rows + per_cta - 1) / per_cta;
     int64_t blocks = slots / groups < 1 ? 1 : slots / groups;
     if (blocks > need) blocks = need;
-    Q8K_CUDA_OK(launch_dependent(kern, (unsigned)(blocks * groups), Geo::THREADS, Geo::SMEM, st, 1, x, out, scales, (unsigned)rows,
+    // A CTA stays inside one batch entry: where one turn takes all rows of an entry and there are more entries than CTAs fit
+    // the device, it gets only as many units, so that more fit.  4096 x 1 x 2048 30.1 -> 15.0 us, 512 x 2 x 2048 6.8 ->
+    // 5.9 us (before the streamed kernel: 16.3 and 6.1).  With fewer entries the other units help to load the modulation
+    // rows (1 x 1 x 2048: 3.2 us, 3.4 with one unit).
+    const int units = NORM_MOD && need == 1 && groups > slots ? (int)((group_rows + Geo::RPU - 1) / Geo::RPU) : Geo::UNITS;
+    Q8K_CUDA_OK(launch_dependent(kern, (unsigned)(blocks * groups), units * Geo::UNIT, Geo::smem(units), st, 1, x, out, scales, (unsigned)rows,
                                  dim, stride, scale, ms, mh, (unsigned)group_rows, (unsigned)blocks));
     return Q8K_OK;
 }

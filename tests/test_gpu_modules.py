@@ -190,7 +190,7 @@ def test_norm_modulate_quant_matches_unfused_chain(q8, cuda_device):
 
 
 @pytest.mark.parametrize("B,S,C", [(3, 5, 512), (1, 4801, 1024), (2, 901, 2048), (2, 901, 1552), (2, 901, 1536), (5, 33, 4096), (3, 201, 8192),
-                                   (700, 1, 2048)])
+                                   (700, 1, 2048), (4096, 1, 512), (600, 2, 1536), (1000, 9, 512), (300, 5, 1024)])
 def test_norm_modulate_quant_groups_and_turns(q8, cuda_device, B, S, C):
     """Every batch entry keeps to its own modulation rows, over group tails, several turns of a CTA, ragged dims and
     more entries than the grid has CTAs: against the op chain on the device (the mean square is summed in another
