@@ -56,6 +56,10 @@ Q8K_API int         q8k_version(void);
  * `tries` (1..65536) tests and records  Q8K_STATUS_TIMEOUT | (9 << 8)  in *dev_status.  The kernel
  * returns normally and the context stays usable.  No counterpart in the reference.              */
 Q8K_API int         q8k_wait_selftest(int* dev_status, unsigned tries, void* stream);
+/* Which tiles a GEMM call of this shape runs on the current device (148 SMs assumed without one), for tests and tuning:
+ * plan = {1 if 256 x 256 pair tiles else 0, tile columns, CTAs that share a tile's K range}.  Launches nothing; no
+ * counterpart in the reference.                                                                    */
+Q8K_API int         q8k_mm_plan(int int8, int bs_a, int bs_b, int M, int N, int K, int plan[3]);
 Q8K_API const char* q8k_error_string(int code);
 Q8K_API const char* q8k_last_error_detail(void);
 

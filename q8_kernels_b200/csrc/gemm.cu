@@ -76,6 +76,15 @@ static SplitChoice choose_split(bool int8, int M, int N, int K, int batch, int s
     return c;
 }
 
+// On shared weights a batch is more rows of one product.  Returns the batch that is left.
+static int fold_batch(int& bs_a, int bs_b, int& M) {
+    if (bs_b == 1) {
+        M *= bs_a;
+        bs_a = 1;
+    }
+    return bs_a > bs_b ? bs_a : bs_b;
+}
+
 static int gemm_8bit(bool int8, const void* a, const void* b, const float* bias, const float* a_scales,
                      const float* b_scales, void* out, int out_dtype, int bs_a, int bs_b, int M, int N, int K,
                      int fuse_gelu, int* dev_status, void* stream, const void* resid = nullptr,
@@ -93,11 +102,7 @@ static int gemm_8bit(bool int8, const void* a, const void* b, const float* bias,
     Q8K_REQUIRE((int64_t)bs_a * M <= 0x7fffffffLL && (int64_t)bs_b * N <= 0x7fffffffLL, Q8K_ERR_TOO_LARGE,
                 "%s: batch * rows exceeds 2^31", op);
     if (M == 0) return Q8K_OK;
-    if (bs_b == 1) {                                           // shared weights: the batch is more rows of one product
-        M *= bs_a;
-        bs_a = 1;
-    }
-    const int batch = bs_a > bs_b ? bs_a : bs_b;
+    const int batch = fold_batch(bs_a, bs_b, M);
 
     GemmParams p;
     p.a_scales = a_scales;
@@ -128,6 +133,18 @@ static int gemm_8bit(bool int8, const void* a, const void* b, const float* bias,
 }
 
 }  // namespace q8k
+
+extern "C" int q8k_mm_plan(int int8, int bs_a, int bs_b, int M, int N, int K, int plan[3]) {
+    using q8k::set_error_detail;
+    Q8K_REQUIRE(plan != nullptr && bs_a >= 1 && bs_b >= 1 && M > 0 && N > 0 && K > 0 && (int64_t)bs_a * M <= 0x7fffffffLL,
+                Q8K_ERR_INVALID_ARG, "mm_plan: null plan or bad shape");
+    const int batch = q8k::fold_batch(bs_a, bs_b, M);
+    const q8k::SplitChoice c = q8k::choose_split(int8 != 0, M, N, K, batch, q8k::gemm_num_sms());
+    plan[0] = c.use ? 0 : 1;
+    plan[1] = c.use ? c.bn : 256;
+    plan[2] = c.use ? c.sk : 1;
+    return Q8K_OK;
+}
 
 extern "C" int q8k_q8_mm(const void* a, const void* b, const float* bias, const float* a_scales,
                          const float* b_scales, void* out, int out_dtype, int bs_a, int bs_b, int M, int N,

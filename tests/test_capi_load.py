@@ -129,3 +129,26 @@ def test_row_arguments_describe_the_same_rows_for_every_layout(i):
     assert (rows, dim) == tuple(want.shape) and t.is_contiguous() and torch.equal(t.reshape(rows, dim), want)
     c, s, n = native._tables(x, x.clone(), dim)
     assert n == rows and c.is_contiguous() and s.is_contiguous() and torch.equal(c.reshape(rows, dim), want)
+
+
+def test_gemm_plan_keeps_to_what_the_split_kernel_can_run():
+    """Over sizes from one row up: tile widths are multiples of 16 (of 32 for four shares of K) up to 256, every CTA of a
+    K split has at least two slabs, FP8 never splits K, and batches on shared weights are planned as rows."""
+    import ctypes
+    from q8_kernels_b200 import _lib
+    plan, folded = (ctypes.c_int * 3)(), (ctypes.c_int * 3)()
+
+    def ask(p, *a):
+        assert _lib.lib.q8k_mm_plan(*a, ctypes.cast(p, ctypes.c_void_p)) == 0
+        return tuple(p)
+
+    for int8 in (0, 1):
+        for batch in (1, 3, 64):
+            for m in (1, 16, 77, 128, 129, 512, 2002, 24576):
+                for n in (16, 48, 128, 144, 2048, 10240):
+                    for k in (16, 256, 272, 1024, 4240, 8192):
+                        pair, bn, sk = ask(plan, int8, batch, batch, m, n, k)
+                        assert (pair, bn, sk) == (1, 256, 1) or (pair == 0 and bn % (32 if sk == 4 else 16) == 0 and 32 <= bn <= 256)
+                        assert sk == 1 or (int8 and sk in (2, 4) and (k + 127) // 128 >= 2 * sk)
+                        assert ask(plan, int8, batch, 1, m, n, k) == ask(folded, int8, 1, 1, batch * m, n, k)
+    assert _lib.lib.q8k_mm_plan(1, 1, 1, 0, 16, 16, ctypes.cast(plan, ctypes.c_void_p)) != 0

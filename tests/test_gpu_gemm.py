@@ -167,42 +167,68 @@ def test_gemm_argument_errors(nat, cuda_device):
                   torch.ones(2, 8, device=d), torch.ones(3, 16, device=d), False, torch.bfloat16)
 
 
+def _check_epilogues(nat, d, kind, B, Bw, M, N, K):
+    """Every epilogue against float64.  INT8 sums are exact and FP8 sums fp32, so a bf16 result is one rounding (at most
+    2^-8 of the value: half of a step of 2^-7) and a few fp32 ones away; GELU adds half of |y| times the 2^-11 of
+    tanh.approx; an e4m3 result is one rounding of 2^-4, or half of the subnormal step."""
+    qd = torch.int8 if kind == "int8" else E4M3
+    g = Hp.gen(M + N + K)
+
+    def mk(*s):
+        if kind == "int8":
+            return torch.randint(-127, 128, s, generator=g, dtype=torch.int8).to(d)
+        return torch.randn(s, generator=g).to(qd).to(d)
+
+    ad, wd = mk(B, M, K), mk(*((Bw, N, K) if Bw > 1 else (N, K)))
+    sad = (torch.rand(B, M, generator=g) * 0.01 + 0.001).to(d)
+    swd = (torch.rand(*((Bw, N) if Bw > 1 else (N,)), generator=g) * 0.01 + 0.001).to(d)
+    bd = (torch.randn(N, generator=g) * 0.1).to(d)
+    y = (ad.double() @ wd.double().transpose(-1, -2)) * sad.double().unsqueeze(-1)
+    y = y * (swd.double().unsqueeze(1) if Bw > 1 else swd.double()) + bd.double()
+    fp32 = 2e-6 * y.abs().max()
+    mm, mmb = (nat.q8_mm, nat.q8_mm_bias) if kind == "int8" else (nat.fp8_mm, nat.fp8_mm_bias)
+    lin = mmb(ad, wd, bd, sad, swd, False, torch.bfloat16)
+    assert bool(((lin.double() - y).abs() <= 2.0 ** -8 * y.abs() + fp32).all())
+    ge = torch.nn.functional.gelu(y, approximate="tanh")
+    out = mmb(ad, wd, bd, sad, swd, True, torch.bfloat16)
+    assert bool(((out.double() - ge).abs() <= 2.0 ** -8 * ge.abs() + 1.02 * 2.0 ** -12 * y.abs() + fp32).all())
+    out8 = mm(ad, wd, sad, swd, False, None)
+    y8 = (y - bd.double()).clamp(-448, 448)
+    assert bool(((out8.double() - y8).abs() <= 2.0 ** -3.9 * y8.abs() + 2.0 ** -9).all())
+    if Bw == 1:
+        gate = torch.randn(B, 1, N, generator=g).to(torch.bfloat16).to(d)
+        resid = torch.randn(B, M, N, generator=g).to(torch.bfloat16).to(d)
+        fused = nat.mm_gate_residual(ad, wd, bd, sad, swd, gate, resid)
+        Hp.assert_bit_equal(fused, (gate * lin + resid).cpu(), "gate and residual in the epilogue")
+
+
 @pytest.mark.parametrize("kind", ["int8", "fp8"])
 @pytest.mark.parametrize("B,M,N,K", [(1, 1, 16, 16), (1, 7, 48, 112), (2, 9, 2064, 640), (1, 77, 10240, 1040), (1, 127, 144, 4112),
                                      (1, 128, 2048, 2048), (3, 129, 272, 272), (1, 300, 2048, 2048), (1, 512, 2064, 8208),
                                      (2, 260, 1040, 1024), (1, 4000, 128, 512), (1, 1000, 96, 144)])
 def test_split_tiles_and_split_k(nat, cuda_device, kind, B, M, N, K):
-    """Tiles of every width, K split over 1, 2 and 4 CTAs with uneven shares, row / column / K tails, batches, and each
-    epilogue.  INT8 partial sums are exact, so only the fp32 epilogue may round differently from float64; FP8 sums are
-    fp32 in another order.  Bounds: half a bf16 step (2^-9) and, for GELU, tanh.approx (2^-11) on top of it."""
-    qd = torch.int8 if kind == "int8" else E4M3
-    g = Hp.gen(M + N + K)
-    if kind == "int8":
-        a = torch.randint(-127, 128, (B, M, K), generator=g, dtype=torch.int8)
-        w = torch.randint(-127, 128, (N, K), generator=g, dtype=torch.int8)
-    else:
-        a, w = torch.randn(B, M, K, generator=g).to(qd), torch.randn(N, K, generator=g).to(qd)
-    sa = torch.rand(B, M, generator=g) * 0.01 + 0.001
-    sw = torch.rand(N, generator=g) * 0.01 + 0.001
-    bias = torch.randn(N, generator=g) * 0.1
-    d = cuda_device
-    ad, wd, sad, swd, bd = (t.to(d) for t in (a, w, sa, sw, bias))
-    y = (ad.double() @ wd.double().T) * sad.double().unsqueeze(-1) * swd.double() + bd.double()
-    mm, mmb = (nat.q8_mm, nat.q8_mm_bias) if kind == "int8" else (nat.fp8_mm, nat.fp8_mm_bias)
-    out = mmb(ad, wd, bd, sad, swd, False, torch.bfloat16)
-    err = (out.double() - y).abs()
-    assert bool((err <= 2.0 ** -8 * y.abs() + 2e-6 * y.abs().max()).all())
-    ge = torch.nn.functional.gelu(y, approximate="tanh")
-    out = mmb(ad, wd, bd, sad, swd, True, torch.bfloat16)
-    assert bool(((out.double() - ge).abs() <= 2.0 ** -8 * ge.abs() + 2.0 ** -10 * y.abs() + 2e-6 * y.abs().max()).all())
-    out8 = mm(ad, wd, sad, swd, False, None)
-    y8 = (y - bd.double()).clamp(-448, 448)
-    assert bool(((out8.double() - y8).abs() <= 2.0 ** -3.9 * y8.abs() + 2.0 ** -9).all())
-    gate = torch.randn(B, 1, N, generator=g).to(torch.bfloat16).to(d)
-    resid = torch.randn(B, M, N, generator=g).to(torch.bfloat16).to(d)
-    lin = mmb(ad, wd, bd, sad, swd, False, torch.bfloat16)
-    fused = nat.mm_gate_residual(ad, wd, bd, sad, swd, gate, resid)
-    Hp.assert_bit_equal(fused, (gate * lin + resid).cpu(), "gate and residual in the epilogue")
+    """Shapes as they come: row / column / K tails and batches on shared weights, each epilogue."""
+    _check_epilogues(nat, cuda_device, kind, B, 1, M, N, K)
+
+
+@pytest.mark.parametrize("bn,sk,Bw,M,N,K", [
+    (32, 1, 3, 33, 96, 272), (48, 1, 1, 120, 6160, 144), (64, 1, 2, 9, 4112, 272), (80, 1, 1, 400, 2576, 272),
+    (96, 1, 1, 900, 1552, 272), (112, 1, 1, 260, 5136, 272), (128, 1, 2, 1000, 1040, 144), (144, 1, 3, 1000, 784, 144),
+    (160, 1, 1, 1300, 2064, 144), (176, 1, 1, 511, 6160, 112), (208, 1, 1, 1300, 2576, 112), (224, 1, 3, 127, 10256, 112),
+    (32, 2, 2, 77, 656, 4112), (48, 2, 1, 100, 3088, 4112), (64, 2, 3, 127, 1168, 4112), (80, 2, 3, 129, 784, 8208),
+    (96, 2, 1, 127, 6160, 4112), (112, 2, 3, 129, 1168, 8208), (128, 2, 2, 129, 2064, 8208), (144, 2, 1, 129, 5136, 8208),
+    (32, 4, 2, 100, 144, 4112), (64, 4, 2, 200, 528, 4112), (96, 4, 2, 260, 528, 8208), (96, 4, 1, 100, 3088, 8208)])
+def test_every_tile_width_and_k_split(nat, cuda_device, bn, sk, Bw, M, N, K):
+    """One shape per tile width and number of K shares that the dispatch uses on 148 SMs, with tails in every direction
+    and, where there is one, a batch of weights.  The choice itself is asserted, so that another cost model cannot take the
+    coverage away unnoticed.  FP8 takes the same width where K is not split, and never splits."""
+    import ctypes
+    from q8_kernels_b200 import _lib
+    plan = (ctypes.c_int * 3)()
+    for kind in ("int8", "fp8"):
+        assert _lib.lib.q8k_mm_plan(int(kind == "int8"), Bw, Bw, M, N, K, ctypes.cast(plan, ctypes.c_void_p)) == 0
+        assert tuple(plan) == (0, bn, sk) if kind == "int8" or sk == 1 else plan[2] == 1, kind
+        _check_epilogues(nat, cuda_device, kind, Bw, Bw, M, N, K)
 
 
 @pytest.mark.parametrize("N,K", [(2048, 8192), (944, 4240), (2064, 4096), (4096, 1024)])
@@ -232,7 +258,7 @@ def test_fp8_row_has_the_same_bits_in_every_call(nat, cuda_device, N, K):
 def test_padded_pair_tiles_and_folded_batches(nat, cuda_device, kind, B, Bw, M, N, K):
     """Pair tiles half of which is padding (three rounds of them, N or M at most 128), a batch on shared weights as rows
     of one product (tiles that straddle batch entries and their gate rows), one activation on a batch of weights.
-    Bounds as in test_split_tiles_and_split_k, without GELU."""
+    Bounds as in _check_epilogues."""
     qd = torch.int8 if kind == "int8" else E4M3
     d = cuda_device
     g = torch.Generator(device=d).manual_seed(M + N + K)
