@@ -370,8 +370,8 @@ def detail_attention(q8, dev, peaks):
     qkv = [torch.randn(B, S, H * D, generator=g, device=dev).to(torch.bfloat16).view(B, S, H, D).transpose(1, 2)
            for _ in range(3)]
     F = q8.functional.flash_attention.flash_attn_func
-    q8_, k8_, vt_ = nat.attention_prep(qkv[0], qkv[1], qkv[2], True, QK_SCALE)
-    ms_core = timed(lambda: nat.flash_attention(q8_, k8_, vt_, 1.0, None, torch.bfloat16), 10)
+    q8_, k8_, v8_ = nat.attention_prep_rows(qkv[0], qkv[1], qkv[2], True, QK_SCALE)     # the route of flash_attn_func
+    ms_core = timed(lambda: nat.flash_attention(q8_, k8_, v8_, 1.0, None, torch.bfloat16, v_rows=True), 10)
     ms_full = timed(lambda: F(qkv[0], qkv[1], qkv[2], apply_qk_hadamard=True, out_dtype=torch.bfloat16), 10)
     fl = 4.0 * B * H * S * S * D
     sm_mhz = float(peaks.get("sm_max_mhz") or 1965.0)
@@ -384,8 +384,8 @@ def detail_attention(q8, dev, peaks):
     kx = [torch.randn(B, 128, H * D, generator=g, device=dev).to(torch.bfloat16).view(B, 128, H, D).transpose(1, 2)
           for _ in range(2)]
     lens = torch.randint(16, 129, (B,), generator=g, device=dev, dtype=torch.int32)
-    q8c, k8c, vtc = nat.attention_prep(qkv[0], kx[0], kx[1], True, QK_SCALE)
-    ms_x = timed(lambda: nat.flash_attention(q8c, k8c, vtc, 1.0, lens, torch.bfloat16), 20)
+    q8c, k8c, v8c = nat.attention_prep_rows(qkv[0], kx[0], kx[1], True, QK_SCALE)
+    ms_x = timed(lambda: nat.flash_attention(q8c, k8c, v8c, 1.0, lens, torch.bfloat16, v_rows=True), 20)
     bytes_x = B * H * S * D * (1 + 2) + 2 * B * H * 128 * D
     gbs = bytes_x / ms_x / 1e6
     out["cross_attention"] = {"shape": "Q [2,32,6144,64] x K/V [2,32,128,64], key lengths " + str(lens.tolist()),
@@ -628,11 +628,11 @@ def run_case(a):
             fn = lambda: nat.attention_prep_v(hv(vf))                                                 # noqa: E731
             work, unit = a.b * skv * a.h * 64 * 3 / 1e9, "GB/s"
         else:
-            q8_, k8_, vt_ = nat.attention_prep(hv(qf), hv(kf), hv(vf), True, QK_SCALE)
+            q8_, k8_, v8_ = nat.attention_prep_rows(hv(qf), hv(kf), hv(vf), True, QK_SCALE)
             lens = None
             if a.case == "cross_attention":
                 lens = torch.randint(16, 129, (a.b,), generator=g, device=dev, dtype=torch.int32)
-            fn = lambda: nat.flash_attention(q8_, k8_, vt_, 1.0, lens, torch.bfloat16)              # noqa: E731
+            fn = lambda: nat.flash_attention(q8_, k8_, v8_, 1.0, lens, torch.bfloat16, v_rows=True)   # noqa: E731
             work = 4.0 * a.b * a.h * a.s * skv * 64 / 1e12
     elif a.case == "dit_block":
         cfg = q8.blocks.LTXStackConfig(num_layers=1)

@@ -509,7 +509,8 @@ def attention_prep(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, apply_hada
     q8_kernels/functional/flash_attention.py:30-60 for bf16 inputs with head dim
     64: q, k, v are [B,H,S,64] tensors or views (any batch / token / head
     strides, last dim contiguous).  Returns q8, k8 [B,H,S,64] and
-    vt8 [B,H,64,ceil16(S_kv)] in e4m3."""
+    vt8 [B,H,64,ceil16(S_kv)] in e4m3: the reference's layout of V, for callers of ``flash_attention`` without
+    ``v_rows``.  ``flash_attn_func`` uses ``attention_prep_rows``."""
     return _attention_prep(lib.q8k_attention_prep, "attention_prep", q, k, v, lambda S: (64, (S + 15) // 16 * 16),
                            apply_hadamard, qk_scale)
 
