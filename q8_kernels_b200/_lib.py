@@ -136,7 +136,7 @@ def ptr(t: Optional[torch.Tensor]) -> Optional[int]:
 
 
 def stream_ptr(device: torch.device) -> int:
-    return torch._C._cuda_getCurrentRawStream(device.index)
+    return torch._C._cuda_getCurrentRawStream(device.index if device.index is not None else torch.cuda.current_device())
 
 
 def launch(dev: torch.device, op: str, fn, *args) -> None:

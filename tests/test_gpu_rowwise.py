@@ -352,3 +352,11 @@ def test_weight_operand_routes(nat, cuda_device, monkeypatch, N, K, fused):
     q_ref, s_ref = nat.tokenwise_quant((b.to(torch.bfloat16) * s[:, None]).T.contiguous(), E4M3)
     Hp.assert_bit_equal(q, q_ref.cpu(), "bytes")
     Hp.assert_bit_equal(sc, s_ref.cpu(), "scales")
+
+
+def test_stream_of_a_device_without_an_index(cuda_device):
+    """The current stream of ``torch.device("cuda")`` is that of the current device."""
+    from q8_kernels_b200 import _lib
+    side = torch.cuda.Stream(cuda_device)
+    with torch.cuda.stream(side):
+        assert _lib.stream_ptr(torch.device("cuda")) == _lib.stream_ptr(cuda_device) == side.cuda_stream
