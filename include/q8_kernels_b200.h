@@ -3,7 +3,11 @@
  *
  * Every entry point takes plain device pointers, sizes and a CUDA stream
  * (passed as void*, i.e. a cudaStream_t), launches asynchronously on that
- * stream, allocates nothing and never synchronises.  The return value is 0 on
+ * stream, allocates nothing and never synchronises.  Most kernels are launched as programmatic dependents of the kernel
+ * before them on the stream and release their own dependents early: a caller's kernel that carries the
+ * programmatic-stream-serialization attribute must execute griddepcontrol.wait (cudaGridDependencySynchronize)
+ * before it touches memory; a kernel launched without the attribute starts after full completion, as always.
+ * The return value is 0 on
  * success or a negative Q8K_ERR_* code; q8k_error_string() explains it and
  * q8k_last_error_detail() gives the message of the last failing call on the
  * calling thread.

@@ -745,7 +745,7 @@ attn_prep_rows_kernel(const __grid_constant__ PrepParams p) {
 // result), optional rotary embedding with shared fp32 tables [S, H*64] (bf16 result), then per head
 // the 64-point Hadamard times `scale` and the c10 e4m3 cast, written head-major [B,H,S,64].  One
 // CTA per token row, 8 elements per thread (thread t owns channels 8t..8t+7, head t/8).  The
-// roundings are those of the separate kernels (rms_norm_kernel, rope_kernel, attn_prep_qk_kernel);
+// roundings are those of the separate kernels (rms_norm_kernel, rope_kernel, attn_prep_rows_kernel);
 // only the summation order of the mean square differs from rms_norm_kernel.
 // MODE 0: one row per CTA.  MODE 1 (x2 / norm_w2 / out2: K next to Q, same shape and row stride): the CTA
 // handles the Q row and the K row of its token, so the rotary table row is loaded once for both and the

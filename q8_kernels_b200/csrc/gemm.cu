@@ -30,10 +30,11 @@ int gemm_num_sms() {
 
 // Tile width and K split of the split kernel, and whether the pair kernel is the better one.  The times (us) come from
 // CUDA-graph timings with weights streamed from HBM, M = 1 .. 6144, N = 1024 .. 10240, K = 1024 .. 8192, and reproduce
-// those to about 10 %:
+// those to about 10 %.  (Fitted without dependent launch, which hides about 2 us of either kernel's set-up.)
 //   split: 4.0 for launch, set-up and drain; per 128-byte K slab the larger of 0.165 (one slab through the issuing
 //          threads) and its bytes at 140 GB/s (one SM's L2 port; 1.7 x the bytes where K is not a multiple of 128 and
-//          rows straddle cache lines), times the CTAs of the busiest SM, and 1.5 for every CTA beyond the first there; 3.85e-5 bn^2 for the epilogue; the exchange of a K split; 0.06 per MB of weights
+//          rows straddle cache lines), times the CTAs of the busiest SM, and 1.5 for every CTA beyond the first there;
+//          3.85e-5 bn^2 for the epilogue; the exchange of a K split; 0.06 per MB of weights
 //   pair:  6.5 + 0.31 per slab and wave of 74 tiles
 // Examples, int8 (pair or 128 x 128 tiles before -> now): M = 128, N = K = 2048 9.5 -> 5.2 (bn 32);  M = 77, N = 10240,
 // K = 4096 15.4 -> 11.6 (bn 80);  M = 128, N = 2048, K = 8192 23.1 -> 9.0 (bn 64, sk 4);  M = 1024, N = 2048, K = 8192

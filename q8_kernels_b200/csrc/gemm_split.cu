@@ -346,8 +346,8 @@ int launch_gemm_split(bool int8, bool gelu, bool out_e4m3, bool resid, const voi
     sp.g.m_tiles = (int)m_tiles;
     sp.g.n_tiles = (int)n_tiles;
     sp.g.total_tiles = (int)total;
-    // A grid that fits the device once gets a deep ring; otherwise two CTAs share an SM.  The ring holds at least two
-    // stages, and with sk > 1 the exchange of 128 x bn words.
+    // A grid that fits the device once gets a deep ring; otherwise two CTAs share an SM.  No more stages than slabs (one for
+    // K <= 128), and with sk > 1 room for the exchange of 128 x bn words.
     const int budget = total * sk <= gemm_num_sms() ? 208 * 1024 : 104 * 1024;
     int stages = budget / sp.stage_bytes;
     const int per_cta = ((p.K + kGemmBK - 1) / kGemmBK + sk - 1) / sk;

@@ -190,7 +190,7 @@ __device__ __forceinline__ void butterfly_groups(float (&v)[V]) {
 // and 2 x the input size of staging, all accesses conflict-free with immediate offsets.  128 registers, 16 warps per SM.
 // Measured, 24576 x 2048, bf16 in, CUDA graph over inputs larger than L2 (one CTA per row pair, block-wide barriers,
 // two exchanges before): bf16 out 43.6 -> 33.7 us (0.92 of the copy rate), e4m3 rows 45.3 -> 35.9 us, int8 rows
-// 47.1 -> 41.5 us (one F2I per element on the 8-clock conversion unit), with norm + modulation 72.3 -> 52.1 us (int8).
+// 47.1 -> 42 us (one F2I per element on the 8-clock conversion unit), with norm + modulation 72.3 -> 52.1 us (int8).
 // 6144 x 8192: 49.5 -> 41.2, 50.1 -> 43.1, 53.2 -> 49.0, 109 -> 73.7 us.  Tried: 128 values per thread for 4096 and
 // 8192 (one exchange, half the warps; 59 us for int8 rows of 8192), XOR swizzles instead of pads (39.4 us, e4m3 rows).
 
