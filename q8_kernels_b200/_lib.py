@@ -99,6 +99,12 @@ def _load() -> ctypes.CDLL:
 
 lib = _load()
 
+try:
+    from . import _host                  # csrc/host.cpp: checks, allocation and launch of the common calls
+except ImportError as e:
+    raise ImportError(f"q8_kernels_b200._host is missing or does not load ({e}): build it with "
+                      "`python q8_kernels_b200/build.py`") from e
+
 
 class Q8KernelError(RuntimeError):
     """A native entry point rejected its arguments or a CUDA call failed."""
@@ -108,6 +114,9 @@ def check(rc: int, op: str) -> None:
     if rc != 0:
         detail = lib.q8k_last_error_detail().decode()
         raise Q8KernelError(f"{op}: {lib.q8k_error_string(rc).decode()} ({rc}): {detail}")
+
+
+_host.set_check(check)
 
 
 def dt(dtype: torch.dtype) -> int:
@@ -164,6 +173,8 @@ def status_word(device: torch.device) -> torch.Tensor:
     if t is None:
         t = torch.zeros(1, dtype=torch.int32, device=device)
         _status_words[key] = t
+        if t.is_cuda:
+            _host.set_status_word(t)
     return t
 
 

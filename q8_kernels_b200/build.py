@@ -1,6 +1,7 @@
 """Build recipe for the native library: every .cu under csrc/ is compiled for
 sm_100a with nvcc into one shared object, ``q8_kernels_b200/libq8k_b200.so``,
-which exports the C ABI declared in ``include/q8_kernels_b200.h``.
+which exports the C ABI declared in ``include/q8_kernels_b200.h``; ``csrc/host.cpp`` becomes the CPython extension
+``q8_kernels_b200/_host.so`` over it, against the headers and libraries of the installed torch.
 
 Run ``python q8_kernels_b200/build.py`` (add ``--force`` to rebuild, ``-v`` for
 ptxas resource usage).  nvcc cross-compiles without a GPU present.
@@ -8,15 +9,18 @@ ptxas resource usage).  nvcc cross-compiles without a GPU present.
 from __future__ import annotations
 
 import argparse
+import importlib.util
 import os
 import subprocess
 import sys
+import sysconfig
 from concurrent.futures import ThreadPoolExecutor
 
 PKG_DIR = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(PKG_DIR, "csrc")
 OBJ_DIR = os.path.join(PKG_DIR, "build")
 LIB_PATH = os.path.join(PKG_DIR, "libq8k_b200.so")
+HOST_PATH = os.path.join(PKG_DIR, "_host.so")
 
 SOURCES = ["capi.cu", "rowwise.cu", "hadamard.cu", "gemm.cu", "gemm_pair.cu", "gemm_split.cu", "attention.cu"]
 
@@ -40,6 +44,25 @@ def _stale(target: str, deps) -> bool:
         return True
     t = os.path.getmtime(target)
     return any(os.path.getmtime(d) > t for d in deps)
+
+
+def _build_host(force: bool) -> None:
+    src = os.path.join(CSRC, "host.cpp")
+    header = os.path.join(PKG_DIR, "..", "include", "q8_kernels_b200.h")
+    torch_dir = os.path.dirname(importlib.util.find_spec("torch").origin)
+    version = os.path.join(torch_dir, "version.py")              # another torch needs another build
+    if not (force or _stale(HOST_PATH, [src, header, version])):
+        return
+    inc = [sysconfig.get_paths()["include"], os.path.join(torch_dir, "include"),
+           os.path.join(torch_dir, "include", "torch", "csrc", "api", "include"),
+           os.path.join(os.path.dirname(os.path.dirname(_nvcc())) if os.path.isabs(_nvcc()) else "/usr/local/cuda", "include")]
+    cmd = (["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden"] + ["-I" + d for d in inc]
+           + [src, "-o", HOST_PATH, "-L" + os.path.join(torch_dir, "lib"), "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_python",
+              "-L" + PKG_DIR, "-l:libq8k_b200.so", "-Wl,-rpath,$ORIGIN"])
+    res = subprocess.run(cmd, capture_output=True, text=True)
+    if res.returncode != 0:
+        sys.stderr.write(res.stdout + res.stderr)
+        raise RuntimeError("g++ failed on host.cpp")
 
 
 def build(force: bool = False, verbose: bool = False) -> str:
@@ -70,6 +93,7 @@ def build(force: bool = False, verbose: bool = False) -> str:
         if res.returncode != 0:
             sys.stderr.write(res.stdout + res.stderr)
             raise RuntimeError("link failed")
+    _build_host(force)
     return LIB_PATH
 
 

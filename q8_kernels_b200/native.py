@@ -4,7 +4,9 @@ names, positional arguments, ``None`` for ``std::optional`` and the same output
 shapes / default dtypes.  Each function checks its arguments, allocates the
 output with torch's caching allocator on the input's device and launches the
 sm_100a kernel through the C ABI on torch's current stream.  Nothing here
-synchronises.
+synchronises.  The ops of the inference and training path first ask ``_host`` (csrc/host.cpp), which does the same in
+native code for plain contiguous tensors on the current device and answers None for everything else; what a function
+accepts and refuses is what its Python body says.
 """
 from __future__ import annotations
 
@@ -15,7 +17,7 @@ import ctypes
 
 import torch
 
-from . import _lib
+from . import _host, _lib
 from ._lib import Q8KernelError, dt, launch, lib, ptr, require_cuda, stream_ptr
 
 E4M3 = torch.float8_e4m3fn
@@ -57,6 +59,9 @@ def _dense_rows(x: torch.Tensor):
 def tokenwise_quant(x: torch.Tensor, out_type: Optional[torch.dtype] = None) -> List[torch.Tensor]:
     """csrc/quantizer/tokenwise_quant.cpp:74-111.  Returns ``[q, scales]`` with
     q shaped like x (int8 by default, or e4m3) and fp32 scales shaped x.shape[:-1]."""
+    fast = _host.tokenwise_quant(x, out_type)
+    if fast is not None:
+        return fast
     dev = require_cuda(x)
     out_type = torch.int8 if out_type is None else out_type
     if out_type not in (torch.int8, E4M3):
@@ -73,6 +78,9 @@ def transpose_quant(x: torch.Tensor, row_scales: Optional[torch.Tensor]) -> List
     """``tokenwise_quant((x * row_scales[:, None]).T.contiguous(), e4m3)`` in one pass, bit-identical: the weight
     operand of the linear backward passes.  x [N,K] int8 / e4m3 with fp32 ``row_scales`` [N], or bf16 with None;
     returns ``[q, scales]`` with q e4m3 [K,N] and fp32 scales [K].  N and K must be multiples of 16."""
+    fast = _host.transpose_quant(x, row_scales)
+    if fast is not None:
+        return fast
     dev = require_cuda(x, row_scales)
     if x.dim() != 2:
         raise Q8KernelError("transpose_quant: x must be [N,K]")
@@ -90,6 +98,9 @@ def transpose_quant(x: torch.Tensor, row_scales: Optional[torch.Tensor]) -> List
 def dequant_hadamard(x: torch.Tensor, row_scales: torch.Tensor, scale: float) -> torch.Tensor:
     """``fast_hadamard_transform((x * row_scales[:, None]).to(bfloat16), scale)`` for int8 x [N,K] with fp32
     ``row_scales`` [N] and 256 < K <= 16384 in one pass, bit-identical."""
+    fast = _host.dequant_hadamard(x, row_scales, scale)
+    if fast is not None:
+        return fast
     dev = require_cuda(x, row_scales)
     if x.dtype != torch.int8 or x.dim() != 2 or row_scales.dtype != torch.float32 or row_scales.numel() != x.shape[0]:
         raise Q8KernelError("dequant_hadamard: x must be int8 [N,K] with float32 row_scales [N]")
@@ -104,6 +115,9 @@ def dequant_hadamard(x: torch.Tensor, row_scales: torch.Tensor, scale: float) ->
 
 def fast_hadamard_transform(x: torch.Tensor, scale: float, out_type: Optional[torch.dtype] = None) -> torch.Tensor:
     """csrc/fast_hadamard/fast_hadamard_transform.cpp:70-121."""
+    fast = _host.fast_hadamard_transform(x, scale, out_type)
+    if fast is not None:
+        return fast
     dev = require_cuda(x)
     if x.dtype not in (torch.bfloat16, E4M3):
         raise Q8KernelError(f"fast_hadamard_transform: input dtype {x.dtype} must be bfloat16 or float8_e4m3fn")
@@ -124,6 +138,9 @@ def hadamard_quant(x: torch.Tensor, scale: float, out_type: Optional[torch.dtype
     """Fused ``tokenwise_quant(fast_hadamard_transform(x, scale), out_type)`` in
     one pass; bit-identical to the two-kernel chain of
     q8_kernels/functional/linear.py:30-31."""
+    fast = _host.hadamard_quant(x, scale, out_type)
+    if fast is not None:
+        return fast
     dev = require_cuda(x)
     out_type = torch.int8 if out_type is None else out_type
     x2, rows, dim, stride = _rows(x)
@@ -140,6 +157,9 @@ def norm_modulate_quant(x: torch.Tensor, mod_scale: torch.Tensor, mod_shift: tor
     per-token quantizer in one kernel, keeping the bf16 roundings of the separate ops
     (q8_kernels/blocks/ltx_transformer_block.py:38-39,53-54 + functional/linear.py:30-31).
     x bf16 [B, S, dim]; mod_scale / mod_shift bf16 [B, 1, dim].  Returns ``[q, scales]``."""
+    fast = _host.norm_modulate_quant(x, mod_scale, mod_shift, out_type)
+    if fast is not None:
+        return fast
     dev = require_cuda(x, mod_scale, mod_shift)
     out_type = torch.int8 if out_type is None else out_type
     if x.dtype != torch.bfloat16 or mod_scale.dtype != torch.bfloat16 or mod_shift.dtype != torch.bfloat16:
@@ -160,6 +180,9 @@ def norm_modulate_quant(x: torch.Tensor, mod_scale: torch.Tensor, mod_shift: tor
 def rms_norm(x: torch.Tensor, weights: Optional[torch.Tensor] = None,
              out_type: Optional[torch.dtype] = None) -> List[torch.Tensor]:
     """csrc/ops/rms_norm.cpp:103-154.  Returns ``[out, rsqrt_per_row]``."""
+    fast = _host.rms_norm(x, weights, out_type)
+    if fast is not None:
+        return fast
     dev = require_cuda(x, weights)
     if weights is not None and weights.dtype != torch.float32:
         raise Q8KernelError("rms_norm: weights must be float32")
@@ -188,6 +211,9 @@ def rope(x: torch.Tensor, cos_freqs: torch.Tensor, sin_freqs: torch.Tensor,
          out_type: Optional[torch.dtype] = None) -> torch.Tensor:
     """csrc/ops/rope.cpp:96-146.  cos/sin are fp32 with x's shape, or with a
     leading batch of 1 that is shared by every batch entry of x."""
+    fast = _host.rope(x, cos_freqs, sin_freqs, out_type)
+    if fast is not None:
+        return fast
     dev = require_cuda(x, cos_freqs, sin_freqs)
     if cos_freqs.dtype != torch.float32 or sin_freqs.dtype != torch.float32:
         raise Q8KernelError("rope: cos/sin tables must be float32")
@@ -264,6 +290,9 @@ def gelu_backward(x: torch.Tensor, grad_output: torch.Tensor, out_type: Optional
 def rope_backward(grad_out: torch.Tensor, cos_freqs: torch.Tensor, sin_freqs: torch.Tensor,
                   out_type: Optional[torch.dtype] = None) -> torch.Tensor:
     """csrc/ops/rope.cpp:150-199: the transposed rotation applied to the incoming gradient."""
+    fast = _host.rope_backward(grad_out, cos_freqs, sin_freqs, out_type)
+    if fast is not None:
+        return fast
     dev = require_cuda(grad_out, cos_freqs, sin_freqs)
     if cos_freqs.dtype != torch.float32 or sin_freqs.dtype != torch.float32:
         raise Q8KernelError("rope_backward: cos/sin tables must be float32")
@@ -289,6 +318,9 @@ def rms_norm_backward(x_normed: torch.Tensor, x_norms: torch.Tensor, grad_out: t
                       weights: Optional[torch.Tensor] = None, out_type: Optional[torch.dtype] = None) -> torch.Tensor:
     """csrc/ops/rms_norm.cpp:157-214: gradient w.r.t. the input of ``rms_norm`` from its saved output
     ``x_normed`` and per-row ``x_norms``.  ``grad_out`` is read in the output dtype, as in the reference."""
+    fast = _host.rms_norm_backward(x_normed, x_norms, grad_out, weights, out_type)
+    if fast is not None:
+        return fast
     dev = require_cuda(x_normed, x_norms, grad_out, weights)
     if weights is not None and weights.dtype != torch.float32:
         raise Q8KernelError("rms_norm_backward: weights must be float32")
@@ -314,6 +346,9 @@ def rms_norm_backward(x_normed: torch.Tensor, x_norms: torch.Tensor, grad_out: t
 # ---------------------------------------------------------------- gemm._C
 
 def _gemm(fn, name, a, b, bias, a_scales, b_scales, fuse_gelu, out_type, in_dtype):
+    fast = _host.mm(a, b, bias, a_scales, b_scales, fuse_gelu, out_type, in_dtype)
+    if fast is not None:
+        return fast
     dev = require_cuda(a, b, bias, a_scales, b_scales)
     for t, what in ((a, "a"), (b, "b"), (bias, "bias"), (a_scales, "a_scales"), (b_scales, "b_scales")):
         if t is not None and not t.is_contiguous():
@@ -369,6 +404,9 @@ def mm_gate_residual(a: torch.Tensor, b: torch.Tensor, bias: Optional[torch.Tens
     q8_mm_bias (or fp8_mm_bias) call plus the two torch ops of
     q8_kernels/blocks/ltx_transformer_block.py:41,52,56, bit-identical to running them separately.
     a int8|e4m3 [B,S,K] (or [M,K]); b [N,K]; gate bf16 [B,1,N] or None; resid bf16 shaped like the output."""
+    fast = _host.mm_gate_residual(a, b, bias, a_scales, b_scales, gate, resid)
+    if fast is not None:
+        return fast
     dev = require_cuda(a, b, bias, a_scales, b_scales, gate, resid)
     if a.dtype != b.dtype or a.dtype not in (torch.int8, E4M3):
         raise Q8KernelError("mm_gate_residual: a and b must both be int8 or both float8_e4m3fn")
@@ -405,6 +443,10 @@ def flash_attention(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, softmax_s
     ``token_major_out`` stores the result as [B,M,H,64] and returns its [B,H,M,64] view, so the
     caller's ``transpose(1,2).reshape(B,M,H*64)`` is free.  ``v_rows``: v is [B,H,N,64] (rows, like k)
     instead of the reference's transposed layout; same result, no transpose pass needed."""
+    if v_rows:
+        fast = _host.flash_attention(q, k, v, softmax_scale, batch_mask, out_type, token_major_out)
+        if fast is not None:
+            return fast
     dev = require_cuda(q, k, v, batch_mask)
     if q.dtype != E4M3 or k.dtype != E4M3 or v.dtype != E4M3:
         raise Q8KernelError("flash_attention: q, k, v must be float8_e4m3fn")
@@ -518,6 +560,9 @@ def attention_prep(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, apply_hada
 def attention_prep_rows(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, apply_hadamard: bool,
                         qk_scale: float) -> Tuple[torch.Tensor, torch.Tensor, torch.Tensor]:
     """attention_prep with V cast to rows [B,H,S_kv,64], for ``flash_attention(v_rows=True)``: one launch."""
+    fast = _host.attention_prep_rows(q, k, v, apply_hadamard, qk_scale)
+    if fast is not None:
+        return fast
     return _attention_prep(lib.q8k_attention_prep_rows, "attention_prep_rows", q, k, v, lambda S: (S, 64),
                            apply_hadamard, qk_scale)
 
@@ -528,6 +573,9 @@ def qk_norm_rope_prep(x: torch.Tensor, norm_w: torch.Tensor, freqs_cis, num_head
     e4m3 cast in one kernel: x bf16 [B,S,H*64] (row-strided views allowed) -> e4m3 [B,H,S,64], with the
     bf16 roundings of q8_kernels/modules/attention.py:54-68 and functional/flash_attention.py:50-54.
     ``freqs_cis`` is None or (cos, sin) fp32 [1,S,H*64]."""
+    fast = _host.qkv_prep(None, x, None, None, norm_w, *(freqs_cis if freqs_cis is not None else (None, None)), num_heads, apply_hadamard, qk_scale)
+    if fast is not None:
+        return fast
     dev = require_cuda(x, norm_w)
     if x.dtype != torch.bfloat16 or x.dim() != 3 or x.shape[2] != num_heads * 64 or x.stride(2) != 1:
         raise Q8KernelError("qk_norm_rope_prep: x must be bfloat16 [B,S,H*64] with contiguous channels")
@@ -552,6 +600,9 @@ def kv_prep(xk: torch.Tensor, xv: torch.Tensor, norm_wk: torch.Tensor, num_heads
             qk_scale: float):
     """K and V of a cross-attention (two column slices of one fused projection output, same strides) in one
     launch: K as qk_norm_rope_prep without rotation, V cast to e4m3 rows; returns (k8, v8), each [B,H,S,64]."""
+    fast = _host.qkv_prep(None, xk, xv, None, norm_wk, None, None, num_heads, apply_hadamard, qk_scale)
+    if fast is not None:
+        return fast
     dev = require_cuda(xk, xv, norm_wk)
     C = num_heads * 64
     for x in (xk, xv):
@@ -578,6 +629,9 @@ def qk_norm_rope_prep_pair(xq: torch.Tensor, xk: torch.Tensor, norm_wq: torch.Te
     strides, e.g. column slices of a fused projection output); returns (q8, k8), each e4m3 [B,H,S,64],
     byte-identical to two separate calls.  With ``xv`` (a third slice of the same kind) the launch also
     casts V to e4m3 rows [B,H,S,64] (what attention_cast_rows gives) and (q8, k8, v8) is returned."""
+    fast = _host.qkv_prep(xq, xk, xv, norm_wq, norm_wk, *(freqs_cis if freqs_cis is not None else (None, None)), num_heads, apply_hadamard, qk_scale)
+    if fast is not None:
+        return fast
     dev = require_cuda(xq, xk, norm_wq, norm_wk, xv)
     C = num_heads * 64
     xs = (xq, xk) if xv is None else (xq, xk, xv)
@@ -654,6 +708,9 @@ def linear(x: torch.Tensor, w: torch.Tensor, w_scales: torch.Tensor, bias: Optio
            use_hadamard: bool, fuse_gelu: bool, out_type: torch.dtype) -> torch.Tensor:
     """Hadamard + per-token quantizer + GEMM in one native call over a cached
     per-device scratch buffer (q8_kernels/functional/linear.py:24-42,138-159)."""
+    fast = _host.linear(x, w, w_scales, bias, use_hadamard, fuse_gelu, out_type)
+    if fast is not None:
+        return fast
     dev = require_cuda(x, w, w_scales, bias)
     K = x.shape[-1]
     x2 = x.contiguous()

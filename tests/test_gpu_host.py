@@ -1,0 +1,121 @@
+"""The native host path (csrc/host.cpp) against the Python bodies of the same functions: the same bits where it answers, and
+no answer where the Python body has to decide."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+E4M3 = torch.float8_e4m3fn
+BF16 = torch.bfloat16
+
+
+class _NoHost:
+    """Stands in for the extension: answers nothing, so the Python body runs."""
+
+    def __getattr__(self, name):
+        return lambda *a: None
+
+
+class _Counting:
+    def __init__(self, host):
+        self.host, self.answers = host, []
+
+    def __getattr__(self, name):
+        def call(*a):
+            r = getattr(self.host, name)(*a)
+            self.answers.append((name, r is not None))
+            return r
+        return call
+
+
+def _cases(dev):
+    g = torch.Generator(device=dev).manual_seed(7)
+
+    def r(*shape):
+        return torch.randn(*shape, generator=g, device=dev)
+
+    def i8(*shape):
+        return torch.randint(-127, 128, shape, generator=g, device=dev, dtype=torch.int8)
+    x, cos, sin = r(2, 33, 512).to(BF16), r(1, 33, 512), r(1, 33, 512)
+    sa, sb, bias = r(66).abs(), r(96).abs(), r(96)
+    qkv = r(2, 33, 1536).to(BF16)
+    heads = r(2, 33, 8, 64).to(BF16).transpose(1, 2)
+    h8 = [r(2, 8, n, 64).to(E4M3) for n in (33, 70, 70)]
+    lens = torch.tensor([70, 3], dtype=torch.int32, device=dev)
+    row = (r(2, 1, 512).to(BF16), r(2, 1, 512).to(BF16))
+    w8 = i8(96, 512)
+    return {
+        "tokenwise_quant": [(x, None), (x, E4M3)],
+        "hadamard_quant": [(x, 0.05, None), (x.to(E4M3), 0.05, E4M3)],
+        "fast_hadamard_transform": [(x, 0.05, None), (x, 0.05, E4M3)],
+        "norm_modulate_quant": [(x,) + row + (None,)],
+        "transpose_quant": [(w8, sb), (x[0, :32].contiguous(), None)],
+        "dequant_hadamard": [(w8, sb, 0.05)],
+        "rms_norm": [(x, None, None), (x, r(512), BF16)],
+        "rms_norm_backward": [(x, sa.view(2, 33), x, r(512), None)],
+        "rope": [(x, cos, sin, None), (x, cos.expand(2, -1, -1).contiguous(), sin.expand(2, -1, -1).contiguous(), torch.float32)],
+        "rope_backward": [(x, cos, sin, BF16)],
+        "q8_mm_bias": [(i8(2, 33, 512), w8, bias, sa, sb, True, BF16)],
+        "q8_mm": [(i8(2, 33, 512), w8, sa, sb, False, None)],
+        "fp8_mm": [(x.to(E4M3), w8.to(BF16).to(E4M3), sa, sb, False, BF16)],
+        "mm_gate_residual": [(i8(2, 33, 512), w8, bias, sa, sb, r(2, 1, 96).to(BF16), r(2, 33, 96).to(BF16)),
+                             (i8(2, 33, 512), w8, None, sa, sb, None, r(2, 33, 96).to(BF16))],
+        "linear": [(x, w8, sb, bias, True, True, BF16), (x[0], w8.to(BF16).to(E4M3), sb, None, False, False, BF16)],
+        "flash_attention": [(*h8, 0.125, None, None, False, True), (*h8, 0.125, lens, BF16, True, True)],
+        "attention_prep_rows": [(heads, heads, heads, True, 0.05)],
+        "qk_norm_rope_prep": [(qkv[..., :512], r(512), (cos, sin), 8, True, 0.05), (qkv[..., :512], r(512), None, 8, False, 1.0)],
+        "kv_prep": [(qkv[..., :512], qkv[..., 512:1024], r(512), 8, True, 0.05)],
+        "qk_norm_rope_prep_pair": [(qkv[..., :512], qkv[..., 512:1024], r(512), r(512), (cos, sin), 8, True, 0.05),
+                                   (qkv[..., :512], qkv[..., 512:1024], r(512), r(512), None, 8, True, 0.05, qkv[..., 1024:])],
+    }
+
+
+def _flat(r):
+    return [r] if isinstance(r, torch.Tensor) else list(r)
+
+
+def _bits(t):
+    return t.contiguous().view({1: torch.uint8, 2: torch.int16, 4: torch.int32}[t.element_size()])
+
+
+def test_host_path_gives_what_the_python_bodies_give(cuda_device, monkeypatch):
+    from q8_kernels_b200 import _lib, native
+    _lib.status_word(cuda_device)
+    host = native._host
+    for name, calls in _cases(cuda_device).items():
+        for args in calls:
+            counting = _Counting(host)
+            monkeypatch.setattr(native, "_host", counting)
+            got = getattr(native, name)(*args)
+            assert counting.answers and counting.answers[0][1], f"{name}: the native path did not answer"
+            monkeypatch.setattr(native, "_host", _NoHost())
+            want = getattr(native, name)(*args)
+            assert type(got) is type(want), name
+            for a, b in zip(_flat(got), _flat(want)):
+                assert a.shape == b.shape and a.stride() == b.stride() and a.dtype == b.dtype, name
+                assert torch.equal(_bits(a), _bits(b)), name
+
+
+def test_host_path_leaves_everything_else_to_python(cuda_device):
+    """Strided, wrapped, traced and mistyped arguments, and what is to be refused: None, and the Python body's own error."""
+    from torch.utils._python_dispatch import TorchDispatchMode
+    from q8_kernels_b200 import _host, native
+
+    class Mode(TorchDispatchMode):
+        def __torch_dispatch__(self, func, types, args=(), kwargs=None):
+            return func(*args, **(kwargs or {}))
+    x = torch.randn(4, 32, 512, device=cuda_device).to(BF16)
+    assert _host.hadamard_quant(x, 0.05, None) is not None
+    assert _host.hadamard_quant(x[:, ::2], 0.05, None) is None
+    assert _host.hadamard_quant(x.cpu(), 0.05, None) is None
+    assert _host.hadamard_quant(x, 1, None) is None              # not a float
+    assert _host.hadamard_quant(x, 0.05) is None
+    assert _host.hadamard_quant(x, 0.05, BF16) is None
+    with Mode():
+        assert _host.hadamard_quant(x, 0.05, None) is None
+    assert torch.func.vmap(lambda t: torch.tensor(_host.hadamard_quant(t, 0.05, None) is None))(x).all()
+    with pytest.raises(native.Q8KernelError):
+        native.hadamard_quant(x, 0.05, BF16)
+    with pytest.raises(native.Q8KernelError):                   # refused by the kernel's entry point, not by a check before it
+        native.fast_hadamard_transform(torch.zeros(2, 32768, device=cuda_device, dtype=BF16), 1.0)
+    with pytest.raises(native.Q8KernelError):
+        native.q8_mm(x.to(E4M3), x[0].to(E4M3), torch.ones(128, device=cuda_device), torch.ones(32, device=cuda_device), False, BF16)
