@@ -70,19 +70,41 @@ struct PairParams {
     int m_tiles2;                            // 256-row tiles per batch entry
     int n_tiles2;
     int total_tiles2;
+    // tiles below full_tiles2 are 256 columns wide; those from it on cover the row blocks from narrow_m on, in narrow_n tiles of
+    // narrow_bn columns each (one batch entry; see narrow_plan)
+    int full_tiles2, narrow_m, narrow_n, narrow_bn;
     int tma_store;                           // 1: the epilogue stores through tmap_c
 };
 
-template <bool INT8, bool GELU, bool OUT_E4M3, bool RESID>
+// Where a tile of the launch lies.
+struct PairTile { int m_blk, batch, n0, bn; };
+template <bool NARROW>
+__device__ __forceinline__ PairTile pair_tile(const PairParams& pp, int tile) {
+    PairTile t;
+    if (!NARROW || tile < pp.full_tiles2) {
+        t.bn = kPairBN;
+        t.n0 = tile % pp.n_tiles2 * kPairBN;
+        t.m_blk = (tile / pp.n_tiles2) % pp.m_tiles2;
+        t.batch = tile / (pp.n_tiles2 * pp.m_tiles2);
+    } else {
+        const int i = tile - pp.full_tiles2;
+        t.bn = pp.narrow_bn;
+        t.n0 = i % pp.narrow_n * pp.narrow_bn;
+        t.m_blk = pp.narrow_m + i / pp.narrow_n;
+        t.batch = 0;
+    }
+    return t;
+}
+
+// NARROW: the launch has narrow tiles (see narrow_plan).
+template <bool INT8, bool GELU, bool OUT_E4M3, bool RESID, bool NARROW>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1)
 gemm_8bit_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
-                      const __grid_constant__ CUtensorMap tmap_c, const __grid_constant__ CUtensorMap tmap_r,
+                      const __grid_constant__ CUtensorMap tmap_bn, const __grid_constant__ CUtensorMap tmap_c, const __grid_constant__ CUtensorMap tmap_r,
                       const PairParams pp) {
     using L = PairSmemT<RESID>;
     constexpr int kPairStages = L::kStages;
     const GemmParams& p = pp.g;
-    constexpr uint32_t IDESC = INT8 ? ptx::make_idesc_s8(2 * kGemmBM, kPairBN) : ptx::make_idesc_e4m3(2 * kGemmBM, kPairBN);
-
     extern __shared__ __align__(1024) uint8_t smem[];
     const uint32_t smem_base = ptx::smem_u32(smem);
     if (smem_base & 1023u) {                                   // same offset in both CTAs: both leave
@@ -167,18 +189,18 @@ gemm_8bit_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
             uint32_t ph = 1;                                   // empty_bar phase to wait for: the first round passes
             bool ok = true;
             for (int tile = cluster_id; ok && tile < pp.total_tiles2; tile += num_clusters) {
-                const int n_blk = tile % pp.n_tiles2;
-                const int m_blk = (tile / pp.n_tiles2) % pp.m_tiles2;
-                const int batch = tile / (pp.n_tiles2 * pp.m_tiles2);
-                const int a_row = (p.batch_a ? batch * p.M : 0) + m_blk * 2 * kGemmBM + (int)rank * kGemmBM;
-                const int b_row = (p.batch_b ? batch * p.N : 0) + n_blk * kPairBN + (int)rank * (kPairBN / 2);
+                const PairTile pt = pair_tile<NARROW>(pp, tile);
+                const int a_row = (p.batch_a ? pt.batch * p.M : 0) + pt.m_blk * 2 * kGemmBM + (int)rank * kGemmBM;
+                const int b_row = (p.batch_b ? pt.batch * p.N : 0) + pt.n0 + (int)rank * (pt.bn / 2);
+                const CUtensorMap* map_b = !NARROW || pt.bn == kPairBN ? &tmap_b : &tmap_bn;
+                const uint32_t bytes = L::kABytes + (uint32_t)(pt.bn / 2) * kGemmBK;
                 for (int kb = 0; kb < k_iters; ++kb) {
                     if (!ptx::mbar_wait(empty_bar(s), ph, abort_flag)) { ok = false; break; }
                     const uint32_t fb = leader_full0 + 8u * s;
-                    ptx::mbar_arrive_expect_tx_cluster(fb, L::kStageBytes);
+                    ptx::mbar_arrive_expect_tx_cluster(fb, bytes);
                     const uint32_t a_dst = smem_base + s * L::kStageBytes;
                     ptx::tma_load_2d_pair(a_dst, &tmap_a, fb, kb * kGemmBK, a_row);
-                    ptx::tma_load_2d_pair(a_dst + L::kABytes, &tmap_b, fb, kb * kGemmBK, b_row);
+                    ptx::tma_load_2d_pair(a_dst + L::kABytes, map_b, fb, kb * kGemmBK, b_row);
                     if (++s == kPairStages) { s = 0; ph ^= 1u; }
                 }
             }
@@ -197,6 +219,8 @@ gemm_8bit_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
                 if (!ptx::mbar_wait(tmem_empty_bar(acc), acc_ph ^ 1u, abort_flag)) { ok = false; break; }
                 ptx::tcgen05_fence_after_sync();
                 const uint32_t d_tmem = tmem_base + acc * kPairBN;
+                const int bn = !NARROW || tile < pp.full_tiles2 ? kPairBN : pp.narrow_bn;
+                const uint32_t idesc = INT8 ? ptx::make_idesc_s8(2 * kGemmBM, bn) : ptx::make_idesc_e4m3(2 * kGemmBM, bn);
                 for (int kb = 0; kb < k_iters; ++kb) {
                     if (!ptx::mbar_wait(full_bar(s), ph, abort_flag)) { ok = false; break; }
                     ptx::tcgen05_fence_after_sync();
@@ -206,8 +230,8 @@ gemm_8bit_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
 #pragma unroll
                     for (int k = 0; k < kGemmBK / 32; ++k) {
                         const uint32_t accumulate = (kb > 0 || k > 0) ? 1u : 0u;
-                        if constexpr (INT8) ptx::mma_i8_pair(d_tmem, a_desc + 2 * k, b_desc + 2 * k, IDESC, accumulate);
-                        else ptx::mma_f8f6f4_pair(d_tmem, a_desc + 2 * k, b_desc + 2 * k, IDESC, accumulate);
+                        if constexpr (INT8) ptx::mma_i8_pair(d_tmem, a_desc + 2 * k, b_desc + 2 * k, idesc, accumulate);
+                        else ptx::mma_f8f6f4_pair(d_tmem, a_desc + 2 * k, b_desc + 2 * k, idesc, accumulate);
                     }
                     // the stage is reusable in BOTH CTAs once these MMAs retire
                     ptx::tcgen05_commit_both(empty_bar(s));
@@ -222,8 +246,7 @@ gemm_8bit_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
         const int quarter = warp & 3;
         const int half = (warp - 2) >> 2;
         const int epi_tid = threadIdx.x - 64;
-        constexpr int HALF_COLS = kPairBN / 2;
-        constexpr int NCH = HALF_COLS / 32;
+        constexpr int NCH = kPairBN / 2 / 32;                  // 32-column chunks of this warp, at most
         const bool staged = pp.tma_store != 0;
         const uint32_t store_base = smem_base + L::kStoreOffset + (uint32_t)(warp - 2) * 2u * L::kStoreBoxBytes;
         uint32_t tile_i = 0;
@@ -232,10 +255,11 @@ gemm_8bit_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
         const uint32_t resid_base = smem_base + L::kResidOffset + (uint32_t)(warp - 2) * 2u * L::kStoreBoxBytes;
         bool ok = true;
         for (int tile = cluster_id; tile < pp.total_tiles2; tile += num_clusters, ++tile_i) {
-            const int n_blk = tile % pp.n_tiles2;
-            const int m_blk = (tile / pp.n_tiles2) % pp.m_tiles2;
-            const int batch = tile / (pp.n_tiles2 * pp.m_tiles2);
-            const int n0 = n_blk * kPairBN;
+            const PairTile pt = pair_tile<NARROW>(pp, tile);
+            const int m_blk = pt.m_blk, batch = pt.batch, n0 = pt.n0;
+            // 32-column chunks of the tile: the first half of them (rounded up) are those of warps 2-5, the rest of 6-9
+            const int nch_lo = NARROW ? (pt.bn / 32 + 1) / 2 : NCH;
+            const int nch = !NARROW || half == 0 ? nch_lo : pt.bn / 32 - nch_lo;
             const uint32_t acc = tile_i & 1u;
             const uint32_t acc_ph = (tile_i >> 1) & 1u;
 
@@ -244,7 +268,7 @@ gemm_8bit_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
             if constexpr (RESID)
                 gate_row_tile = (((int64_t)batch * p.M + m_blk * 2 * kGemmBM + (int)rank * kGemmBM) / p.rows_per_gate) * p.N;
             asm volatile("bar.sync 1, 256;" ::: "memory");
-            for (int c = epi_tid; c < kPairBN; c += kGemmEpilogueThreads) {
+            for (int c = epi_tid; c < pt.bn; c += kGemmEpilogueThreads) {
                 const int n = n0 + c;
                 const bool in = n < p.N;
                 col_scale_smem[c] = in ? p.b_scales[(p.batch_b ? (int64_t)batch * p.N : 0) + n] : 0.f;
@@ -260,7 +284,7 @@ gemm_8bit_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
             const float sa = row_ok ? p.a_scales[(p.batch_a ? (int64_t)batch * p.M : 0) + row] : 0.f;
             const int64_t out_row = ((int64_t)batch * p.M + row) * p.N;
             const int64_t gate_row = RESID ? (((int64_t)batch * p.M + row) / p.rows_per_gate) * p.N : 0;
-            const int col_base = half * HALF_COLS;
+            const int col_base = half * nch_lo * 32;
             const uint32_t t_row = tmem_base + ((uint32_t)(quarter * 32) << 16) + acc * kPairBN + col_base;
 
             // Residual of this warp's 32 rows, one 32-column chunk per box (staged bf16 path): TMA loads it
@@ -269,7 +293,7 @@ gemm_8bit_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
             // residual is not paid inside the chunk that uses it.
             auto issue_resid = [&](int c) {                     // lane 0; chunks with columns inside N only
                 const int nc = n0 + col_base + c * 32;
-                if (nc < p.N) {
+                if (nc < p.N && (!NARROW || c < nch)) {
                     const uint32_t rb = resid_bar(warp - 2, (int)(resid_i & 1u));
                     ptx::mbar_arrive_expect_tx(rb, L::kStoreBoxBytes);
                     ptx::tma_load_3d(resid_base + (resid_i & 1u) * L::kStoreBoxBytes, &tmap_r, rb, nc * 2,
@@ -294,8 +318,9 @@ gemm_8bit_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
             ptx::tmem_ld_32x32b_x32(t_row, r[0]);
 #pragma unroll
             for (int c = 0; c < NCH; ++c) {
+                if (NARROW && c >= nch) break;                 // (warp-uniform)
                 ptx::tmem_wait_ld();
-                if (c + 1 < NCH) ptx::tmem_ld_32x32b_x32(t_row + (c + 1) * 32, r[(c + 1) & 1]);
+                if (c + 1 < NCH && (!NARROW || c + 1 < nch)) ptx::tmem_ld_32x32b_x32(t_row + (c + 1) * 32, r[(c + 1) & 1]);
                 const int cl = col_base + c * 32;
                 const int nc = n0 + cl;
                 uint32_t rs_cur[16];
@@ -481,11 +506,11 @@ gemm_8bit_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
 }
 
 // ------------------------------------------------------------------ host side
-template <bool INT8, bool GELU, bool OUT_E4M3, bool RESID = false>
-static int launch_pair(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tc, const CUtensorMap& tr,
-                       const PairParams& pp, cudaStream_t st) {
+template <bool INT8, bool GELU, bool OUT_E4M3, bool RESID, bool NARROW>
+static int launch_pair_as(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tbn, const CUtensorMap& tc,
+                       const CUtensorMap& tr, const PairParams& pp, cudaStream_t st) {
     using PairSmem = PairSmemT<RESID>;
-    auto kern = gemm_8bit_pair_kernel<INT8, GELU, OUT_E4M3, RESID>;
+    auto kern = gemm_8bit_pair_kernel<INT8, GELU, OUT_E4M3, RESID, NARROW>;
     static std::atomic<uint64_t> smem_done{0};
     if (int rc = allow_dynamic_smem((const void*)kern, PairSmem::kDynamic, smem_done)) return rc;
     // how many 2-CTA clusters can be resident at once (cached per kernel variant)
@@ -506,8 +531,46 @@ static int launch_pair(const CUtensorMap& ta, const CUtensorMap& tb, const CUten
     }
     if (max_clusters < 8) return Q8K_ERR_UNSUPPORTED;
     const int clusters = pp.total_tiles2 < max_clusters ? pp.total_tiles2 : max_clusters;
-    Q8K_CUDA_OK(launch_dependent(kern, 2 * clusters, kGemmThreads, PairSmem::kDynamic, st, 1, ta, tb, tc, tr, pp));
+    Q8K_CUDA_OK(launch_dependent(kern, 2 * clusters, kGemmThreads, PairSmem::kDynamic, st, 1, ta, tb, tbn, tc, tr, pp));
     return Q8K_OK;
+}
+
+template <bool INT8, bool GELU, bool OUT_E4M3, bool RESID = false>
+static int launch_pair(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tbn, const CUtensorMap& tc,
+                       const CUtensorMap& tr, const PairParams& pp, cudaStream_t st) {
+    return pp.narrow_bn != kPairBN ? launch_pair_as<INT8, GELU, OUT_E4M3, RESID, true>(ta, tb, tbn, tc, tr, pp, st)
+                                   : launch_pair_as<INT8, GELU, OUT_E4M3, RESID, false>(ta, tb, tbn, tc, tr, pp, st);
+}
+
+// The last round of 256 x 256 tiles may leave most of the clusters idle: M = 6144, N = 2048 are 192 tiles, two rounds of 74 and
+// one of 44.  Then only the row blocks that fill whole rounds keep the wide tiles, and those left are cut into tiles of
+// equal, smaller width, as many as the clusters that are free: 18 row blocks of 8 wide tiles, 6 of 13 tiles of 160 columns.
+// Widths are multiples of 32 (cta_group::2).  An element's accumulator takes the same products in the same order.
+// Measured (CUDA graphs, us, wide tiles only -> with narrow ones): M = 6144, N = 2048 int8 K = 2048 20.6 -> 19.5, fp8 21.6 ->
+// 20.6, K = 8192 75.2 -> 72.3, with the residual 72.9 -> 70.9;  M = 2002, N = 6144, K = 2048 21.6 -> 20.6;  M = 7401, N = 2048
+// 25.9 -> 24.6;  M = 10416, N = 2048, K = 8192 125 -> 117.  A narrow tile costs more than its width (the A rows are
+// loaded for fewer columns, and there is one more epilogue), so 224 columns gain nothing (576 tiles 57.0 against 57.4, 504
+// tiles 59.3 against 64.1), nor does a short K: K = 1024 26.0 against 26.9, with the residual, whose epilogue is the
+// slower part of a short tile, K = 2048 25.5 against 26.2 and K = 1024 33.2 against 35.0.
+static void narrow_plan(PairParams& pp, int64_t batch, int clusters, bool resid) {
+    pp.full_tiles2 = pp.total_tiles2;
+    pp.narrow_m = pp.m_tiles2;
+    pp.narrow_n = 1;
+    pp.narrow_bn = kPairBN;
+    const int rounds = pp.total_tiles2 / clusters;
+    if (batch != 1 || rounds < 1 || rounds > 8 || pp.total_tiles2 % clusters == 0 || pp.g.K < (resid ? 4096 : 2048)) return;
+    const int full_m = rounds * clusters / pp.n_tiles2;        // row blocks in the full rounds
+    const int rest = pp.m_tiles2 - full_m;                     // (at least one: a round is left over)
+    const int slots = rounds * clusters - full_m * pp.n_tiles2 + clusters;   // what is left of them, and one more round
+    const int per_row = slots / rest;                          // tiles that a row block may have
+    if (per_row <= pp.n_tiles2) return;
+    const int bn = ((pp.g.N + per_row - 1) / per_row + 31) / 32 * 32;
+    if (bn > 192) return;
+    pp.full_tiles2 = full_m * pp.n_tiles2;
+    pp.narrow_m = full_m;
+    pp.narrow_bn = bn;
+    pp.narrow_n = (pp.g.N + bn - 1) / bn;
+    pp.total_tiles2 = pp.full_tiles2 + rest * pp.narrow_n;
 }
 
 int launch_gemm_pair(bool int8, bool gelu, bool out_e4m3, bool resid, const void* a, const void* b, const GemmParams& p,
@@ -550,16 +613,24 @@ int launch_gemm_pair(bool int8, bool gelu, bool out_e4m3, bool resid, const void
     const int64_t total = (int64_t)pp.m_tiles2 * pp.n_tiles2 * batch;
     if (total > 0x7fffffffLL) return Q8K_ERR_UNSUPPORTED;
     pp.total_tiles2 = (int)total;
+    narrow_plan(pp, batch, gemm_num_sms() / 2, resid);
+    CUtensorMap tbn = tb;
+    if (pp.narrow_bn != kPairBN) {
+        const uint64_t dims[2] = {(uint64_t)p.K, (uint64_t)p.N};
+        const uint64_t strides[1] = {(uint64_t)p.K};
+        const uint32_t box[2] = {(uint32_t)kGemmBK, (uint32_t)(pp.narrow_bn / 2)};
+        if (int rc = make_byte_tensor_map(&tbn, b, 2, dims, strides, box, 128, op)) return rc;
+    }
 #define Q8K_PAIR(I8)                                                                  \
     do {                                                                              \
-        if (gelu) return out_e4m3 ? launch_pair<I8, true, true>(ta, tb, tc, tr, pp, st)       \
-                                  : launch_pair<I8, true, false>(ta, tb, tc, tr, pp, st);     \
-        return out_e4m3 ? launch_pair<I8, false, true>(ta, tb, tc, tr, pp, st)                \
-                        : launch_pair<I8, false, false>(ta, tb, tc, tr, pp, st);              \
+        if (gelu) return out_e4m3 ? launch_pair<I8, true, true>(ta, tb, tbn, tc, tr, pp, st)       \
+                                  : launch_pair<I8, true, false>(ta, tb, tbn, tc, tr, pp, st);     \
+        return out_e4m3 ? launch_pair<I8, false, true>(ta, tb, tbn, tc, tr, pp, st)                \
+                        : launch_pair<I8, false, false>(ta, tb, tbn, tc, tr, pp, st);              \
     } while (0)
     if (resid) {
-        return int8 ? launch_pair<true, false, false, true>(ta, tb, tc, tr, pp, st)
-                    : launch_pair<false, false, false, true>(ta, tb, tc, tr, pp, st);
+        return int8 ? launch_pair<true, false, false, true>(ta, tb, tbn, tc, tr, pp, st)
+                    : launch_pair<false, false, false, true>(ta, tb, tbn, tc, tr, pp, st);
     }
     if (int8) Q8K_PAIR(true);
     Q8K_PAIR(false);

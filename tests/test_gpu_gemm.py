@@ -284,3 +284,34 @@ def test_padded_pair_tiles_and_folded_batches(nat, cuda_device, kind, B, Bw, M, 
         resid = torch.randn(B, M, N, generator=g, device=d).to(torch.bfloat16)
         fused = nat.mm_gate_residual(a, w, bias, sa, sw, gate, resid)
         Hp.assert_bit_equal(fused, gate * out + resid, "gate and residual in the epilogue")
+
+
+@pytest.mark.parametrize("M,N,K", [(6144, 2048, 2048),            # 13 tiles of 160 columns for each of 6 row blocks
+                                   (6100, 2000, 2064),            # M, N and K tails, the last narrow tile partial
+                                   (2002, 6144, 2048), (3096, 2048, 4112), (12510, 2048, 2048), (7401, 2048, 4096)])
+@pytest.mark.parametrize("kind", ["int8", "fp8", "fp8 e4m3 out", "int8 gelu", "int8 residual", "fp8 residual"])
+def test_narrow_tiles_of_the_last_round(cuda_device, M, N, K, kind):
+    """Products whose last round is cut into narrow tiles: every row has the bits that it has in a call of few rows (other
+    tiles on the other kernel), where int8 sums are exact and fp8 sums have one order."""
+    from q8_kernels_b200 import native as nat
+    g = torch.Generator(device=cuda_device).manual_seed(M + N + K)
+    if kind.startswith("int8"):
+        a, b = (torch.randint(-127, 128, s, generator=g, device=cuda_device, dtype=torch.int8) for s in ((M, K), (N, K)))
+    else:
+        a, b = (torch.randn(s, generator=g, device=cuda_device).to(torch.float8_e4m3fn) for s in ((M, K), (N, K)))
+    sa, sb = torch.rand(M, generator=g, device=cuda_device) / K, torch.rand(N, generator=g, device=cuda_device)
+    bias = torch.randn(N, generator=g, device=cuda_device)
+    resid = torch.randn(1, M, N, generator=g, device=cuda_device).to(torch.bfloat16)
+    gate = torch.randn(1, 1, N, generator=g, device=cuda_device).to(torch.bfloat16)
+    out = torch.float8_e4m3fn if "e4m3" in kind else torch.bfloat16
+
+    def product(r):
+        if "residual" in kind:
+            return nat.mm_gate_residual(a[r], b, bias, sa[r], sb, gate, resid[:, r])
+        mm = nat.q8_mm_bias if kind.startswith("int8") else nat.fp8_mm_bias
+        return mm(a[r], b, bias, sa[r], sb, "gelu" in kind, out)
+    got = product(slice(0, M))[0]
+    for r0 in range(0, M, 512):
+        r = slice(r0, min(r0 + 512, M))
+        want = product(r)[0]
+        assert torch.equal(got[r].view(torch.uint8), want.view(torch.uint8)), (r0, (got[r] != want).sum())
