@@ -30,9 +30,9 @@
 //               row max of the warp moved -- O *= alpha in TMEM through the
 //               registers of the finished half; at the end O / l is parked in the warp's own
 //               P rows and leaves through TMA stores (whole-row plain stores for several outputs)
-// Three mbarriers carry the steady state: step_end (softmax -> MMA threads: P written, O
+// These mbarriers carry the steady state: step_end (softmax -> MMA threads: P written, O
 // rescaled, S read), s_full (one commit from each MMA thread -> softmax: next scores landed AND the
-// previous P.V retired) and slot_free (MMA -> TMA).  Every wait is on consecutive phases
+// previous P.V retired) and one slot_free per K/V slot (MMA -> TMA).  Every wait is on consecutive phases
 // of its barrier, no barrier can complete a second phase before its waiters have seen the first,
 // so a parity is never ambiguous; and every wait is bounded.
 // With at most three key blocks (cross-attention) a CTA keeps K/V and walks over several query
@@ -68,8 +68,8 @@ struct AttnSmem {
     static constexpr int kPOff = kVOff + kAttnKS * kVBytes;
     static constexpr int kQ2Off = kPOff + 2 * kPBytes;             // second Q buffer (several query tiles per CTA)
     static constexpr int kBarOff = kQ2Off + kQBytes;
-    // q_full[2], k_full[3], v_full[3], slot_free, s_full, step_end, q_free[2]
-    static constexpr int kNumBars = 2 + 2 * kAttnKS + 3 + 2;
+    // q_full[2], k_full[3], v_full[3], slot_free[3], s_full, step_end, q_free[2]
+    static constexpr int kNumBars = 2 + 3 * kAttnKS + 2 + 2;
     static constexpr int kTmemPtrOff = kBarOff + kNumBars * 8;
     static constexpr int kAbortOff = kTmemPtrOff + 4;
     static constexpr int kTotal = kAbortOff + 4;
@@ -169,14 +169,18 @@ flash_attn_fp8_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
     auto q_full = [&](int i) { return bar_base + 8u * i; };
     auto k_full = [&](int s) { return bar_base + 8u * (2 + s); };
     auto v_full = [&](int s) { return bar_base + 8u * (2 + kAttnKS + s); };
-    // The three below complete their phases in a fixed order (per query tile: slot_free nblk, s_full nblk + 2,
-    // step_end nblk + 1, or nblk + 2 with MULTI) and every waiter consumes them in that order.  No barrier can
-    // be more than one completed phase ahead of a thread that still has to wait on it: the protocol makes
-    // every producer depend on that waiter before it can complete a second one.
-    const uint32_t slot_free = bar_base + 8u * (2 + 2 * kAttnKS);   // P.V(i) and Q.K^T(i+2) retired
-    const uint32_t s_full = slot_free + 8u;                         // see the MMA issuer
-    const uint32_t step_end = slot_free + 16u;                      // softmax: prologue, one per step, (MULTI) epilogue reached
-    auto q_free = [&](int i) { return slot_free + 24u + 8u * i; };  // MULTI: all tensor-core reads of Q buffer i retired
+    // K and V slot s: P.V(i) (i = s mod 3) retired, and with it all reads of the slot.  One barrier per slot: its next
+    // phase needs the block that the producer loads after it has seen this one.  A barrier shared by the slots could
+    // complete two phases while the producer is held up between two waits (the two blocks behind are loaded already),
+    // and a wait for a parity then never ends.
+    auto slot_free = [&](int s) { return bar_base + 8u * (2 + 2 * kAttnKS + s); };
+    // The two below complete their phases in a fixed order (per query tile: s_full nblk + 2, step_end nblk + 1, or
+    // nblk + 2 with MULTI) and every waiter consumes them in that order.  No barrier can be more than one completed
+    // phase ahead of a thread that still has to wait on it: each phase needs every waiter of the one before.
+    // tests/test_attention_protocol.py walks through all orders of events.
+    const uint32_t s_full = bar_base + 8u * (2 + 3 * kAttnKS);      // see the MMA issuer
+    const uint32_t step_end = s_full + 8u;                          // softmax: prologue, one per step, (MULTI) epilogue reached
+    auto q_free = [&](int i) { return s_full + 16u + 8u * i; };     // MULTI: all tensor-core reads of Q buffer i retired
     auto q_off = [&](int i) { return (uint32_t)(i ? L::kQ2Off : L::kQOff); };
     volatile uint32_t* tmem_ptr_smem = reinterpret_cast<volatile uint32_t*>(smem + L::kTmemPtrOff);
     const uint32_t abort_addr = smem_base + L::kAbortOff;
@@ -221,8 +225,8 @@ flash_attn_fp8_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
         for (int s = 0; s < kAttnKS; ++s) {
             ptx::mbar_init(k_full(s), 1);
             ptx::mbar_init(v_full(s), 1);
+            ptx::mbar_init(slot_free(s), 1);
         }
-        ptx::mbar_init(slot_free, 1);
         ptx::mbar_init(s_full, 2);                              // one commit from each of the two MMA-issuing threads
         ptx::mbar_init(step_end, 4);
         ptx::mbar_init(q_free(0), 1);
@@ -293,12 +297,11 @@ flash_attn_fp8_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
                 } else {
                     for (int i = 0; i + kAttnKS < nblk; ++i) {
                         // K(i) was consumed before step i, V(i) by P.V(i): both slots i % 3 are free
-                        bounded_wait(slot_free, (uint32_t)i & 1u, abort_addr, 4);
+                        bounded_wait(slot_free(i % kAttnKS), (uint32_t)(i / kAttnKS) & 1u, abort_addr, 4);
                         if (*abort_flag != 0) break;            // a wait was abandoned: issue nothing more
                         load_kv(i + kAttnKS);
                     }
                 }
-                // (slot_free phases that are never waited on simply complete.)
                 if (*abort_flag != 0) {
                     // grace period for copies still in flight: they land within microseconds
                     const unsigned long long t0 = ptx::globaltimer_ns();
@@ -343,10 +346,10 @@ flash_attn_fp8_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
                                 ptx::mma_f8f6f4(o_tmem, p_desc + 2 * k, v_desc + V_KSTEP * k, IDESC_PV, (i > 0 || k > 0) ? 1u : 0u);
                             ptx::tcgen05_commit(s_full);
                             // K(i) was read by Q.K^T(i), whose scores the softmax warps have long consumed
-                            ptx::tcgen05_commit(slot_free);
+                            if (!MULTI && i + kAttnKS < nblk) ptx::tcgen05_commit(slot_free(s));
                         }
                         // (the last Q.K^T of the tile retired before the softmax warps could finish its block)
-                        if (MULTI) ptx::tcgen05_commit(q_free(t & 1));
+                        if (MULTI && t + 2 < n_tiles) ptx::tcgen05_commit(q_free(t & 1));
                     } else {
                         const uint64_t q_desc = ptx::make_kmajor_desc(smem_base + q_off(t & 1), 64);
                         auto issue_qk = [&](int j) {
