@@ -439,3 +439,42 @@ def test_gate_residual_tail_over_wide_exponent_ranges(q8, cuda_device):
     got = q8.native.mm_gate_residual(aq, wq, bias, sa, sw, gate, resid)
     assert torch.equal(Hp.bits(got), Hp.bits(want))
 
+
+
+@pytest.mark.parametrize("shape,rank", [((2, 33), 4), ((1, 130), 16), ((70,), 8)])
+@pytest.mark.parametrize("gelu", [False, True])
+def test_adapter_products_over_all_batch_entries(cuda_device, shape, rank, gelu):
+    """Output and low-rank gradients of the adapter linear against the same products in fp32 on the tensors that the 16-bit
+    path holds: one rounding of each 16-bit result (2^-8), and of the intermediate (s @ r) products."""
+    import q8_kernels_b200 as q8
+    g = torch.Generator(device=cuda_device).manual_seed(rank)
+    K, N = 512, 384
+    m = q8.modules.Q8LinearLora(K, N, rank, device=cuda_device)
+    w = torch.randn(N, K, generator=g, device=cuda_device).to(torch.bfloat16)
+    m.weight.data, m.scales.data = q8.native.hadamard_quant(w, K ** -0.5, torch.int8)
+    m.bias.data = torch.randn(N, generator=g, device=cuda_device)
+    m.lora_b.data = torch.randn(N, rank, generator=g, device=cuda_device).to(torch.bfloat16)
+    x = torch.randn(*shape, K, generator=g, device=cuda_device).to(torch.bfloat16).requires_grad_(True)
+    go = torch.randn(*shape, N, generator=g, device=cuda_device).to(torch.bfloat16)
+    y = m(x, fuse_gelu=gelu, out_dtype=torch.bfloat16)
+    gx, ga, gb = torch.autograd.grad(y, [x, m.lora_a, m.lora_b], go, retain_graph=True)
+    assert y.shape == shape + (N,) and gx.shape == x.shape and ga.shape == m.lora_a.shape and gb.shape == m.lora_b.shape
+
+    with torch.no_grad():
+        a, A, B = x.detach().float().reshape(-1, K), m.lora_a.float(), m.lora_b.float()
+        base = q8.functional.linear.q8_linear(x.detach(), m.weight.data, m.bias.data, None, m.scales, False, torch.bfloat16)
+        pre = base.float().reshape(-1, N) + (a @ A.T) @ B.T
+        want = torch.nn.functional.gelu(pre, approximate="tanh") if gelu else pre
+        d = go.float().reshape(-1, N)
+    if gelu:
+        p = pre.clone().requires_grad_(True)
+        (d,) = torch.autograd.grad(torch.nn.functional.gelu(p, approximate="tanh"), [p], d)
+
+    def rel(t, r):
+        return ((t.float().reshape(r.shape) - r).norm() / r.norm()).item()
+    assert rel(y.detach(), want) < 2 ** -7
+    assert rel(ga, (d @ B).T @ a) < 2 ** -6
+    assert rel(gb, d.T @ (a @ A.T)) < 2 ** -6
+    if not gelu:                                                 # the low-rank gradients stay functions of a, lora_a and g
+        again = torch.autograd.grad(y, [m.lora_b], go, create_graph=True)[0]
+        assert again.requires_grad and rel(again.detach(), gb.float()) < 2 ** -6
