@@ -282,14 +282,16 @@ __device__ __forceinline__ float warp_sum(float v) {
     return v;
 }
 
-// Walsh-Hadamard stages 0 .. log2(V)-1 over V consecutive elements: stride 1 scalar, the rest packed
-template <int V>
+// Walsh-Hadamard stages of stride FIRST (1 or 2) .. V/2 over V consecutive elements: stride 1 scalar, the rest packed
+template <int V, int FIRST = 1>
 __device__ __forceinline__ void butterfly_consecutive(float (&v)[V]) {
+    if constexpr (FIRST == 1) {
 #pragma unroll
-    for (int i = 0; i < V; i += 2) {
-        const float a = v[i], b = v[i + 1];
-        v[i] = __fadd_rn(a, b);
-        v[i + 1] = __fsub_rn(a, b);
+        for (int i = 0; i < V; i += 2) {
+            const float a = v[i], b = v[i + 1];
+            v[i] = __fadd_rn(a, b);
+            v[i + 1] = __fsub_rn(a, b);
+        }
     }
 #pragma unroll
     for (int st = 2; st < V; st <<= 1) {

@@ -37,6 +37,23 @@ __device__ __forceinline__ void fwht_regs(float (&v)[N]) {
     }
 }
 
+// The stride-1 stage of a pair of bf16 values: both as fp32, their sum and difference.  The mixed-precision add takes one
+// operand as bf16, so only the other one has to be widened.  The fused kernels are bound by instruction issue: this and the
+// absmax taken before the 16-bit rounding (see the streamed kernel) bring int8 rows, 24576 x 2048, from 41.3 to 40.3 us,
+// e4m3 rows from 35.1 to 34.1, with norm + modulation from 52.4 to 51.2 and 45.5 to 44.6; 6144 x 8192 48.5 -> 47.8 and
+// 42.6 -> 42.2 (CUDA graphs).
+__device__ __forceinline__ void butterfly_bf16x2(uint32_t w, float& sum, float& diff) {
+    const float hi = __uint_as_float(w & 0xffff0000u);
+    asm("{\n\t"
+        ".reg .b16 lo, up;\n\t"
+        "mov.b32 {lo, up}, %2;\n\t"
+        "add.rn.f32.bf16 %0, lo, %3;\n\t"
+        "sub.rn.f32.bf16 %1, lo, %3;\n\t"
+        "}"
+        : "=f"(sum), "=f"(diff)
+        : "r"(w), "f"(hi));
+}
+
 // One butterfly stage between lanes that differ in bit `mask`.
 template <int N>
 __device__ __forceinline__ void fwht_lanes(float (&v)[N], int lane, int mask) {
@@ -189,9 +206,9 @@ __device__ __forceinline__ void butterfly_groups(float (&v)[V]) {
 // element and scheduler), no longer by barriers and shared memory: 8 bytes per element of exchange (16 above 2048)
 // and 2 x the input size of staging, all accesses conflict-free with immediate offsets.  128 registers, 16 warps per SM.
 // Measured, 24576 x 2048, bf16 in, CUDA graph over inputs larger than L2 (one CTA per row pair, block-wide barriers,
-// two exchanges before): bf16 out 43.6 -> 33.7 us (0.92 of the copy rate), e4m3 rows 45.3 -> 35.9 us, int8 rows
-// 47.1 -> 42 us (one F2I per element on the 8-clock conversion unit), with norm + modulation 72.3 -> 52.1 us (int8).
-// 6144 x 8192: 49.5 -> 41.2, 50.1 -> 43.1, 53.2 -> 49.0, 109 -> 73.7 us.  Tried: 128 values per thread for 4096 and
+// two exchanges before): bf16 out 43.6 -> 33.7 us (0.92 of the copy rate), e4m3 rows 45.3 -> 34.1 us, int8 rows
+// 47.1 -> 40.3 us (one F2I per element on the 8-clock conversion unit), with norm + modulation 72.3 -> 51.2 us (int8).
+// 6144 x 8192: 49.5 -> 41.2, 50.1 -> 42.2, 53.2 -> 47.8, 109 -> 73.7 us.  Tried: 128 values per thread for 4096 and
 // 8192 (one exchange, half the warps; 59 us for int8 rows of 8192), XOR swizzles instead of pads (39.4 us, e4m3 rows).
 
 __device__ __forceinline__ void cp_async_zfill(uint32_t dst, const void* src, int cp_bytes, bool valid) {
@@ -391,8 +408,12 @@ hadamard_stream_kernel(const Tin* __restrict__ x, Tout* __restrict__ out, float*
                 const uint32_t w[4] = {u.x, u.y, u.z, u.w};
 #pragma unroll
                 for (int i = 0; i < 4; ++i) {
-                    v[k * 8 + 2 * i] = __uint_as_float(w[i] << 16);
-                    v[k * 8 + 2 * i + 1] = __uint_as_float(w[i] & 0xffff0000u);
+                    if constexpr (NORM_MOD) {
+                        v[k * 8 + 2 * i] = __uint_as_float(w[i] << 16);
+                        v[k * 8 + 2 * i + 1] = __uint_as_float(w[i] & 0xffff0000u);
+                    } else {
+                        butterfly_bf16x2(w[i], v[k * 8 + 2 * i], v[k * 8 + 2 * i + 1]);
+                    }
                 }
             }
         }
@@ -436,12 +457,11 @@ hadamard_stream_kernel(const Tin* __restrict__ x, Tout* __restrict__ out, float*
                     const __nv_bfloat162 u = __hadd2_rn(__hmul2_rn(n, *reinterpret_cast<const __nv_bfloat162*>(sw + i)),
                                                         *reinterpret_cast<const __nv_bfloat162*>(hw + i));
                     const uint32_t uw = *reinterpret_cast<const uint32_t*>(&u);
-                    v[k * 8 + 2 * i] = __uint_as_float(uw << 16);
-                    v[k * 8 + 2 * i + 1] = __uint_as_float(uw & 0xffff0000u);
+                    butterfly_bf16x2(uw, v[k * 8 + 2 * i], v[k * 8 + 2 * i + 1]);
                 }
             }
         }
-        butterfly_consecutive<V>(v);
+        butterfly_consecutive<V, IN8 ? 1 : 2>(v);
         xch_access<L0, PAD8, true>(xch, v, t);
         __syncwarp();
         load_rows(rel + step);                                 // this warp has read its part of the staging buffer
@@ -499,8 +519,8 @@ hadamard_stream_kernel(const Tin* __restrict__ x, Tout* __restrict__ out, float*
                 }
             }
         } else {
-            // Round to the input dtype (what the unfused chain stores) and take the row's absmax on the packed
-            // values: bf16 pairs, or e4m3 bytes widened to fp16 pairs (exact).  NaNs do not count, as with fmaxf.
+            // Round to the input dtype (what the unfused chain stores) and take the row's absmax: of the fp32 values, rounded
+            // afterwards (bf16), or of the e4m3 bytes widened to fp16 pairs (exact).  NaNs do not count, as with fmaxf.
             uint32_t pk[V / (IN8 ? 4 : 2)];
             float amax;
             if constexpr (IN8) {
@@ -527,7 +547,7 @@ hadamard_stream_kernel(const Tin* __restrict__ x, Tout* __restrict__ out, float*
                 }
                 amax = fmaxf(__low2float(m2), __high2float(m2));
             } else {
-                __nv_bfloat162 m2 = __floats2bfloat162_rn(0.f, 0.f);
+                float mx[2] = {0.f, 0.f};
 #pragma unroll
                 for (int jc = 0; jc < LF::G; jc += SKIP) {
                     if (any_in_row(jc)) {
@@ -535,11 +555,12 @@ hadamard_stream_kernel(const Tin* __restrict__ x, Tout* __restrict__ out, float*
                         for (int f = jc * C; f < (jc + SKIP) * C; f += 2) {
                             const __nv_bfloat162 w = __floats2bfloat162_rn(v[f], v[f + 1]);
                             pk[f / 2] = *reinterpret_cast<const uint32_t*>(&w);
-                            if (in_row(f / C)) m2 = __hmax2(m2, __habs2(w));
+                            float& m = mx[(f / 2) & 1];
+                            if (in_row(f / C)) asm("max.f32 %0, %0, %1, %2;" : "+f"(m) : "f"(fabsf(v[f])), "f"(fabsf(v[f + 1])));
                         }
                     }
                 }
-                amax = fmaxf(__low2float(m2), __high2float(m2));
+                amax = __bfloat162float(__float2bfloat16_rn(fmaxf(mx[0], mx[1])));   // rounding keeps the order
             }
 #pragma unroll
             for (int m = 1; m < (T < 32 ? T : 32); m <<= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, m));
