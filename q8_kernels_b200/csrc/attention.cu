@@ -15,7 +15,7 @@
 // and the result is the mean of V, as in the reference.
 //
 // Structure: one CTA per 128 query rows of one (batch, head), two warpgroups
-// whose register budgets are rebalanced with setmaxnreg (24 / 136 per thread),
+// whose register budgets are rebalanced with setmaxnreg (32 / 128 per thread),
 // three CTAs per SM (registers; 3 x 128 TMEM columns).
 //   warp 0      TMA: Q tile once, then K (64 keys x 64 B) and V (as 64 x 64 rows, or V^T as the
 //               reference lays it out) tiles, all 64B-swizzled, into rings of three; one wait per block
@@ -52,8 +52,10 @@ constexpr int kAttnBN = 64;
 constexpr int kAttnKS = 3;                   // K and V ring depth
 constexpr int kAttnThreads = 256;            // warpgroup 0: TMA + MMA, warpgroup 1: softmax
 constexpr int kAttnRegsLaunch = 80;          // registers per thread at launch: 3 CTAs x 256 threads x 80 = 61440
-constexpr int kAttnRegsIo = 24;              // after setmaxnreg: TMA / MMA warpgroup
-constexpr int kAttnRegsSoftmax = 136;        //                    softmax warpgroup (2 * 80 = 24 + 136)
+// After setmaxnreg (2 * 80 = 32 + 128).  24 and 136 left the issuing threads of the short kernel (MULTI) with more spills and
+// the long one slower: B = 1, H = 32, S = 6144 403.3 -> 400.9 us; 40 and 120: 401.8 us.
+constexpr int kAttnRegsIo = 32;              // TMA / MMA warpgroup
+constexpr int kAttnRegsSoftmax = 128;        // softmax warpgroup
 constexpr int kAttnTmemCols = 128;           // S: [0,64), O: [64,128)
 constexpr uint32_t kAttnOCol = kAttnBN;
 
@@ -416,19 +418,24 @@ flash_attn_fp8_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
             __syncwarp();
         }
 
-        // columns >= N get -inf, columns >= key_lens[b] the reference's mask value
+        // Columns >= key_lens[b] get the reference's mask value, columns >= N -inf.  One after the other, each only where
+        // the block has such columns: one compare and one select per score where both in one pass took two of each, and
+        // the short kernel, with a masked block in nearly every tile, is bound by issue and latency.  B = 2, H = 32,
+        // S_q = 6144, S_kv = 128, lengths 51 and 79: 34.1 -> 30.2 us; B = 1, length 100: 20.3 -> 18.4 us; B = 2, H = 32, S = 1001
+        // (ragged, long kernel): 35.7 -> 34.9 us (with the register budgets above).
         auto mask_scores = [&](int i) {
             const int col0 = (nblk - 1 - i) * kAttnBN;
-            if (col0 + kAttnBN > valid || col0 + kAttnBN > p.N) {
+            auto fill_from = [&](int col, float value) {        // columns of this block from `col` on
+                if (col < kAttnBN) {
 #pragma unroll
-                for (int h = 0; h < 2; ++h)
+                    for (int h = 0; h < 2; ++h)
 #pragma unroll
-                    for (int j = 0; j < 32; ++j) {
-                        const int col = col0 + h * 32 + j;
-                        const float sv = __uint_as_float(cur[h][j]);
-                        cur[h][j] = __float_as_uint(col >= p.N ? -INFINITY : (col >= valid ? -1.0e6f : sv));
-                    }
-            }
+                        for (int j = 0; j < 32; ++j)
+                            if (h * 32 + j >= col) cur[h][j] = __float_as_uint(value);
+                }
+            };
+            if (valid < p.N) fill_from(valid - col0, -1.0e6f);
+            fill_from(p.N - col0, -INFINITY);
         };
 
         // One step.  UNFUSED: products rounded before the subtraction (batch entries without a

@@ -216,6 +216,22 @@ def test_paired_qk_prep_is_two_single_calls(nat, cuda_device):
     assert torch.equal(Hp.bits(k8), Hp.bits(nat.qk_norm_rope_prep(qkv[..., C:2 * C], wk, fc, H, True, scale)))
 
 
+@pytest.mark.parametrize("N,lens", [(77, [1, 31, 32, 33]), (128, [63, 64, 65, 95]), (128, [96, 97, 127, 128]),
+                                    (300, [192, 223, 289, 300])])
+def test_masked_tail_is_the_same_as_fewer_keys(nat, cuda_device, N, lens):
+    """The block visited first is masked per half: key lengths around the edges of halves and blocks, short and long
+    kernel.  A masked key weighs exactly zero, so each batch entry has the bits of a call on its first keys alone (whose
+    own tail, beyond N, is masked with -inf)."""
+    d = cuda_device
+    q8, k8, vt, ks = (t.to(d) if isinstance(t, torch.Tensor) else t for t in _fp8_operands(4, 2, 256, N, seed=N + lens[0]))
+    v = vt[..., :N].transpose(2, 3).contiguous()
+    got = nat.flash_attention(q8, k8, v, ks, torch.tensor(lens, dtype=torch.int32, device=d), torch.bfloat16, v_rows=True)
+    for b, n in enumerate(lens):
+        one = nat.flash_attention(q8[b:b + 1], k8[b:b + 1, :, :n].contiguous(), v[b:b + 1, :, :n].contiguous(), ks, None,
+                                  torch.bfloat16, v_rows=True)
+        assert torch.equal(got[b:b + 1], one), n
+
+
 @pytest.mark.parametrize("B,H,M,N,lens,out", [(2, 32, 900, 128, [77, 128], torch.bfloat16),
                                               (2, 32, 900, 192, None, torch.bfloat16),
                                               (3, 24, 1100, 100, [0, 100, 33], None),
