@@ -660,7 +660,9 @@ flash_attn_fp8_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
 // is the memory order of a [B,S,H*64] projection; a block takes 128 rows of one batch entry of one tensor and fetches
 // all of them before it computes.  Bound by memory: 3 bytes per element.  Measured, B = 2, H = 32, S = 6144 (Q, K and V,
 // 226 MB): 98 us as three launches of 8 lanes per row (64-bit row divisions, 3 shuffles per element) and a V
-// transpose -> 42 us (0.83 of the copy rate).
+// transpose -> 40.2 us; -> 37.0 us (0.93 of the copy rate) with a loop for each form instead of a branch in the loop (63
+// registers instead of 74: eight blocks per SM, not six) and the stride-1 stage on mixed-precision adds (37.4 without).  Q of that
+// size with K and V of 128 rows 16.8 -> 15.6 us, S = 1001 7.6 -> 7.1, S = 50 .. 100 2.45 -> 2.27; the cast alone 33.9 -> 34.3.
 struct PrepSeg {
     const __nv_bfloat16* x;
     uint8_t* out;
@@ -711,44 +713,52 @@ attn_prep_rows_kernel(const __grid_constant__ PrepParams p) {
         s += g.step_s;
         if (h >= H) { h -= H; ++s; }
     }
+    auto rows = [&](auto tag) {
+        constexpr bool HADAMARD = decltype(tag)::value;
 #pragma unroll
-    for (int it = 0; it < 4; ++it) {
-        float v[16];
-        const uint32_t w[8] = {raw[it][0].x, raw[it][0].y, raw[it][0].z, raw[it][0].w,
-                               raw[it][1].x, raw[it][1].y, raw[it][1].z, raw[it][1].w};
+        for (int it = 0; it < 4; ++it) {
+            float v[16];
+            const uint32_t w[8] = {raw[it][0].x, raw[it][0].y, raw[it][0].z, raw[it][0].w,
+                                   raw[it][1].x, raw[it][1].y, raw[it][1].z, raw[it][1].w};
+            if constexpr (!HADAMARD) {
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            v[2 * j] = __uint_as_float(w[j] << 16);
-            v[2 * j + 1] = __uint_as_float(w[j] & 0xffff0000u);
-        }
-        if (g.hadamard) {                     // uniform in the block
-            butterfly_consecutive<16>(v);
+                for (int j = 0; j < 8; ++j) {
+                    v[2 * j] = __uint_as_float(w[j] << 16);
+                    v[2 * j + 1] = __uint_as_float(w[j] & 0xffff0000u);
+                }
+            } else {
 #pragma unroll
-            for (int mk = 1; mk < 4; mk <<= 1) {
-                const float sg = (lane & mk) ? -1.f : 1.f;
-                const float2 sign = make_float2(sg, sg);
+                for (int j = 0; j < 8; ++j) butterfly_bf16x2(w[j], v[2 * j], v[2 * j + 1]);
+                butterfly_consecutive<16, 2>(v);
 #pragma unroll
-                for (int j = 0; j < 16; j += 2) {   // other - u for the upper lane, u + other for the lower: exact
-                    const float2 other = make_float2(__shfl_xor_sync(0xffffffffu, v[j], mk), __shfl_xor_sync(0xffffffffu, v[j + 1], mk));
-                    const float2 u = ffma2(sign, make_float2(v[j], v[j + 1]), other);
+                for (int mk = 1; mk < 4; mk <<= 1) {
+                    const float sg = (lane & mk) ? -1.f : 1.f;
+                    const float2 sign = make_float2(sg, sg);
+#pragma unroll
+                    for (int j = 0; j < 16; j += 2) {   // other - u for the upper lane, u + other for the lower: exact
+                        const float2 other = make_float2(__shfl_xor_sync(0xffffffffu, v[j], mk), __shfl_xor_sync(0xffffffffu, v[j + 1], mk));
+                        const float2 u = ffma2(sign, make_float2(v[j], v[j + 1]), other);
+                        v[j] = u.x;
+                        v[j + 1] = u.y;
+                    }
+                }
+                const float2 sc = make_float2(g.scale, g.scale);
+#pragma unroll
+                for (int j = 0; j < 16; j += 2) {
+                    const float2 u = fmul2(make_float2(v[j], v[j + 1]), sc);
                     v[j] = u.x;
                     v[j + 1] = u.y;
                 }
             }
-            const float2 sc = make_float2(g.scale, g.scale);
+            float lo[8], hi[8];
 #pragma unroll
-            for (int j = 0; j < 16; j += 2) {
-                const float2 u = fmul2(make_float2(v[j], v[j + 1]), sc);
-                v[j] = u.x;
-                v[j + 1] = u.y;
-            }
+            for (int j = 0; j < 8; ++j) { lo[j] = v[j]; hi[j] = v[8 + j]; }
+            const uint2 a = pack8_e4m3_c10(lo), c = pack8_e4m3_c10(hi);
+            if (off[it] >= 0) *reinterpret_cast<uint4*>(ob + off[it] * 64) = make_uint4(a.x, a.y, c.x, c.y);
         }
-        float lo[8], hi[8];
-#pragma unroll
-        for (int j = 0; j < 8; ++j) { lo[j] = v[j]; hi[j] = v[8 + j]; }
-        const uint2 a = pack8_e4m3_c10(lo), c = pack8_e4m3_c10(hi);
-        if (off[it] >= 0) *reinterpret_cast<uint4*>(ob + off[it] * 64) = make_uint4(a.x, a.y, c.x, c.y);
-    }
+    };
+    if (g.hadamard) rows(std::true_type{});                // uniform in the block
+    else rows(std::false_type{});
 }
 
 // Q / K after their projection, fused: RMS norm over all H*64 channels with an fp32 weight (bf16

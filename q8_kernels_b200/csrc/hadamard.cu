@@ -37,23 +37,6 @@ __device__ __forceinline__ void fwht_regs(float (&v)[N]) {
     }
 }
 
-// The stride-1 stage of a pair of bf16 values: both as fp32, their sum and difference.  The mixed-precision add takes one
-// operand as bf16, so only the other one has to be widened.  The fused kernels are bound by instruction issue: this and the
-// absmax taken before the 16-bit rounding (see the streamed kernel) bring int8 rows, 24576 x 2048, from 41.3 to 40.3 us,
-// e4m3 rows from 35.1 to 34.1, with norm + modulation from 52.4 to 51.2 and 45.5 to 44.6; 6144 x 8192 48.5 -> 47.8 and
-// 42.6 -> 42.2 (CUDA graphs).
-__device__ __forceinline__ void butterfly_bf16x2(uint32_t w, float& sum, float& diff) {
-    const float hi = __uint_as_float(w & 0xffff0000u);
-    asm("{\n\t"
-        ".reg .b16 lo, up;\n\t"
-        "mov.b32 {lo, up}, %2;\n\t"
-        "add.rn.f32.bf16 %0, lo, %3;\n\t"
-        "sub.rn.f32.bf16 %1, lo, %3;\n\t"
-        "}"
-        : "=f"(sum), "=f"(diff)
-        : "r"(w), "f"(hi));
-}
-
 // One butterfly stage between lanes that differ in bit `mask`.
 template <int N>
 __device__ __forceinline__ void fwht_lanes(float (&v)[N], int lane, int mask) {
