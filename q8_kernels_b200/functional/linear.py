@@ -199,30 +199,23 @@ class Q8LinearLora(torch.autograd.Function):
         ctx.fuse_gelu = fuse_gelu
         ctx.out_dtype = out_dtype
         ctx.use_hadamard = use_hadamard
-        # The low-rank products run on the rows of all batch entries at once, and their second one adds into the result of
-        # the first term: one rounding where the sum of two 16-bit terms has three, and no kernel for the sum.
-        low = torch.nn.functional.linear(a.reshape(-1, a.shape[-1]), lora_a)
+        lora_y = torch.nn.functional.linear(torch.nn.functional.linear(a, lora_a), lora_b)
         o = _q8_linear_forward(a, b, bias, None, scale_b, False, out_dtype)
-        shape = a.shape[:-1] + lora_b.shape[:1]
-        if o.dtype == low.dtype:
-            o = o.view(-1, shape[-1]).addmm_(low, lora_b.T).view(shape)
-        else:
-            o = o.reshape(shape) + torch.nn.functional.linear(low, lora_b).view(shape)
-        ctx.save_for_backward(o if fuse_gelu else None, a, b, scale_b, lora_a, lora_b, low)
+        o = o.reshape(lora_y.shape) + lora_y
         if fuse_gelu:
+            ctx.save_for_backward(o, a, b, scale_b, lora_a, lora_b)
             o = native.gelu_forward(o, out_dtype)
+        else:
+            ctx.save_for_backward(None, a, b, scale_b, lora_a, lora_b)
         return o
 
     @staticmethod
     def backward(ctx, grad_output):
-        o, a, b, scale_b, lora_a, lora_b, low = ctx.saved_tensors
+        o, a, b, scale_b, lora_a, lora_b = ctx.saved_tensors
         out_dtype = ctx.out_dtype
         if ctx.fuse_gelu:
             grad_output = native.gelu_backward(o, grad_output, out_dtype)
-        a2, g2 = a.reshape(-1, a.shape[-1]), grad_output.reshape(-1, grad_output.shape[-1])
-        if torch.is_grad_enabled():                                             # create_graph: not a constant
-            low = a2 @ lora_a.T
-        grad_out_lora_b = g2 @ lora_b                                           # [s, d] @ [d, r]
+        grad_out_lora_b = grad_output @ lora_b                                  # [.., s, d] @ [d, r]
         if not ctx.use_hadamard:
             raise NotImplementedError("q8_linear_lora backward: only use_hadamard=True is defined "
                                       "(the reference's other branch reads an unset variable)")
@@ -234,14 +227,9 @@ class Q8LinearLora(torch.autograd.Function):
             w = (b * scale_b[:, None]).to(out_dtype)
             w8, ws = quantize_fp8(hadamard_transform(w).T.contiguous())
         g8, gs = quantize_fp8(grad_output.contiguous())
-        grad_x = native.fp8_mm(g8, w8, gs, ws, False, out_dtype).view(a2.shape)
-        if grad_x.dtype == grad_out_lora_b.dtype:
-            grad_x = grad_x.addmm_(grad_out_lora_b, lora_a)
-        else:
-            grad_x = grad_x + grad_out_lora_b @ lora_a
-        grad_x = grad_x.view(a.shape)
-        grad_lora_a = grad_out_lora_b.T @ a2                                    # [r, s] @ [s, h], over all batch entries
-        grad_lora_b = g2.T @ low                                                # [d, s] @ [s, r]
+        grad_x = native.fp8_mm(g8, w8, gs, ws, False, out_dtype).reshape(a.shape) + grad_out_lora_b @ lora_a
+        grad_lora_a = grad_out_lora_b.transpose(-1, -2) @ a                     # [.., r, s] @ [.., s, h]
+        grad_lora_b = grad_output.transpose(-1, -2) @ (a @ lora_a.T)            # [.., d, s] @ [.., s, r]
         return grad_x, None, None, None, None, grad_lora_a, grad_lora_b, None, None, None
 
 

@@ -478,3 +478,50 @@ def test_adapter_products_over_all_batch_entries(cuda_device, shape, rank, gelu)
     if not gelu:                                                 # the low-rank gradients stay functions of a, lora_a and g
         again = torch.autograd.grad(y, [m.lora_b], go, create_graph=True)[0]
         assert again.requires_grad and rel(again.detach(), gb.float()) < 2 ** -6
+
+
+def _adapter(device, K, N, rank, factors=torch.bfloat16):
+    import q8_kernels_b200 as q8
+    g = torch.Generator(device=device).manual_seed(K + N + rank)
+    m = q8.modules.Q8LinearLora(K, N, rank, device=device, dtype=factors)
+    w = torch.randn(N, K, generator=g, device=device).to(torch.bfloat16)
+    m.weight.data, m.scales.data = q8.native.hadamard_quant(w, K ** -0.5, torch.int8)
+    m.bias.data = torch.randn(N, generator=g, device=device)
+    m.lora_b.data = torch.randn(N, rank, generator=g, device=device).to(factors)
+    return m, g
+
+
+@pytest.mark.parametrize("shape,rank", [((2, 33), 4), ((2, 1001), 16), ((70,), 8)])
+def test_adapter_has_the_roundings_of_the_separate_products(cuda_device, shape, rank):
+    """Output and all three gradients, bit for bit: each term rounded to 16 bits, then their sum; the weight gradients per batch
+    entry, then summed over the entries by autograd."""
+    import q8_kernels_b200 as q8
+    K, N = 512, 384
+    m, g = _adapter(cuda_device, K, N, rank)
+    x = torch.randn(*shape, K, generator=g, device=cuda_device).to(torch.bfloat16).requires_grad_(True)
+    go = torch.randn(*shape, N, generator=g, device=cuda_device).to(torch.bfloat16)
+    y = m(x, out_dtype=torch.bfloat16)
+    gx, ga, gb = torch.autograd.grad(y, [x, m.lora_a, m.lora_b], go)
+    with torch.no_grad():
+        a, A, B, w, sw = x.detach(), m.lora_a.detach(), m.lora_b.detach(), m.weight.data, m.scales
+        base = q8.functional.linear.q8_linear(a, w, m.bias.data, None, sw, False, torch.bfloat16)
+        want_y = base.reshape(y.shape) + torch.nn.functional.linear(torch.nn.functional.linear(a, A), B)
+        w8, ws = q8.native.transpose_quant(q8.native.dequant_hadamard(w, sw, K ** -0.5), None)
+        g8, gs = q8.functional.quantizer.quantize_fp8(go)
+        low = go @ B
+        want_x = q8.native.fp8_mm(g8, w8, gs, ws, False, torch.bfloat16).reshape(x.shape) + low @ A
+        want_a = (low.transpose(-1, -2) @ a).sum_to_size(A.shape)
+        want_b = (go.transpose(-1, -2) @ (a @ A.T)).sum_to_size(B.shape)
+    for name, got, want in (("output", y, want_y), ("activation", gx, want_x), ("lora_a", ga, want_a), ("lora_b", gb, want_b)):
+        assert torch.equal(Hp.bits(got.detach()), Hp.bits(want)), name
+
+
+def test_adapter_with_factors_of_another_type_under_autocast(cuda_device):
+    """The low-rank products follow the region's type: fp16 factors in a bf16 region are those factors rounded to bf16."""
+    m, g = _adapter(cuda_device, 512, 384, 8, torch.float16)
+    plain, _ = _adapter(cuda_device, 512, 384, 8)
+    plain.lora_a.data, plain.lora_b.data = m.lora_a.data.to(torch.bfloat16), m.lora_b.data.to(torch.bfloat16)
+    x = torch.randn(2, 40, 512, generator=g, device=cuda_device).to(torch.bfloat16)
+    with torch.autocast("cuda", torch.bfloat16):
+        y = m(x, out_dtype=torch.bfloat16)
+    assert torch.equal(Hp.bits(y.detach()), Hp.bits(plain(x, out_dtype=torch.bfloat16).detach()))
