@@ -64,6 +64,9 @@ Q8K_API int         q8k_wait_selftest(int* dev_status, unsigned tries, void* str
  * plan = {1 if 256 x 256 pair tiles else 0, tile columns, CTAs that share a tile's K range}.  Launches nothing; no
  * counterpart in the reference.                                                                    */
 Q8K_API int         q8k_mm_plan(int int8, int bs_a, int bs_b, int M, int N, int K, int plan[3]);
+/* Columns of the tiles of the last round if the call runs pair tiles: 256, or fewer where that round is cut into narrower
+ * tiles (resid: the call has the gate / residual tail).  For tests; launches nothing; no counterpart in the reference. */
+Q8K_API int         q8k_mm_last_round_columns(int bs_a, int bs_b, int M, int N, int K, int resid, int* columns);
 Q8K_API const char* q8k_error_string(int code);
 Q8K_API const char* q8k_last_error_detail(void);
 

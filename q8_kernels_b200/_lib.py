@@ -34,6 +34,7 @@ SIGNATURES = {
     "q8k_last_error_detail": (ctypes.c_char_p, []),
     "q8k_wait_selftest": (_c_int, [_c_ptr, ctypes.c_uint, _c_ptr]),
     "q8k_mm_plan": (_c_int, [_c_int] * 6 + [_c_ptr]),
+    "q8k_mm_last_round_columns": (_c_int, [_c_int] * 6 + [_c_ptr]),
     "q8k_tokenwise_quant": (_c_int, [_c_ptr, _c_int, _c_ptr, _c_int, _c_ptr, _c_i64, _c_int, _c_i64, _c_ptr]),
     "q8k_transpose_quant": (_c_int, [_c_ptr, _c_int, _c_ptr, _c_ptr, _c_ptr, _c_int, _c_int, _c_ptr]),
     "q8k_dequant_hadamard": (_c_int, [_c_ptr, _c_ptr, _c_ptr, _c_i64, _c_int, _c_f32, _c_ptr]),

@@ -147,6 +147,15 @@ extern "C" int q8k_mm_plan(int int8, int bs_a, int bs_b, int M, int N, int K, in
     return Q8K_OK;
 }
 
+extern "C" int q8k_mm_last_round_columns(int bs_a, int bs_b, int M, int N, int K, int resid, int* columns) {
+    using q8k::set_error_detail;
+    Q8K_REQUIRE(columns != nullptr && bs_a >= 1 && bs_b >= 1 && M > 0 && N > 0 && K > 0 && (int64_t)bs_a * M <= 0x7fffffffLL,
+                Q8K_ERR_INVALID_ARG, "mm_last_round_columns: null result or bad shape");
+    const int batch = q8k::fold_batch(bs_a, bs_b, M);
+    *columns = q8k::pair_last_round_columns(M, N, K, batch, resid != 0);
+    return Q8K_OK;
+}
+
 extern "C" int q8k_q8_mm(const void* a, const void* b, const float* bias, const float* a_scales,
                          const float* b_scales, void* out, int out_dtype, int bs_a, int bs_b, int M, int N,
                          int K, int fuse_gelu, int* dev_status, void* stream) {

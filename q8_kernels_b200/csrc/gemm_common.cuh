@@ -65,6 +65,8 @@ __device__ __forceinline__ float2 epilogue_pair(uint32_t r0, uint32_t r1, float2
 // the clusters, in which case the caller falls back to the split kernel.
 int launch_gemm_pair(bool int8, bool gelu, bool out_e4m3, bool resid, const void* a, const void* b, const GemmParams& p,
                      int bs_a, int bs_b, cudaStream_t st);
+// Columns of the tiles of the last round of such a launch (256: not cut).
+int pair_last_round_columns(int M, int N, int K, int batch, bool resid);
 
 // 128 x bn tiles, each owned by a cluster of sk CTAs that split K (see gemm_split.cu): bn a multiple of 16 up to 256
 // (with sk = 4 of 32), sk 1, 2 or 4 (fp8: 1) and at most the number of 128-byte K slabs.

@@ -315,7 +315,8 @@ gemm_8bit_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
 
             uint32_t r[2][32];
             __syncwarp();
-            ptx::tmem_ld_32x32b_x32(t_row, r[0]);
+            // a tile of 32 columns has no chunk for warps 6-9: no load then, since the wait for it is in the loop
+            if (!NARROW || nch > 0) ptx::tmem_ld_32x32b_x32(t_row, r[0]);
 #pragma unroll
             for (int c = 0; c < NCH; ++c) {
                 if (NARROW && c >= nch) break;                 // (warp-uniform)
@@ -571,6 +572,19 @@ static void narrow_plan(PairParams& pp, int64_t batch, int clusters, bool resid)
     pp.narrow_bn = bn;
     pp.narrow_n = (pp.g.N + bn - 1) / bn;
     pp.total_tiles2 = pp.full_tiles2 + rest * pp.narrow_n;
+}
+
+int pair_last_round_columns(int M, int N, int K, int batch, bool resid) {
+    PairParams pp = {};
+    pp.g.N = N;
+    pp.g.K = K;
+    pp.m_tiles2 = (M + 2 * kGemmBM - 1) / (2 * kGemmBM);
+    pp.n_tiles2 = (N + kPairBN - 1) / kPairBN;
+    const int64_t total = (int64_t)pp.m_tiles2 * pp.n_tiles2 * batch;
+    if (total > 0x7fffffffLL) return kPairBN;
+    pp.total_tiles2 = (int)total;
+    narrow_plan(pp, batch, gemm_num_sms() / 2, resid);
+    return pp.narrow_bn;
 }
 
 int launch_gemm_pair(bool int8, bool gelu, bool out_e4m3, bool resid, const void* a, const void* b, const GemmParams& p,

@@ -152,3 +152,28 @@ def test_gemm_plan_keeps_to_what_the_split_kernel_can_run():
                         assert sk == 1 or (int8 and sk in (2, 4) and (k + 127) // 128 >= 2 * sk)
                         assert ask(plan, int8, batch, 1, m, n, k) == ask(folded, int8, 1, 1, batch * m, n, k)
     assert _lib.lib.q8k_mm_plan(1, 1, 1, 0, 16, 16, ctypes.cast(plan, ctypes.c_void_p)) != 0
+
+
+def test_last_round_columns_are_what_the_pair_kernel_can_run():
+    """Widths over sizes around the edges of row blocks and rounds: multiples of 32 up to 192 or the whole 256, never with a
+    batch of weights or a short K, and a width that leaves one half of the epilogue warps without a column (32) is among them."""
+    import ctypes
+    from q8_kernels_b200 import _lib
+    c = ctypes.c_int()
+
+    def ask(*a):
+        assert _lib.lib.q8k_mm_last_round_columns(*a, ctypes.cast(ctypes.byref(c), ctypes.c_void_p)) == 0
+        return c.value
+
+    widths = set()
+    for m in list(range(129, 12600, 257)) + [2433, 2560, 24576]:
+        for n in (128, 1008, 1024, 2048, 6144, 10240):
+            for k in (2048, 2064, 4096):
+                bn = ask(1, 1, m, n, k, 0)
+                widths.add(bn)
+                assert bn == 256 or (bn % 32 == 0 and 32 <= bn <= 192)
+                assert ask(1, 1, m, n, k, 1) == (bn if k >= 4096 else 256)
+                assert ask(2, 1, m, n, k, 0) == ask(1, 1, 2 * m, n, k, 0)
+                assert ask(2, 2, m, n, k, 0) == ask(1, 1, m, n, 2032, 0) == 256
+    assert widths == {32, 64, 96, 128, 160, 192, 256}
+    assert _lib.lib.q8k_mm_last_round_columns(1, 1, 0, 16, 16, 0, ctypes.cast(ctypes.byref(c), ctypes.c_void_p)) != 0
