@@ -43,7 +43,8 @@ int dt_code(Dt t) {
     }
 }
 
-// The arguments of one call.  `ok` turns false as soon as one of them is not what the fast path takes.
+// The arguments of one call.  `ok` turns false as soon as one of them is not what the fast path takes, their number first of
+// all; from then on none is looked at any more.
 struct Call {
     PyObject* const* args;
     bool ok;
@@ -88,24 +89,27 @@ struct Call {
         if (t != nullptr && t->scalar_type() != type) ok = false;
         return t;
     }
-    const at::Tensor* optional(int i, Dt type) { return args[i] == Py_None ? nullptr : tensor(i, type); }
+    const at::Tensor* optional(int i, Dt type) { return !ok || args[i] == Py_None ? nullptr : tensor(i, type); }
     Dt dtype(int i, Dt none) {
-        if (args[i] == Py_None) return none;
+        if (!ok || args[i] == Py_None) return none;
         if (!THPDtype_Check(args[i])) { ok = false; return none; }
         return reinterpret_cast<THPDtype*>(args[i])->scalar_type;
     }
     bool flag(int i) {
+        if (!ok) return false;
         if (args[i] == Py_True) return true;
         if (args[i] != Py_False) ok = false;
         return false;
     }
     long integer(int i) {
+        if (!ok) return 0;
         if (!PyLong_CheckExact(args[i])) { ok = false; return 0; }
         const long v = PyLong_AsLong(args[i]);
         if (v < 0) { PyErr_Clear(); ok = false; }
         return v;
     }
     float real(int i) {
+        if (!ok) return 0.f;
         if (!PyFloat_CheckExact(args[i])) { ok = false; return 0.f; }
         return (float)PyFloat_AS_DOUBLE(args[i]);
     }

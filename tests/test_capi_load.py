@@ -177,3 +177,29 @@ def test_last_round_columns_are_what_the_pair_kernel_can_run():
                 assert ask(2, 2, m, n, k, 0) == ask(1, 1, m, n, 2032, 0) == 256
     assert widths == {32, 64, 96, 128, 160, 192, 256}
     assert _lib.lib.q8k_mm_last_round_columns(1, 1, 0, 16, 16, 0, ctypes.cast(ctypes.byref(c), ctypes.c_void_p)) != 0
+
+
+def test_host_path_looks_at_no_argument_of_a_call_with_a_wrong_number_of_them():
+    """Every function of the native host path answers None to any other number of arguments than its own (reading on behind
+    the last one ended the process)."""
+    from q8_kernels_b200 import _host
+    arguments = {"tokenwise_quant": 2, "hadamard_quant": 3, "fast_hadamard_transform": 3, "norm_modulate_quant": 4,
+                 "transpose_quant": 2, "dequant_hadamard": 3, "rms_norm": 3, "rms_norm_backward": 5, "rope": 4, "rope_backward": 4,
+                 "mm": 8, "mm_gate_residual": 7, "linear": 7, "flash_attention": 7, "attention_prep_rows": 5, "qkv_prep": 10}
+    assert set(arguments) == {n for n in dir(_host) if not n.startswith(("_", "set_"))}
+    x = torch.zeros(2, 16)
+    for name, want in arguments.items():
+        for n in list(range(want)) + [want + 1, 20]:
+            for a in (x, None, True, 1.0, torch.int8):
+                assert getattr(_host, name)(*[a] * n) is None, (name, n)
+
+
+def test_rotary_tables_of_a_wrong_number_are_refused():
+    """A sequence of tables that is not (cos, sin) reaches the Python body, which refuses it."""
+    from q8_kernels_b200 import native
+    x, w, c = torch.zeros(1, 4, 512, dtype=torch.bfloat16), torch.ones(512), torch.zeros(1, 4, 512)
+    for freqs in ((), (c,), (c, c, c)):
+        for call in (lambda: native.qk_norm_rope_prep(x, w, freqs, 8, True, 0.5),
+                     lambda: native.qk_norm_rope_prep_pair(x, x, w, w, freqs, 8, True, 0.5)):
+            with pytest.raises((ValueError, native.Q8KernelError)):
+                call()
