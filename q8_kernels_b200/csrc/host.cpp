@@ -63,12 +63,11 @@ struct Call {
             ok = false;
     }
     // A plain CUDA tensor of the device that is current; contiguous unless `strided`.
-    const at::Tensor* tensor(int i, bool strided = false) {
+    const at::Tensor* tensor(int i, bool strided = false) { return ok ? tensor_of(args[i], strided) : nullptr; }
+    const at::Tensor* tensor_of(PyObject* o, bool strided = false) {
         static const uint64_t plain =
             c10::DispatchKeySet({c10::DispatchKey::CUDA, c10::DispatchKey::ADInplaceOrView, c10::DispatchKey::AutogradCUDA,
                                  c10::DispatchKey::AutocastCUDA}).raw_repr();
-        if (!ok) return nullptr;
-        PyObject* o = args[i];
         ok = false;
         if (!THPVariable_Check(o)) return nullptr;
         const at::Tensor& t = THPVariable_Unpack(o);
@@ -105,7 +104,7 @@ struct Call {
         if (!ok) return 0;
         if (!PyLong_CheckExact(args[i])) { ok = false; return 0; }
         const long v = PyLong_AsLong(args[i]);
-        if (v < 0) { PyErr_Clear(); ok = false; }
+        if (v < 0 || v > 0x7fffffff) { PyErr_Clear(); ok = false; }
         return v;
     }
     float real(int i) {
@@ -547,52 +546,112 @@ PyObject* attention_prep_rows(PyObject*, PyObject* const* args, Py_ssize_t n) {
     FAST_END
 }
 
-// qkv_prep(xq | None, xk, xv | None, norm_wq | None, norm_wk, cos | None, sin | None, heads, apply_hadamard, scale): column
-// slices [B,S,H*64] of one projection; returns the e4m3 tensors of those that were given
-PyObject* qkv_prep(PyObject*, PyObject* const* args, Py_ssize_t n) {
-    FAST_BEGIN
-    Call c(args, n, 10);
-    const at::Tensor* x[3] = {nullptr, nullptr, nullptr};
-    for (int i = 0; i < 3; ++i)
-        if (c.ok && args[i] != Py_None) x[i] = c.tensor(i, Dt::BFloat16, true);
-    const at::Tensor* wq = c.optional(3, Dt::Float);
-    const at::Tensor* wk = c.tensor(4, Dt::Float);
-    const at::Tensor* co = c.optional(5, Dt::Float);
-    const at::Tensor* si = c.optional(6, Dt::Float);
-    const int64_t H = c.integer(7);
-    const bool had = c.flag(8);
-    const float scale = c.real(9);
+// The pre-passes of a projection's output.  Q, K and V (those that an op has) are column slices [B,S,H*64] of one tensor; the
+// result is their e4m3 tensors.
+struct Prep {
+    const at::Tensor *q = nullptr, *k = nullptr, *v = nullptr, *wq = nullptr, *wk = nullptr;
+    at::Tensor cos, sin;                                       // owned: a list may change while the lock is given up
+    int64_t heads = 0;
+    bool hadamard = false;
+    float scale = 0.f;
+    bool rotate = false;
+
+    // freqs_cis: None or a (cos, sin) tuple or list; anything else is left as it is, an iterator unread
+    void tables(Call& c, int i) {
+        if (!c.ok || c.args[i] == Py_None) return;
+        PyObject* f = c.args[i];
+        if (!(PyTuple_CheckExact(f) || PyList_CheckExact(f)) || PySequence_Fast_GET_SIZE(f) != 2) { c.ok = false; return; }
+        const at::Tensor* t[2] = {nullptr, nullptr};
+        for (int k = 0; k < 2 && c.ok; ++k) t[k] = c.tensor_of(PySequence_Fast_GET_ITEM(f, k));
+        c.need(c.ok && t[0]->scalar_type() == Dt::Float && t[1]->scalar_type() == Dt::Float);
+        if (!c.ok) return;
+        cos = *t[0];
+        sin = *t[1];
+        rotate = true;
+    }
+};
+
+PyObject* prep(Call& c, const Prep& a, const char* op) {
     OR_NONE(c);
-    const at::Tensor* xk = x[1];
-    c.need(xk != nullptr && xk->dim() == 3 && xk->size(2) == H * 64 && (x[0] == nullptr) == (wq == nullptr) &&
-           (co == nullptr) == (si == nullptr));
+    const at::Tensor& k = *a.k;
+    const at::Tensor* x[3] = {a.q, a.k, a.v};
+    c.need(k.dim() == 3 && k.size(2) == a.heads * 64);
     OR_NONE(c);
-    const int64_t B = xk->size(0), S = xk->size(1), C = H * 64, rs = xk->stride(1);
+    const int64_t B = k.size(0), S = k.size(1), C = a.heads * 64, rs = k.stride(1);
     for (const at::Tensor* t : x)
-        c.need(t == nullptr || (t->sizes() == xk->sizes() && t->strides() == xk->strides() && (uintptr_t)cptr(t) % 16 == 0));
-    c.need(xk->stride(2) == 1 && xk->stride(0) == S * rs && rs % 8 == 0 && int_sized(B) && int_sized(S) && int_sized(C) &&
-           wk->numel() == C && (wq == nullptr || wq->numel() == C) &&
-           (co == nullptr || (co->numel() == S * C && si->numel() == S * C)));
+        c.need(t == nullptr || (t->sizes() == k.sizes() && t->strides() == k.strides() && (uintptr_t)cptr(t) % 16 == 0));
+    c.need(k.stride(2) == 1 && k.stride(0) == S * rs && rs % 8 == 0 && int_sized(B) && int_sized(S) && int_sized(C) &&
+           a.wk->numel() == C && (a.wq == nullptr || a.wq->numel() == C) &&
+           (!a.rotate || (a.cos.numel() == S * C && a.sin.numel() == S * C)));
     OR_NONE(c);
+    const float* co = a.rotate ? fptr(&a.cos) : nullptr;
+    const float* si = a.rotate ? fptr(&a.sin) : nullptr;
     at::Tensor o[3];
     void* p[3] = {nullptr, nullptr, nullptr};
-    const int given = (x[0] != nullptr) + 1 + (x[2] != nullptr);
     const int rc = launch([&] {
         for (int i = 0; i < 3; ++i)
             if (x[i] != nullptr) {
-                o[i] = c.empty({B, H, S, 64}, Dt::Float8_e4m3fn);
+                o[i] = c.empty({B, a.heads, S, 64}, Dt::Float8_e4m3fn);
                 p[i] = o[i].data_ptr();
             }
-        if (given == 1)
-            return q8k_qk_norm_rope_prep(cptr(xk), rs, fptr(wk), fptr(co), fptr(si), p[1], (int)B, (int)S, (int)H, had, scale, c.stream());
-        if (x[2] == nullptr)
-            return q8k_qk_norm_rope_prep_pair(cptr(x[0]), cptr(xk), rs, fptr(wq), fptr(wk), fptr(co), fptr(si), p[0], p[1], (int)B,
-                                              (int)S, (int)H, had, scale, c.stream());
-        return q8k_qkv_prep(cptr(x[0]), cptr(xk), cptr(x[2]), rs, fptr(wq), fptr(wk), fptr(co), fptr(si), p[0], p[1], p[2],
-                            (int)B, (int)S, (int)H, had, scale, c.stream());
+        if (a.v != nullptr)
+            return q8k_qkv_prep(cptr(a.q), cptr(a.k), cptr(a.v), rs, fptr(a.wq), fptr(a.wk), co, si, p[0], p[1], p[2], (int)B,
+                                (int)S, (int)a.heads, a.hadamard, a.scale, c.stream());
+        if (a.q != nullptr)
+            return q8k_qk_norm_rope_prep_pair(cptr(a.q), cptr(a.k), rs, fptr(a.wq), fptr(a.wk), co, si, p[0], p[1], (int)B, (int)S,
+                                              (int)a.heads, a.hadamard, a.scale, c.stream());
+        return q8k_qk_norm_rope_prep(cptr(a.k), rs, fptr(a.wk), co, si, p[1], (int)B, (int)S, (int)a.heads, a.hadamard, a.scale,
+                                     c.stream());
     });
-    if (!launched(rc, "qkv_prep")) return nullptr;
-    return given == 1 ? wrap(std::move(o[1])) : tuple_of(o);
+    if (!launched(rc, op)) return nullptr;
+    return a.q == nullptr && a.v == nullptr ? wrap(std::move(o[1])) : tuple_of(o);
+}
+
+// qk_norm_rope_prep(x, norm_w, freqs_cis, heads, apply_hadamard, scale)
+PyObject* qk_norm_rope_prep(PyObject*, PyObject* const* args, Py_ssize_t n) {
+    FAST_BEGIN
+    Call c(args, n, 6);
+    Prep a;
+    a.k = c.tensor(0, Dt::BFloat16, true);
+    a.wk = c.tensor(1, Dt::Float);
+    a.tables(c, 2);
+    a.heads = c.integer(3);
+    a.hadamard = c.flag(4);
+    a.scale = c.real(5);
+    return prep(c, a, "qk_norm_rope_prep");
+    FAST_END
+}
+
+// kv_prep(xk, xv, norm_wk, heads, apply_hadamard, scale)
+PyObject* kv_prep(PyObject*, PyObject* const* args, Py_ssize_t n) {
+    FAST_BEGIN
+    Call c(args, n, 6);
+    Prep a;
+    a.k = c.tensor(0, Dt::BFloat16, true);
+    a.v = c.tensor(1, Dt::BFloat16, true);
+    a.wk = c.tensor(2, Dt::Float);
+    a.heads = c.integer(3);
+    a.hadamard = c.flag(4);
+    a.scale = c.real(5);
+    return prep(c, a, "qkv_prep");
+    FAST_END
+}
+
+// qk_norm_rope_prep_pair(xq, xk, norm_wq, norm_wk, freqs_cis, heads, apply_hadamard, scale, xv | None)
+PyObject* qk_norm_rope_prep_pair(PyObject*, PyObject* const* args, Py_ssize_t n) {
+    FAST_BEGIN
+    Call c(args, n, 9);
+    Prep a;
+    a.q = c.tensor(0, Dt::BFloat16, true);
+    a.k = c.tensor(1, Dt::BFloat16, true);
+    a.wq = c.tensor(2, Dt::Float);
+    a.wk = c.tensor(3, Dt::Float);
+    a.tables(c, 4);
+    a.heads = c.integer(5);
+    a.hadamard = c.flag(6);
+    a.scale = c.real(7);
+    if (c.ok && args[8] != Py_None) a.v = c.tensor(8, Dt::BFloat16, true);
+    return prep(c, a, a.v == nullptr ? "qk_norm_rope_prep_pair" : "qkv_prep");
     FAST_END
 }
 
@@ -623,7 +682,8 @@ PyObject* set_status_word(PyObject*, PyObject* o) {
 PyMethodDef methods[] = {
     FAST(tokenwise_quant), FAST(hadamard_quant), FAST(fast_hadamard_transform), FAST(norm_modulate_quant), FAST(transpose_quant),
     FAST(dequant_hadamard), FAST(rms_norm), FAST(rms_norm_backward), FAST(rope), FAST(rope_backward), FAST(mm),
-    FAST(mm_gate_residual), FAST(linear), FAST(flash_attention), FAST(attention_prep_rows), FAST(qkv_prep),
+    FAST(mm_gate_residual), FAST(linear), FAST(flash_attention), FAST(attention_prep_rows), FAST(qk_norm_rope_prep),
+    FAST(kv_prep), FAST(qk_norm_rope_prep_pair),
     {"set_check", set_check, METH_O, nullptr}, {"set_status_word", set_status_word, METH_O, nullptr}, {nullptr, nullptr, 0, nullptr}};
 PyModuleDef module = {PyModuleDef_HEAD_INIT, "_host", nullptr, -1, methods, nullptr, nullptr, nullptr, nullptr};
 

@@ -573,7 +573,7 @@ def qk_norm_rope_prep(x: torch.Tensor, norm_w: torch.Tensor, freqs_cis, num_head
     e4m3 cast in one kernel: x bf16 [B,S,H*64] (row-strided views allowed) -> e4m3 [B,H,S,64], with the
     bf16 roundings of q8_kernels/modules/attention.py:54-68 and functional/flash_attention.py:50-54.
     ``freqs_cis`` is None or (cos, sin) fp32 [1,S,H*64]."""
-    fast = _host.qkv_prep(None, x, None, None, norm_w, *(freqs_cis if freqs_cis is not None else (None, None)), num_heads, apply_hadamard, qk_scale)
+    fast = _host.qk_norm_rope_prep(x, norm_w, freqs_cis, num_heads, apply_hadamard, qk_scale)
     if fast is not None:
         return fast
     dev = require_cuda(x, norm_w)
@@ -600,7 +600,7 @@ def kv_prep(xk: torch.Tensor, xv: torch.Tensor, norm_wk: torch.Tensor, num_heads
             qk_scale: float):
     """K and V of a cross-attention (two column slices of one fused projection output, same strides) in one
     launch: K as qk_norm_rope_prep without rotation, V cast to e4m3 rows; returns (k8, v8), each [B,H,S,64]."""
-    fast = _host.qkv_prep(None, xk, xv, None, norm_wk, None, None, num_heads, apply_hadamard, qk_scale)
+    fast = _host.kv_prep(xk, xv, norm_wk, num_heads, apply_hadamard, qk_scale)
     if fast is not None:
         return fast
     dev = require_cuda(xk, xv, norm_wk)
@@ -629,7 +629,7 @@ def qk_norm_rope_prep_pair(xq: torch.Tensor, xk: torch.Tensor, norm_wq: torch.Te
     strides, e.g. column slices of a fused projection output); returns (q8, k8), each e4m3 [B,H,S,64],
     byte-identical to two separate calls.  With ``xv`` (a third slice of the same kind) the launch also
     casts V to e4m3 rows [B,H,S,64] (what attention_cast_rows gives) and (q8, k8, v8) is returned."""
-    fast = _host.qkv_prep(xq, xk, xv, norm_wq, norm_wk, *(freqs_cis if freqs_cis is not None else (None, None)), num_heads, apply_hadamard, qk_scale)
+    fast = _host.qk_norm_rope_prep_pair(xq, xk, norm_wq, norm_wk, freqs_cis, num_heads, apply_hadamard, qk_scale, xv)
     if fast is not None:
         return fast
     dev = require_cuda(xq, xk, norm_wq, norm_wk, xv)

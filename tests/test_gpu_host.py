@@ -119,3 +119,30 @@ def test_host_path_leaves_everything_else_to_python(cuda_device):
         native.fast_hadamard_transform(torch.zeros(2, 32768, device=cuda_device, dtype=BF16), 1.0)
     with pytest.raises(native.Q8KernelError):
         native.q8_mm(x.to(E4M3), x[0].to(E4M3), torch.ones(128, device=cuda_device), torch.ones(32, device=cuda_device), False, BF16)
+
+
+def test_pre_passes_refuse_what_their_python_bodies_refuse(cuda_device, monkeypatch):
+    """None in a required place, in the rotary tables too, is no shorter form of the call; other sequences of the two tables are
+    taken as before."""
+    from q8_kernels_b200 import _lib, native
+    _lib.status_word(cuda_device)
+    qkv = torch.randn(2, 33, 1536, device=cuda_device).to(BF16)
+    q, k, v = qkv[..., :512], qkv[..., 512:1024], qkv[..., 1024:]
+    w = torch.rand(512, device=cuda_device)
+    cos, sin = torch.randn(1, 33, 512, device=cuda_device), torch.randn(1, 33, 512, device=cuda_device)
+    refused = [(native.kv_prep, (k, None, w, 8, True, 0.05)), (native.kv_prep, (None, v, w, 8, True, 0.05)),
+               (native.kv_prep, (k, v, None, 8, True, 0.05)), (native.qk_norm_rope_prep, (q, None, None, 8, True, 0.05)),
+               (native.qk_norm_rope_prep, (q, w, (None, None), 8, True, 0.05)), (native.qk_norm_rope_prep, (q, w, (cos,), 8, True, 0.05)),
+               (native.qk_norm_rope_prep, (q, w, (cos, sin, cos), 8, True, 0.05)), (native.qk_norm_rope_prep, (q, w, None, 2 ** 58 + 8, True, 0.05)),
+               (native.qk_norm_rope_prep_pair, (None, k, None, w, None, 8, True, 0.05)),
+               (native.qk_norm_rope_prep_pair, (None, k, None, w, None, 8, True, 0.05, v)),
+               (native.qk_norm_rope_prep_pair, (q, k, None, w, None, 8, True, 0.05)),
+               (native.qk_norm_rope_prep_pair, (q, k, w, w, (cos, None), 8, True, 0.05))]
+    for fn, args in refused:
+        with pytest.raises((AttributeError, ValueError, native.Q8KernelError)):
+            fn(*args)
+    with monkeypatch.context() as m:
+        m.setattr(native, "_host", _NoHost())
+        want = native.qk_norm_rope_prep(q, w, (cos, sin), 8, True, 0.05)
+    for freqs in ((cos, sin), [cos, sin], iter((cos, sin)), torch.stack((cos, sin))):
+        assert torch.equal(_bits(native.qk_norm_rope_prep(q, w, freqs, 8, True, 0.05)), _bits(want))
