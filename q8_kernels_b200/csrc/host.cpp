@@ -386,10 +386,10 @@ PyObject* rope_backward(PyObject*, PyObject* const* args, Py_ssize_t n) {
 }
 
 // ---------------------------------------------------------------- products
-// mm(a, b, bias | None, a_scales, b_scales, fuse_gelu, out_type, in_type): in_type int8 or e4m3
+// mm(a, b, bias | None, a_scales, b_scales, fuse_gelu, out_type, in_type, op): in_type int8 or e4m3, op the public name
 PyObject* mm(PyObject*, PyObject* const* args, Py_ssize_t n) {
     FAST_BEGIN
-    Call c(args, n, 8);
+    Call c(args, n, 9);
     const Dt in = c.dtype(7, Dt::Undefined);
     const at::Tensor* a = c.tensor(0, in);
     const at::Tensor* b = c.tensor(1, in);
@@ -398,6 +398,7 @@ PyObject* mm(PyObject*, PyObject* const* args, Py_ssize_t n) {
     const at::Tensor* sb = c.tensor(4, Dt::Float);
     const bool gelu = c.flag(5);
     const Dt out = c.dtype(6, Dt::Float8_e4m3fn);
+    c.need(c.ok && PyUnicode_Check(args[8]));
     OR_NONE(c);
     c.need(quant_type(in) && dt_code(out) >= 0 &&
            (a->dim() == 2 || a->dim() == 3) && (b->dim() == 2 || b->dim() == 3));
@@ -415,7 +416,8 @@ PyObject* mm(PyObject*, PyObject* const* args, Py_ssize_t n) {
         return (i8 ? q8k_q8_mm : q8k_fp8_mm)(cptr(a), cptr(b), fptr(bias), fptr(sa), fptr(sb), y.data_ptr(), dt_code(out), (int)ba,
                                              (int)bb, (int)m, (int)nn, (int)k, gelu, word, c.stream());
     });
-    return launched(rc, i8 ? "q8_mm" : "fp8_mm") ? wrap(std::move(y)) : nullptr;
+    const char* op = rc == Q8K_OK ? "" : PyUnicode_AsUTF8(args[8]);
+    return op != nullptr && launched(rc, op) ? wrap(std::move(y)) : nullptr;
     FAST_END
 }
 

@@ -346,7 +346,7 @@ def rms_norm_backward(x_normed: torch.Tensor, x_norms: torch.Tensor, grad_out: t
 # ---------------------------------------------------------------- gemm._C
 
 def _gemm(fn, name, a, b, bias, a_scales, b_scales, fuse_gelu, out_type, in_dtype):
-    fast = _host.mm(a, b, bias, a_scales, b_scales, fuse_gelu, out_type, in_dtype)
+    fast = _host.mm(a, b, bias, a_scales, b_scales, fuse_gelu, out_type, in_dtype, name)
     if fast is not None:
         return fast
     dev = require_cuda(a, b, bias, a_scales, b_scales)

@@ -185,7 +185,7 @@ def test_host_path_looks_at_no_argument_of_a_call_with_a_wrong_number_of_them():
     from q8_kernels_b200 import _host
     arguments = {"tokenwise_quant": 2, "hadamard_quant": 3, "fast_hadamard_transform": 3, "norm_modulate_quant": 4,
                  "transpose_quant": 2, "dequant_hadamard": 3, "rms_norm": 3, "rms_norm_backward": 5, "rope": 4, "rope_backward": 4,
-                 "mm": 8, "mm_gate_residual": 7, "linear": 7, "flash_attention": 7, "attention_prep_rows": 5, "qk_norm_rope_prep": 6,
+                 "mm": 9, "mm_gate_residual": 7, "linear": 7, "flash_attention": 7, "attention_prep_rows": 5, "qk_norm_rope_prep": 6,
                  "kv_prep": 6, "qk_norm_rope_prep_pair": 9}
     assert set(arguments) == {n for n in dir(_host) if not n.startswith(("_", "set_"))}
     x = torch.zeros(2, 16)

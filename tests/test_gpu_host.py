@@ -146,3 +146,14 @@ def test_pre_passes_refuse_what_their_python_bodies_refuse(cuda_device, monkeypa
         want = native.qk_norm_rope_prep(q, w, (cos, sin), 8, True, 0.05)
     for freqs in ((cos, sin), [cos, sin], iter((cos, sin)), torch.stack((cos, sin))):
         assert torch.equal(_bits(native.qk_norm_rope_prep(q, w, freqs, 8, True, 0.05)), _bits(want))
+
+
+def test_an_error_of_a_product_names_the_function_that_was_called(cuda_device):
+    from q8_kernels_b200 import native
+    a = torch.ones(4, 24, dtype=torch.int8, device=cuda_device)  # K is no multiple of 16
+    s, bias = torch.ones(4, device=cuda_device), torch.zeros(4, device=cuda_device)
+    f = torch.ones(4, 24, device=cuda_device).to(E4M3)
+    for name, call in (("q8_mm", lambda: native.q8_mm(a, a, s, s, False)), ("q8_mm_bias", lambda: native.q8_mm_bias(a, a, bias, s, s, False)),
+                       ("fp8_mm", lambda: native.fp8_mm(f, f, s, s, False)), ("fp8_mm_bias", lambda: native.fp8_mm_bias(f, f, bias, s, s, False))):
+        with pytest.raises(native.Q8KernelError, match=f"^{name}: "):
+            call()
