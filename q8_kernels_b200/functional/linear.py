@@ -2,8 +2,8 @@
 
 Inference: where the reference launches Hadamard, quantizer and GEMM as three
 kernels with two intermediate tensors, the 16-bit / e4m3 activation path here is
-one native call: a fused Hadamard+quantizer producer writing into a cached
-scratch buffer, then the tcgen05 GEMM.
+one native call: a fused Hadamard+quantizer producer writing into a scratch
+buffer of the call, then the tcgen05 GEMM.
 
 Training side (the activation gradient only, as in the reference: weights are
 frozen): when the activation requires grad the call goes through an autograd

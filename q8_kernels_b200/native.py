@@ -701,13 +701,10 @@ def attention_cast_rows(v: torch.Tensor) -> torch.Tensor:
 
 # ---------------------------------------------------------------- fused linear chain
 
-_workspaces = {}
-
-
 def linear(x: torch.Tensor, w: torch.Tensor, w_scales: torch.Tensor, bias: Optional[torch.Tensor],
            use_hadamard: bool, fuse_gelu: bool, out_type: torch.dtype) -> torch.Tensor:
-    """Hadamard + per-token quantizer + GEMM in one native call over a cached
-    per-device scratch buffer (q8_kernels/functional/linear.py:24-42,138-159)."""
+    """Hadamard + per-token quantizer + GEMM in one native call (q8_kernels/functional/linear.py:24-42,138-159).  The scratch for
+    the quantised rows comes from the caching allocator on the current stream and goes back to it with the call."""
     fast = _host.linear(x, w, w_scales, bias, use_hadamard, fuse_gelu, out_type)
     if fast is not None:
         return fast
@@ -716,15 +713,7 @@ def linear(x: torch.Tensor, w: torch.Tensor, w_scales: torch.Tensor, bias: Optio
     x2 = x.contiguous()
     M, N = x.numel() // K if K else 0, w.shape[0]
     need = lib.q8k_linear_workspace_bytes(M, K)
-    if torch.cuda.is_current_stream_capturing():
-        # a buffer allocated during capture belongs to that graph's private pool: never cache it
-        ws = torch.empty(max(need, 1), dtype=torch.uint8, device=dev)
-    else:
-        key = (dev.index, stream_ptr(dev))
-        ws = _workspaces.get(key)
-        if ws is None or ws.numel() < need:
-            ws = torch.empty(max(need, 1), dtype=torch.uint8, device=dev)
-            _workspaces[key] = ws
+    ws = torch.empty(max(need, 1), dtype=torch.uint8, device=dev)
     out_shape = (x.shape[0], x.shape[1], N) if x.dim() == 3 else (1, M, N)
     out = torch.empty(out_shape, dtype=out_type, device=dev)
     launch(dev, "linear", lib.q8k_linear, ptr(x2), dt(x2.dtype), ptr(w), dt(w.dtype), ptr(w_scales), ptr(bias),

@@ -157,3 +157,21 @@ def test_an_error_of_a_product_names_the_function_that_was_called(cuda_device):
                        ("fp8_mm", lambda: native.fp8_mm(f, f, s, s, False)), ("fp8_mm_bias", lambda: native.fp8_mm_bias(f, f, bias, s, s, False))):
         with pytest.raises(native.Q8KernelError, match=f"^{name}: "):
             call()
+
+
+def test_a_linear_holds_no_scratch_after_the_call(cuda_device, monkeypatch):
+    """Neither path keeps memory: what is allocated after a call is its result."""
+    from q8_kernels_b200 import _lib, native
+    _lib.status_word(cuda_device)
+    x = torch.randn(2, 1000, 512, device=cuda_device).to(BF16)[:, ::2]          # strided: the Python body's
+    w = torch.ones(96, 512, dtype=torch.int8, device=cuda_device)
+    s = torch.ones(96, device=cuda_device)
+    for t in (x, x.contiguous()):
+        for stream in (torch.cuda.current_stream(), torch.cuda.Stream()):
+            stream.wait_stream(torch.cuda.current_stream())
+            with torch.cuda.stream(stream):
+                held = torch.cuda.memory_allocated()
+                out = native.linear(t, w, s, None, True, False, BF16)
+                assert torch.cuda.memory_allocated() - held == (out.nbytes + 511) // 512 * 512
+                del out
+    torch.cuda.synchronize()
