@@ -4,7 +4,8 @@ which exports the C ABI declared in ``include/q8_kernels_b200.h``; ``csrc/host.c
 ``q8_kernels_b200/_host.so`` over it, against the headers and libraries of the installed torch.
 
 Run ``python q8_kernels_b200/build.py`` (add ``--force`` to rebuild, ``-v`` for
-ptxas resource usage).  nvcc cross-compiles without a GPU present.
+ptxas resource usage).  nvcc cross-compiles without a GPU present.  A program that calls the C ABI needs
+neither torch nor Python headers: ``--library-only``, or a machine without torch, builds the library alone.
 """
 from __future__ import annotations
 
@@ -49,7 +50,11 @@ def _stale(target: str, deps) -> bool:
 def _build_host(force: bool) -> None:
     src = os.path.join(CSRC, "host.cpp")
     header = os.path.join(PKG_DIR, "..", "include", "q8_kernels_b200.h")
-    torch_dir = os.path.dirname(importlib.util.find_spec("torch").origin)
+    torch = importlib.util.find_spec("torch")
+    if torch is None:
+        sys.stderr.write(f"torch is not installed: {os.path.basename(LIB_PATH)} is built, the extension of the Python package is not\n")
+        return
+    torch_dir = os.path.dirname(torch.origin)
     version = os.path.join(torch_dir, "version.py")              # another torch needs another build
     if not (force or _stale(HOST_PATH, [src, header, version])):
         return
@@ -65,8 +70,9 @@ def _build_host(force: bool) -> None:
         raise RuntimeError("g++ failed on host.cpp")
 
 
-def build(force: bool = False, verbose: bool = False) -> str:
-    """Compile the library if any source is newer than it; return its path."""
+def build(force: bool = False, verbose: bool = False, library_only: bool = False) -> str:
+    """Compile the library if any source is newer than it, and the Python package's extension over it unless
+    ``library_only``; return the library's path."""
     os.makedirs(OBJ_DIR, exist_ok=True)
     headers = [os.path.join(CSRC, f) for f in os.listdir(CSRC) if f.endswith((".cuh", ".h"))]
     headers.append(os.path.join(PKG_DIR, "..", "include", "q8_kernels_b200.h"))
@@ -93,7 +99,8 @@ def build(force: bool = False, verbose: bool = False) -> str:
         if res.returncode != 0:
             sys.stderr.write(res.stdout + res.stderr)
             raise RuntimeError("link failed")
-    _build_host(force)
+    if not library_only:
+        _build_host(force)
     return LIB_PATH
 
 
@@ -101,5 +108,6 @@ if __name__ == "__main__":
     ap = argparse.ArgumentParser(description=__doc__)
     ap.add_argument("--force", action="store_true")
     ap.add_argument("-v", "--verbose", action="store_true")
+    ap.add_argument("--library-only", action="store_true", help="the C ABI without the Python package's extension")
     a = ap.parse_args()
-    print(build(force=a.force, verbose=a.verbose))
+    print(build(force=a.force, verbose=a.verbose, library_only=a.library_only))
