@@ -105,6 +105,9 @@ try:
 except ImportError as e:
     raise ImportError(f"q8_kernels_b200._host is missing or does not load ({e}): build it with "
                       "`python q8_kernels_b200/build.py`") from e
+if not torch.__version__.startswith(_host.__torch_version__):           # tensors are passed by torch's C++ types
+    raise ImportError(f"q8_kernels_b200._host was built against torch {_host.__torch_version__}, this is {torch.__version__}: "
+                      "run `python q8_kernels_b200/build.py`")
 
 
 class Q8KernelError(RuntimeError):

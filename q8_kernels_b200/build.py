@@ -1,7 +1,8 @@
 """Build recipe for the native library: every .cu under csrc/ is compiled for
 sm_100a with nvcc into one shared object, ``q8_kernels_b200/libq8k_b200.so``,
 which exports the C ABI declared in ``include/q8_kernels_b200.h``; ``csrc/host.cpp`` becomes the CPython extension
-``q8_kernels_b200/_host.so`` over it, against the headers and libraries of the installed torch.
+``q8_kernels_b200/_host.<interpreter>.so`` over it, against the headers and libraries of the installed torch.  Its
+name carries the interpreter's ABI tag, so another Python does not load it.
 
 Run ``python q8_kernels_b200/build.py`` (add ``--force`` to rebuild, ``-v`` for
 ptxas resource usage).  nvcc cross-compiles without a GPU present.  A program that calls the C ABI needs
@@ -21,7 +22,8 @@ PKG_DIR = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(PKG_DIR, "csrc")
 OBJ_DIR = os.path.join(PKG_DIR, "build")
 LIB_PATH = os.path.join(PKG_DIR, "libq8k_b200.so")
-HOST_PATH = os.path.join(PKG_DIR, "_host.so")
+HOST_PATH = os.path.join(PKG_DIR, "_host" + sysconfig.get_config_var("EXT_SUFFIX"))
+HOST_KEY = os.path.join(OBJ_DIR, os.path.basename(HOST_PATH) + ".key")     # what the extension was built against
 
 SOURCES = ["capi.cu", "rowwise.cu", "hadamard.cu", "gemm.cu", "gemm_pair.cu", "gemm_split.cu", "attention.cu"]
 
@@ -54,20 +56,32 @@ def _build_host(force: bool) -> None:
     if torch is None:
         sys.stderr.write(f"torch is not installed: {os.path.basename(LIB_PATH)} is built, the extension of the Python package is not\n")
         return
+    untagged = os.path.join(PKG_DIR, "_host.so")                 # of a build before the names were tagged
+    if os.path.exists(untagged) and untagged != HOST_PATH:
+        os.remove(untagged)
     torch_dir = os.path.dirname(torch.origin)
-    version = os.path.join(torch_dir, "version.py")              # another torch needs another build
-    if not (force or _stale(HOST_PATH, [src, header, version])):
+    with open(os.path.join(torch_dir, "version.py")) as f:
+        key = torch_dir + "\n" + f.read()                        # another torch needs another build
+    if not (force or _stale(HOST_PATH, [src, header]) or not os.path.exists(HOST_KEY) or open(HOST_KEY).read() != key):
         return
+    abi = subprocess.run([sys.executable, "-c", "import torch; print(int(torch.compiled_with_cxx11_abi()))"],
+                         capture_output=True, text=True, cwd=OBJ_DIR)
+    if abi.returncode != 0:
+        sys.stderr.write(abi.stderr)
+        raise RuntimeError("torch does not import")
     inc = [sysconfig.get_paths()["include"], os.path.join(torch_dir, "include"),
            os.path.join(torch_dir, "include", "torch", "csrc", "api", "include"),
            os.path.join(os.path.dirname(os.path.dirname(_nvcc())) if os.path.isabs(_nvcc()) else "/usr/local/cuda", "include")]
-    cmd = (["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden"] + ["-I" + d for d in inc]
+    cmd = (["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden", "-D_GLIBCXX_USE_CXX11_ABI=" + abi.stdout.strip()]
+           + ["-I" + d for d in inc]
            + [src, "-o", HOST_PATH, "-L" + os.path.join(torch_dir, "lib"), "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_python",
               "-L" + PKG_DIR, "-l:libq8k_b200.so", "-Wl,-rpath,$ORIGIN"])
     res = subprocess.run(cmd, capture_output=True, text=True)
     if res.returncode != 0:
         sys.stderr.write(res.stdout + res.stderr)
         raise RuntimeError("g++ failed on host.cpp")
+    with open(HOST_KEY, "w") as f:
+        f.write(key)
 
 
 def build(force: bool = False, verbose: bool = False, library_only: bool = False) -> str:

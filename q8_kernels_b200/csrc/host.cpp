@@ -20,6 +20,7 @@
 #include <torch/csrc/Dtype.h>
 #include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/python_variable.h>
+#include <torch/version.h>
 
 #include <cmath>
 
@@ -691,4 +692,8 @@ PyModuleDef module = {PyModuleDef_HEAD_INIT, "_host", nullptr, -1, methods, null
 
 }  // namespace
 
-PyMODINIT_FUNC PyInit__host() { return PyModule_Create(&module); }
+PyMODINIT_FUNC PyInit__host() {
+    PyObject* m = PyModule_Create(&module);
+    if (m != nullptr && PyModule_AddStringConstant(m, "__torch_version__", TORCH_VERSION) != 0) Py_CLEAR(m);
+    return m;
+}
