@@ -175,3 +175,109 @@ def test_a_linear_holds_no_scratch_after_the_call(cuda_device, monkeypatch):
                 assert torch.cuda.memory_allocated() - held == (out.nbytes + 511) // 512 * 512
                 del out
     torch.cuda.synchronize()
+
+
+class _Recording(_Counting):
+    def __getattr__(self, name):
+        def call(*a):
+            r = getattr(self.host, name)(*a)
+            self.answers.append((name, a, r))
+            return r
+        return call
+
+
+# places of the extension's functions that may be None
+_OPTIONAL = {("transpose_quant", 1), ("rms_norm", 1), ("rms_norm_backward", 3), ("mm", 2), ("mm_gate_residual", 2), ("mm_gate_residual", 5),
+             ("linear", 3), ("flash_attention", 4), ("qk_norm_rope_prep_pair", 8)}
+
+
+def test_host_path_takes_nothing_else_in_the_place_of_a_tensor(cuda_device, monkeypatch):
+    from q8_kernels_b200 import _lib, native
+    _lib.status_word(cuda_device)
+    host = native._host
+    for name, calls in _cases(cuda_device).items():
+        for args in calls:
+            recording = _Recording(host)
+            with monkeypatch.context() as m:
+                m.setattr(native, "_host", recording)
+                getattr(native, name)(*args)
+            fn, a, answer = recording.answers[0]
+            assert answer is not None
+            for i, t in enumerate(a):
+                if isinstance(t, torch.Tensor):
+                    for other in (3, t.cpu(), t.double()) + (() if (fn, i) in _OPTIONAL else (None,)):
+                        assert getattr(host, fn)(*a[:i], other, *a[i + 1:]) is None, (fn, i, type(other))
+
+
+def _map(args, f):
+    return tuple(f(a) if isinstance(a, torch.Tensor) else tuple(map(f, a)) if isinstance(a, tuple) else a for a in args)
+
+
+def _same(got, want, name):
+    for a, b in zip(_flat(got), _flat(want)):
+        assert torch.equal(_bits(a), _bits(b)), name
+
+
+def test_host_path_launches_on_the_current_stream(cuda_device):
+    """Inputs that another stream fills late, behind a delay: only work queued on that stream sees them."""
+    from q8_kernels_b200 import _lib, native
+    _lib.status_word(cuda_device)
+    side = torch.cuda.Stream()
+    for name, calls in _cases(cuda_device).items():
+        for args in calls:
+            want = getattr(native, name)(*args)
+            late = _map(args, torch.zeros_like)
+            torch.cuda.synchronize()
+            with torch.cuda.stream(side):
+                torch.cuda._sleep(1_000_000)
+                for to, t in zip(late, args):
+                    for x, y in zip(to, t) if isinstance(t, tuple) else [(to, t)] if isinstance(t, torch.Tensor) else []:
+                        x.copy_(y)
+                got = getattr(native, name)(*late)
+            side.synchronize()
+            _same(got, want, name)
+
+
+def test_host_path_under_capture(cuda_device):
+    from q8_kernels_b200 import _lib, native
+    _lib.status_word(cuda_device)
+    for name, calls in _cases(cuda_device).items():
+        for args in calls:
+            want = getattr(native, name)(*args)
+            static = _map(args, torch.zeros_like)
+            getattr(native, name)(*static)
+            torch.cuda.synchronize()
+            graph = torch.cuda.CUDAGraph()
+            with torch.cuda.graph(graph):
+                got = getattr(native, name)(*static)
+            for to, t in zip(static, args):
+                for x, y in zip(to, t) if isinstance(t, tuple) else [(to, t)] if isinstance(t, torch.Tensor) else []:
+                    x.copy_(y)
+            graph.replay()
+            torch.cuda.synchronize()
+            _same(got, want, name)
+
+
+def test_host_path_from_several_threads(cuda_device):
+    """The interpreter lock is given up inside a call: threads on streams of their own, all functions at once."""
+    import threading
+    from q8_kernels_b200 import _lib, native
+    _lib.status_word(cuda_device)
+    calls = [(name, args, getattr(native, name)(*args)) for name, c in _cases(cuda_device).items() for args in c]
+    torch.cuda.synchronize()
+    failed = []
+
+    def work(first):
+        try:
+            with torch.cuda.stream(torch.cuda.Stream()):
+                for i in range(3 * len(calls)):
+                    name, args, want = calls[(first + i) % len(calls)]
+                    _same(getattr(native, name)(*args), want, name)
+        except BaseException as e:                              # (an assertion too: it must reach the test)
+            failed.append(e)
+    threads = [threading.Thread(target=work, args=(k * 5,)) for k in range(4)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not failed, failed
