@@ -422,7 +422,8 @@ flash_attn_fp8_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
         // the block has such columns: one compare and one select per score where both in one pass took two of each, and
         // the short kernel, with a masked block in nearly every tile, is bound by issue and latency.  B = 2, H = 32,
         // S_q = 6144, S_kv = 128, lengths 51 and 79: 34.1 -> 30.2 us; B = 1, length 100: 20.3 -> 18.4 us; B = 2, H = 32, S = 1001
-        // (ragged, long kernel): 35.7 -> 34.9 us (with the register budgets above).
+        // (ragged, long kernel): 35.7 -> 34.9 us (with the register budgets above).  Behind: one tile of queries per CTA on one key
+        // block, B = 1, H = 8, 64 x 64 3.90 -> 4.00 us.
         auto mask_scores = [&](int i) {
             const int col0 = (nblk - 1 - i) * kAttnBN;
             auto fill_from = [&](int col, float value) {        // columns of this block from `col` on
@@ -663,6 +664,8 @@ flash_attn_fp8_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
 // transpose -> 40.2 us; -> 37.0 us (0.93 of the copy rate) with a loop for each form instead of a branch in the loop (63
 // registers instead of 74: eight blocks per SM, not six) and the stride-1 stage on mixed-precision adds (37.4 without).  Q of that
 // size with K and V of 128 rows 16.8 -> 15.6 us, S = 1001 7.6 -> 7.1, S = 50 .. 100 2.45 -> 2.27; the cast alone 33.9 -> 34.3.
+// (Two launches of it in a row, four to five blocks per SM each, read 5.3 -> 5.6 us, B = 2, H = 20, S_q = 1500, S_kv = 250: the second
+// launch's waiting blocks hold the slots.  In front of the attention kernel 20.7 -> 19.4 us for both.)
 struct PrepSeg {
     const __nv_bfloat16* x;
     uint8_t* out;

@@ -35,11 +35,16 @@ int gemm_num_sms() {
 //          threads) and its bytes at 140 GB/s (one SM's L2 port; 1.7 x the bytes where K is not a multiple of 128 and
 //          rows straddle cache lines), times the CTAs of the busiest SM, and 1.5 for every CTA beyond the first there;
 //          3.85e-5 bn^2 for the epilogue; the exchange of a K split; 0.06 per MB of weights
-//   pair:  6.5 + 0.31 per slab and wave of 74 tiles
+//   pair:  6.5 + 0.31 per slab and wave of 74 tiles.  This is whole waves: where narrow_plan cuts the last one, the pair kernel
+//          takes up to a sixth less.
 // Examples, int8 (pair or 128 x 128 tiles before -> now): M = 128, N = K = 2048 9.5 -> 5.2 (bn 32);  M = 77, N = 10240,
 // K = 4096 15.4 -> 11.6 (bn 80);  M = 128, N = 2048, K = 8192 23.1 -> 9.0 (bn 64, sk 4);  M = 1024, N = 2048, K = 8192
 // 26.2 -> 18.0 (bn 128).  At N = K = 2048 the line to the pair kernel lies between M = 1024 (12.2 -> 8.4) and M = 2048
 // (12.6 against 14.9).
+// Just above a full wave the whole-wave model still sends to the split kernel what narrow pair tiles do faster (7 % of the sizes
+// that have such tiles, M = 129 .. 12289; split against pair): fp8 M = 2433, N = 2048, K = 4096 31.5 against 24.2;  M = 5000,
+// N = 1024, K = 4096 26.9 against 20.1;  M = 10000, N = 512, K = 8192 51.3 against 38.5;  M = 1200, N = K = 4096 21.9 against
+// 20.2;  but M = 4640, N = 1024, K = 8192 33.5 against 36.4 and M = 300, N = 10240, K = 4096 21.1 against 22.7.
 // Half of a pair tile is padding where M or N is at most 128, so there the split kernel is the rule; but one tile per CTA
 // pays its set-up for every tile, and from three rounds of pair tiles on the persistent pair kernel is faster all the same
 // (int8, pair against split): N = 128, K = 1024 M = 24576 11.5 against 11.4, M = 49152 15.7 against 20.9, M = 196608 45.3

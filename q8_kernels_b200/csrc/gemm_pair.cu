@@ -553,6 +553,12 @@ static int launch_pair(const CUtensorMap& ta, const CUtensorMap& tb, const CUten
 // loaded for fewer columns, and there is one more epilogue), so 224 columns gain nothing (576 tiles 57.0 against 57.4, 504
 // tiles 59.3 against 64.1), nor does a short K: K = 1024 26.0 against 26.9, with the residual, whose epilogue is the
 // slower part of a short tile, K = 2048 25.5 against 26.2 and K = 1024 33.2 against 35.0.
+// The line at eight full rounds is on the safe side of the gain, which is a part of one round: nine and ten rounds would still give
+// 2 to 5 % (wide against narrow tiles, int8: M = 14336, N = 3072, K = 4096 125.0 against 118.8, 64 columns;  M = 24576, N = K = 2048
+// 82.4 against 79.4, 128 columns;  M = 12510, N = 4096, K = 2048 79.8 against 78.5, 160 columns), 31 and 41 rounds nothing that
+// stands out of the power cap's spread (M = 24576, K = 2048, N = 6144 235.9 against 236.8, N = 8192 302.2 against 300.3).  Below the
+// line 108 drawn shapes of M = 256 .. 24576, all kinds and widths, gave 0.98 to 1.21 x, median 1.07 x; the one below 0.99 (int8,
+// M = 2954, N = 10240, K = 8192) gave 0.97, 1.05 and 1.05 when repeated.
 static void narrow_plan(PairParams& pp, int64_t batch, int clusters, bool resid) {
     pp.full_tiles2 = pp.total_tiles2;
     pp.narrow_m = pp.m_tiles2;
