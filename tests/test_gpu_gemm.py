@@ -286,27 +286,14 @@ def test_padded_pair_tiles_and_folded_batches(nat, cuda_device, kind, B, Bw, M, 
         Hp.assert_bit_equal(fused, gate * out + resid, "gate and residual in the epilogue")
 
 
-@pytest.mark.parametrize("M,N,K,bn", [(6144, 2048, 2048, 160),    # 13 tiles of 160 columns for each of 6 row blocks
-                                      (6100, 2000, 2064, 160),    # M, N and K tails, the last narrow tile partial
-                                      (2002, 6144, 2048, 160), (3096, 2048, 4112, 128), (12510, 2048, 2048, 96),
-                                      (7401, 2048, 4096, 64),
-                                      (2560, 2048, 2048, 32),     # half of the epilogue warps have no column
-                                      (2400, 2000, 4112, 32), (4800, 1024, 2048, 32), (7296, 1024, 2064, 192),
-                                      (7500, 1008, 4112, 192)])
+@pytest.mark.parametrize("M,N,K", [(6144, 2048, 2048),            # 13 tiles of 160 columns for each of 6 row blocks
+                                   (6100, 2000, 2064),            # M, N and K tails, the last narrow tile partial
+                                   (2002, 6144, 2048), (3096, 2048, 4112), (12510, 2048, 2048), (7401, 2048, 4096)])
 @pytest.mark.parametrize("kind", ["int8", "fp8", "fp8 e4m3 out", "int8 gelu", "int8 residual", "fp8 residual"])
-def test_narrow_tiles_of_the_last_round(cuda_device, M, N, K, bn, kind):
+def test_narrow_tiles_of_the_last_round(cuda_device, M, N, K, kind):
     """Products whose last round is cut into narrow tiles: every row has the bits that it has in a call of few rows (other
-    tiles on the other kernel), where int8 sums are exact and fp8 sums have one order.  One shape or more for each width that
-    148 SMs give; the width is asserted.  With the residual tail the last round is cut from K = 4096 on."""
-    import ctypes
-    from q8_kernels_b200 import _lib, native as nat
-    resid_tail = "residual" in kind
-    if resid_tail:
-        K = max(K, 4112)
-    plan, columns = (ctypes.c_int * 3)(), ctypes.c_int()
-    assert _lib.lib.q8k_mm_plan(int(kind.startswith("int8")), 1, 1, M, N, K, ctypes.cast(plan, ctypes.c_void_p)) == 0
-    assert _lib.lib.q8k_mm_last_round_columns(1, 1, M, N, K, int(resid_tail), ctypes.cast(ctypes.byref(columns), ctypes.c_void_p)) == 0
-    assert (plan[0], columns.value) == (1, bn)
+    tiles on the other kernel), where int8 sums are exact and fp8 sums have one order."""
+    from q8_kernels_b200 import native as nat
     g = torch.Generator(device=cuda_device).manual_seed(M + N + K)
     if kind.startswith("int8"):
         a, b = (torch.randint(-127, 128, s, generator=g, device=cuda_device, dtype=torch.int8) for s in ((M, K), (N, K)))
@@ -324,8 +311,28 @@ def test_narrow_tiles_of_the_last_round(cuda_device, M, N, K, bn, kind):
         mm = nat.q8_mm_bias if kind.startswith("int8") else nat.fp8_mm_bias
         return mm(a[r], b, bias, sa[r], sb, "gelu" in kind, out)
     got = product(slice(0, M))[0]
-    assert _lib.read_status(cuda_device) == 0
     for r0 in range(0, M, 512):
         r = slice(r0, min(r0 + 512, M))
         want = product(r)[0]
         assert torch.equal(got[r].view(torch.uint8), want.view(torch.uint8)), (r0, (got[r] != want).sum())
+
+
+_NARROW = [(6144, 2048, 2048, 160), (6100, 2000, 2064, 160), (2002, 6144, 2048, 160), (3096, 2048, 4112, 128), (12510, 2048, 2048, 96),
+           (7401, 2048, 4096, 64)]
+_EDGES = [(2560, 2048, 2048, 32), (2400, 2000, 4112, 32), (4800, 1024, 2048, 32),    # half of the epilogue warps have no column
+          (7296, 1024, 2064, 192), (7500, 1008, 4112, 192)]
+
+
+@pytest.mark.parametrize("M,N,K,bn,kind", [c + (k,) for c in _EDGES for k in ("int8", "fp8", "fp8 e4m3 out", "int8 gelu")]
+                         + [(m, n, max(k, 4112), bn, r) for m, n, k, bn in _NARROW + _EDGES for r in ("int8 residual", "fp8 residual")])
+def test_every_width_of_the_last_round(cuda_device, M, N, K, bn, kind):
+    """The narrowest and the widest tiles too, and the residual tail at the K from which its last round is cut; the width that
+    148 SMs give is asserted."""
+    import ctypes
+    from q8_kernels_b200 import _lib
+    plan, columns = (ctypes.c_int * 3)(), ctypes.c_int()
+    assert _lib.lib.q8k_mm_plan(int(kind.startswith("int8")), 1, 1, M, N, K, ctypes.cast(plan, ctypes.c_void_p)) == 0
+    assert _lib.lib.q8k_mm_last_round_columns(1, 1, M, N, K, int("residual" in kind), ctypes.cast(ctypes.byref(columns), ctypes.c_void_p)) == 0
+    assert (plan[0], columns.value) == (1, bn)
+    test_narrow_tiles_of_the_last_round(cuda_device, M, N, K, kind)
+    assert _lib.read_status(cuda_device) == 0
